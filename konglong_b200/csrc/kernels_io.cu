@@ -45,39 +45,131 @@ __global__ void inject_scatter_k(TraceDev t, int it, float *__restrict__ w0, con
   }
 }
 
-// Grouped injection: one CTA per xy tile; every cell of the tile sums the xy
-// weight of the group members whose kernel box covers it, then the tile's
-// columns receive that sum times the common z kernel.
-__global__ void inject_group_k(GroupDev g, TraceDev t, int it, float *__restrict__ w0, const float *__restrict__ vel,
-                               int nx, int ny, int nz) {
-  extern __shared__ float s_xy[];
-  const int T = g.tile;
-  const int tile = blockIdx.x;
-  const int x0 = g.tile_xy[2 * tile], y0 = g.tile_xy[2 * tile + 1];
+// Grouped injection: a CTA of (group tile, quarter of its rows).  Every cell
+// of the quarter sums the xy weight of the group members whose kernel box
+// covers it, then the columns receive that sum times the common z kernel.
+// Bound by latency: a tile of a 4-cell receiver spacing has ~80 members, and
+// reading each member's box, sample and taps from global memory per cell put
+// four dependent loads on every one of them (66 us for 2304 receivers on a
+// 199 x 163 grid, 143 CTAs).  Members are staged in shared memory kInjChunk
+// at a time instead, a warp each: the box and the x / y taps that meet the
+// quarter, the sample folded into the y taps.  A cell's member then costs two
+// shared loads, and a tile is split over kInjSplit CTAs to fill the chip.
+// Sums keep the member order.
+constexpr int kInjTile = kGroupTile, kInjChunk = 32, kInjSplit = 4, kInjRows = kInjTile / kInjSplit;
+__global__ void __launch_bounds__(256) inject_group_k(GroupDev g, TraceDev t, int it, float *__restrict__ w0,
+                                                      const float *__restrict__ vel, int nx, int ny, int nz) {
+  constexpr int CELLS = kInjRows * kInjTile;
+  __shared__ float s_xy[CELLS], s_kx[kInjChunk][kInjTile], s_ky[kInjChunk][kInjRows];
+  __shared__ int4 s_box[kInjChunk];
+  const int tile = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;  // 8 warps
+  const int x0 = g.tile_xy[2 * tile], y0 = g.tile_xy[2 * tile + 1] + blockIdx.y * kInjRows;
   const int b = g.tile_ptr[tile], e = g.tile_ptr[tile + 1];
-  for (int c = threadIdx.x; c < T * T; c += blockDim.x) {
-    const int ix = x0 + c % T, iy = y0 + c / T;
-    float acc = 0.f;
-    for (int k = b; k < e; k++) {
-      const int r = g.tile_list[k];
-      const int *o = t.off + 3 * r, *l = t.len + 3 * r;
-      const int jx = ix - o[0], jy = iy - o[1];
-      if (jx < 0 || jx >= l[0] || jy < 0 || jy >= l[1]) continue;
-      const float val = t.traces[(long long)r * t.nt + it] * t.scaler;
-      acc += val * t.ky[(long long)r * t.ly + jy] * t.kx[(long long)r * t.lx + jx];
+  if (y0 >= ny) return;
+  const int c = threadIdx.x, lx = c % kInjTile, ly = c / kInjTile;
+  float acc = 0.f;
+  for (int k0 = b; k0 < e; k0 += kInjChunk) {
+    const int m = min(kInjChunk, e - k0);
+    // this chunk's members, kInjChunk / 8 per warp: every record and tap load
+    // is issued before the first is stored
+    constexpr int U = kInjChunk / 8;
+    int4 bx[U];
+    float tap[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int j = warp + 8 * u;
+      bx[u] = j < m ? g.tile_list[k0 + j] : make_int4(0, 0, 0, 0);
     }
-    s_xy[c] = acc;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long long r = bx[u].x;
+      // first index relative to the quarter and length of the box
+      bx[u] = make_int4(bx[u].y - x0, bx[u].w & 0xffff, bx[u].z - y0, (int)((unsigned)bx[u].w >> 16));
+      tap[u] = 0.f;
+      if (lane < kInjTile) {
+        const int i = lane - bx[u].x;
+        if ((unsigned)i < (unsigned)bx[u].y) tap[u] = t.kx[r * t.lx + i];
+      } else if (lane < kInjTile + kInjRows) {
+        const int i = lane - kInjTile - bx[u].z;
+        if ((unsigned)i < (unsigned)bx[u].w) tap[u] = t.traces[r * t.nt + it] * t.scaler * t.ky[r * t.ly + i];
+      }
+    }
+    __syncthreads();  // the previous chunk has been read
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int j = warp + 8 * u;
+      if (j >= m) continue;
+      if (lane == 0) s_box[j] = bx[u];
+      if (lane < kInjTile) s_kx[j][lane] = tap[u];
+      else if (lane < kInjTile + kInjRows) s_ky[j][lane - kInjTile] = tap[u];
+    }
+    __syncthreads();
+    if (c < CELLS)
+      for (int j = 0; j < m; j++) {
+        const int4 bx = s_box[j];
+        if ((unsigned)(lx - bx.x) < (unsigned)bx.y && (unsigned)(ly - bx.z) < (unsigned)bx.w)
+          acc += s_ky[j][ly] * s_kx[j][lx];
+      }
   }
+  if (c < CELLS) s_xy[c] = acc;
   __syncthreads();
   const int lz = g.lz;
-  for (int k = threadIdx.x; k < T * T * lz; k += blockDim.x) {
-    const int iz = k % lz, c = k / lz;
-    const int ix = x0 + c % T, iy = y0 + c / T;
-    const float s = s_xy[c];
+#pragma unroll 4
+  for (int k = threadIdx.x; k < CELLS * lz; k += blockDim.x) {
+    const int iz = k % lz, cc = k / lz;
+    const int ix = x0 + cc % kInjTile, iy = y0 + cc / kInjTile;
+    const float s = s_xy[cc];
     if (ix >= nx || iy >= ny || s == 0.f) continue;
     const long long i = ((long long)iy * nx + ix) * nz + g.offz + iz;
     w0[i] += s * g.kz[iz] * vel[i];
   }
+}
+
+// Sum of a receiver's kernel box, one warp: four lanes share a column's z taps
+// (taps z, z + 4, ... in runs of kBoxZ), eight columns at a time walk the xy
+// taps, so a load instruction reads eight short contiguous runs and the column
+// indices advance without divisions; kBoxU steps of columns are loaded before
+// the first is summed.  The flat tap index cost two integer divisions a tap
+// (the batch's 3072 receivers of 20^3 taps took 112 us), one step at a time
+// waited on memory for each (65 us).
+constexpr int kBoxZ = 5, kBoxU = 4;
+__device__ __forceinline__ float extract_box(const TraceDev &t, int r, const float *__restrict__ w0, int nx, int nz,
+                                             int lane) {
+  const int *o = t.off + 3 * r, *l = t.len + 3 * r;
+  const int lx = l[0], ly = l[1], lz = l[2];
+  const float *kx = t.kx + (long long)r * t.lx, *ky = t.ky + (long long)r * t.ly, *kz = t.kz + (long long)r * t.lz;
+  const int zq = lane & 3, cq = lane >> 2;
+  const float *p = w0 + ((long long)o[1] * nx + o[0]) * nz + o[2];
+  float acc = 0.f;
+  if (lx > 0) {
+    const int sy = 8 / lx, sx = 8 - sy * lx;
+    for (int z0 = zq; z0 < lz; z0 += 4 * kBoxZ) {
+      float wz[kBoxZ];
+#pragma unroll
+      for (int k = 0; k < kBoxZ; k++) wz[k] = z0 + 4 * k < lz ? kz[z0 + 4 * k] : 0.f;
+      int iy = cq / lx, ix = cq - iy * lx;
+      while (iy < ly) {
+        float cxy[kBoxU], v[kBoxU][kBoxZ];
+#pragma unroll
+        for (int u = 0; u < kBoxU; u++) {
+          const bool in = iy < ly;
+          cxy[u] = in ? ky[iy] * kx[ix] : 0.f;
+          const float *c = p + ((long long)iy * nx + ix) * nz + z0;
+#pragma unroll
+          for (int k = 0; k < kBoxZ; k++) v[u][k] = in && z0 + 4 * k < lz ? c[4 * k] : 0.f;
+          iy += sy, ix += sx;
+          if (ix >= lx) ix -= lx, iy++;
+        }
+#pragma unroll
+        for (int u = 0; u < kBoxU; u++)
+#pragma unroll
+          for (int k = 0; k < kBoxZ; k++) acc += cxy[u] * wz[k] * v[u][k];
+      }
+    }
+  }
+#pragma unroll
+  for (int s = 16; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  return acc;
 }
 
 // one warp per receiver over its kernel box
@@ -87,54 +179,69 @@ __global__ void extract_direct_k(TraceDev t, const float *__restrict__ w0, float
   const int lane = threadIdx.x & 31;
   if (k0 >= (t.ids ? t.nids : t.ntr)) return;
   const int r = t.ids ? t.ids[k0] : k0;
-  const int *o = t.off + 3 * r, *l = t.len + 3 * r;
-  const int lx = l[0], ly = l[1], lz = l[2];
-  float acc = 0.f;
-  for (int k = lane; k < lx * ly * lz; k += 32) {
-    const int iz = k % lz, ix = (k / lz) % lx, iy = k / (lz * lx);
-    const float cx = t.ky[(long long)r * t.ly + iy] * t.kx[(long long)r * t.lx + ix];
-    acc += cx * t.kz[(long long)r * t.lz + iz] * w0[((long long)(iy + o[1]) * nx + ix + o[0]) * nz + o[2] + iz];
-  }
-#pragma unroll
-  for (int s = 16; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  const float acc = extract_box(t, r, w0, nx, nz, lane);
   if (lane == 0) out[(long long)r * nt_out + jt] = acc;
 }
 
-// z reduction of a group's band on its tiles: plane[iy*nx+ix] = sum kz * w0
-__global__ void extract_zplane_k(GroupDev g, const float *__restrict__ w0, float *__restrict__ plane, int nx, int ny,
-                                 int nz) {
+// z reduction of a group's band on its tiles: plane[iy*nx+ix] = sum kz * w0.
+// Four lanes per column, 64 columns per CTA (grid y: quarters of the tile), so
+// every load of the tile is in flight at once; with a warp walking 32 columns
+// one after the other, a load and five shuffles each, the pass took 28-30 us
+// on every grid, as long as the stencil of a 128^3 shot.
+__global__ void __launch_bounds__(256) extract_zplane_k(GroupDev g, const float *__restrict__ w0,
+                                                        float *__restrict__ plane, int nx, int ny, int nz) {
   const int T = g.tile;
   const int tile = blockIdx.x;
-  const int x0 = g.tile_xy[2 * tile], y0 = g.tile_xy[2 * tile + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x / 32, nw = blockDim.x / 32;
-  for (int c = warp; c < T * T; c += nw) {
-    const int ix = x0 + c % T, iy = y0 + c / T;
-    if (ix >= nx || iy >= ny) continue;
-    const long long base = ((long long)iy * nx + ix) * nz + g.offz;
-    float acc = 0.f;
-    for (int iz = lane; iz < g.lz; iz += 32) acc += g.kz[iz] * w0[base + iz];
-#pragma unroll
-    for (int s = 16; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-    if (lane == 0) plane[(long long)iy * nx + ix] = acc;
+  const int c = blockIdx.y * (blockDim.x / 4) + threadIdx.x / 4, zq = threadIdx.x & 3;
+  const int ix = g.tile_xy[2 * tile] + c % T, iy = g.tile_xy[2 * tile + 1] + c / T;
+  const bool in = c < T * T && ix < nx && iy < ny;
+  float acc = 0.f;
+  if (in) {
+    const float *p = w0 + ((long long)iy * nx + ix) * nz + g.offz;
+#pragma unroll 5
+    for (int iz = zq; iz < g.lz; iz += 4) acc += g.kz[iz] * p[iz];
   }
+  acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+  acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+  if (in && zq == 0) plane[(long long)iy * nx + ix] = acc;
 }
 
-__global__ void extract_xy_k(GroupDev g, TraceDev t, const float *__restrict__ plane, float *__restrict__ out, int jt,
-                             int nt_out, int nx) {
+// xy dot products on the z-reduced plane, one warp per receiver: lane k takes
+// the flat taps k, k + 32, ..., kXyU of them loaded together, their x / y
+// indices advanced without divisions.  Bound by the chain record -> taps and
+// plane -> sum, so the member record holds all that the addresses need.
+constexpr int kXyU = 7;
+__global__ void __launch_bounds__(256) extract_xy_k(GroupDev g, TraceDev t, const float *__restrict__ plane,
+                                                    float *__restrict__ out, int jt, int nt_out, int nx) {
   const int m = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
   if (m >= g.ntr) return;
-  const int r = g.members[m];
-  const int *o = t.off + 3 * r, *l = t.len + 3 * r;
+  const int4 rec = g.members[m];
+  const int lx = rec.z, ly = rec.w;
+  const float *kx = t.kx + (long long)rec.x * t.lx, *ky = t.ky + (long long)rec.x * t.ly;
+  const float *p = plane + rec.y;
   float acc = 0.f;
-  for (int k = lane; k < l[0] * l[1]; k += 32) {
-    const int ix = k % l[0], iy = k / l[0];
-    acc += t.ky[(long long)r * t.ly + iy] * t.kx[(long long)r * t.lx + ix] *
-           plane[(long long)(iy + o[1]) * nx + ix + o[0]];
+  if (lx > 0) {
+    int iy = lane / lx, ix = lane - iy * lx;
+    const int sy = 32 / lx, sx = 32 - sy * lx;
+    while (iy < ly) {
+      float a[kXyU], b[kXyU], v[kXyU];
+#pragma unroll
+      for (int u = 0; u < kXyU; u++) {
+        const bool in = iy < ly;
+        a[u] = in ? ky[iy] : 0.f;
+        b[u] = in ? kx[ix] : 0.f;
+        v[u] = in ? p[(long long)iy * nx + ix] : 0.f;
+        iy += sy, ix += sx;
+        if (ix >= lx) ix -= lx, iy++;
+      }
+#pragma unroll
+      for (int u = 0; u < kXyU; u++) acc += a[u] * b[u] * v[u];
+    }
   }
 #pragma unroll
   for (int s = 16; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (lane == 0) out[(long long)r * nt_out + jt] = acc;
+  if (lane == 0) out[(long long)rec.x * nt_out + jt] = acc;
 }
 
 // per-slab max |w| (one CTA per y slab)
@@ -287,16 +394,7 @@ __global__ void batch_extract_k(const IsoBatchShot *__restrict__ shots, int jt, 
   if (r >= t.ntr || jt < 0 || jt >= t.nt) return;
   const float *w0 = (it & 1) ? S.wa : S.wb;
   const int nx = S.a.nx, nz = S.a.nz;
-  const int *o = t.off + 3 * r, *l = t.len + 3 * r;
-  const int lx = l[0], ly = l[1], lz = l[2];
-  float acc = 0.f;
-  for (int k = lane; k < lx * ly * lz; k += 32) {
-    const int iz = k % lz, ix = (k / lz) % lx, iy = k / (lz * lx);
-    const float cx = t.ky[(long long)r * t.ly + iy] * t.kx[(long long)r * t.lx + ix];
-    acc += cx * t.kz[(long long)r * t.lz + iz] * w0[((long long)(iy + o[1]) * nx + ix + o[0]) * nz + o[2] + iz];
-  }
-#pragma unroll
-  for (int s = 16; s; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  const float acc = extract_box(t, r, w0, nx, nz, lane);
   if (lane == 0) S.ext_out[(long long)r * t.nt + jt] = acc;
 }
 
@@ -452,7 +550,7 @@ void launch_inject_group(const GroupDev &gr, const TraceDev &t, int it, float *p
                          int nx, int ny, int nz, cudaStream_t st) {
   (void)plane;
   if (gr.ntiles <= 0 || it < 0 || it >= t.nt) return;
-  inject_group_k<<<gr.ntiles, 256, gr.tile * gr.tile * sizeof(float), st>>>(gr, t, it, w0, vel, nx, ny, nz);
+  inject_group_k<<<dim3(gr.ntiles, kInjSplit), 256, 0, st>>>(gr, t, it, w0, vel, nx, ny, nz);
 }
 
 void launch_extract_direct(const TraceDev &t, const float *w0, float *out, int jt, int nt_out, int nx, int ny, int nz,
@@ -466,7 +564,7 @@ void launch_extract_direct(const TraceDev &t, const float *w0, float *out, int j
 void launch_extract_group(const GroupDev &gr, const TraceDev &t, const float *w0, float *plane, float *out, int jt,
                           int nt_out, int nx, int ny, int nz, cudaStream_t st) {
   if (gr.ntiles <= 0 || jt < 0 || jt >= nt_out) return;
-  extract_zplane_k<<<gr.ntiles, 256, 0, st>>>(gr, w0, plane, nx, ny, nz);
+  extract_zplane_k<<<dim3(gr.ntiles, (gr.tile * gr.tile + 63) / 64), 256, 0, st>>>(gr, w0, plane, nx, ny, nz);
   extract_xy_k<<<(gr.ntr + 7) / 8, 256, 0, st>>>(gr, t, plane, out, jt, nt_out, nx);
 }
 

@@ -1179,10 +1179,13 @@ static int upload_traces(Engine *h, TraceSetDev &t, int ntr, int lx, int ly, int
     by_z[key].push_back(r);
   }
   std::vector<int> loose;
-  const int T = 16;
+  const int T = kGroupTile;
   for (auto &kv : by_z) {
     const std::vector<int> &mem = kv.second;
-    if (mem.size() < 16) {
+    // the packed member tables hold 16-bit lengths; longer kernels go trace by trace
+    bool packs = mem.size() >= 16;
+    for (int r : mem) packs = packs && len3[3 * r] < 65536 && len3[3 * r + 1] < 65536;
+    if (!packs) {
       loose.insert(loose.end(), mem.begin(), mem.end());
       continue;
     }
@@ -1200,29 +1203,34 @@ static int upload_traces(Engine *h, TraceSetDev &t, int ntr, int lx, int ly, int
       for (int ty = o[1] / T; ty <= (o[1] + l[1] - 1) / T; ty++)
         for (int tx = o[0] / T; tx <= (o[0] + l[0] - 1) / T; tx++) lists[(size_t)ty * ntx + tx].push_back(r);
     }
-    std::vector<int> txy, ptr{0}, lst;
+    std::vector<int> txy, ptr{0};
+    std::vector<int4> lst, recs;
+    for (int r : mem)
+      recs.push_back(make_int4(r, off3[3 * r + 1] * h->d.nx + off3[3 * r], len3[3 * r], len3[3 * r + 1]));
     for (int ty = 0; ty < nty; ty++)
       for (int tx = 0; tx < ntx; tx++) {
         auto &L = lists[(size_t)ty * ntx + tx];
         if (L.empty()) continue;
         txy.push_back(tx * T), txy.push_back(ty * T);
-        lst.insert(lst.end(), L.begin(), L.end());
+        for (int r : L)
+          lst.push_back(make_int4(r, off3[3 * r], off3[3 * r + 1], len3[3 * r] | (int)((unsigned)len3[3 * r + 1] << 16)));
         ptr.push_back((int)lst.size());
       }
     g.ntiles = (int)txy.size() / 2;
-    int *dm, *dxy, *dp, *dl;
+    int *dxy, *dp;
+    int4 *dm, *dl;
     float *dkz;
     TRY(h->alloc(dm, mem.size()));
     TRY(h->alloc(dkz, std::max(1, g.lz)));
     TRY(h->alloc(dxy, std::max<size_t>(2, txy.size())));
     TRY(h->alloc(dp, ptr.size()));
     TRY(h->alloc(dl, std::max<size_t>(1, lst.size())));
-    t.group_allocs.insert(t.group_allocs.end(), {dm, dkz, dxy, dp, dl});
-    CK(cudaMemcpy(dm, mem.data(), 4 * mem.size(), cudaMemcpyHostToDevice));
+    t.group_allocs.insert(t.group_allocs.end(), {(void *)dm, dkz, dxy, dp, dl});
+    CK(cudaMemcpy(dm, recs.data(), sizeof(int4) * recs.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(dkz, kz + (size_t)r0 * lz, 4 * g.lz, cudaMemcpyHostToDevice));
     if (!txy.empty()) CK(cudaMemcpy(dxy, txy.data(), 4 * txy.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(dp, ptr.data(), 4 * ptr.size(), cudaMemcpyHostToDevice));
-    if (!lst.empty()) CK(cudaMemcpy(dl, lst.data(), 4 * lst.size(), cudaMemcpyHostToDevice));
+    if (!lst.empty()) CK(cudaMemcpy(dl, lst.data(), sizeof(int4) * lst.size(), cudaMemcpyHostToDevice));
     g.members = dm, g.kz = dkz, g.tile_xy = dxy, g.tile_ptr = dp, g.tile_list = dl;
     t.groups.push_back(g);
   }

@@ -43,18 +43,20 @@ struct TraceDev {
   float scaler;
 };
 
+constexpr int kGroupTile = 16;  // edge of the groups' xy tiles (cells)
+
 // Receiver / source groups sharing one z kernel (same first index, length
 // and coefficients): the xy part is gathered per cell of an xy tile.
 struct GroupDev {
   int ntr;               // members
-  const int *members;    // trace ids
+  const int4 *members;   // per member: trace id, first cell iy * nx + ix, x and y lengths
   int offz, lz;
   const float *kz;       // [lz]
   // xy tiles covered by the group and, per tile, the member list (CSR)
-  int ntiles, tile;      // tile edge (cells)
+  int ntiles, tile;      // tile edge (cells): kGroupTile
   const int *tile_xy;    // [ntiles][2] tile origin (ix0, iy0)
   const int *tile_ptr;   // [ntiles+1]
-  const int *tile_list;  // member trace ids
+  const int4 *tile_list; // per entry: trace id, first x and y index, lengths x | y << 16
 };
 
 // Snapshot / imaging-condition access fused into the stencil kernels.
