@@ -15,7 +15,7 @@
 #include <type_traits>
 
 #include "kernel_api.h"
-#include "rtm_device.cuh"
+#include "pml4.cuh"
 #include "tma.cuh"
 
 namespace rtm {
@@ -23,157 +23,56 @@ namespace {
 
 constexpr int R4 = 4;  // stencil radius
 
-__device__ __forceinline__ float cmp4(const float4 &v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
-__device__ __forceinline__ void set4(float4 &v, int c, float x) {
-  if (c == 0) v.x = x;
-  else if (c == 1) v.y = x;
-  else if (c == 2) v.z = x;
-  else v.w = x;
-}
-__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
-__device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
-
-// Round-R memory of one PML face for the thread's 4 cells: the arrays of the z, x
-// and y derivative components (pml1's component index per face dimension) at the
-// current plane, the per-plane stride, and the face's recursion constants with the
-// layer of the first cell and its step along z (z faces: one layer per cell).
-struct Face1 {
-  float *zc, *xc, *yc;
-  long long stride;
-  const float *co;
-  int L, dl;
-};
-
-template <int R>
-__device__ __forceinline__ Face1 face1(const PmlFace &F, int d, long long idx, long long stride, int L, int dl) {
-  const int cz = d == DZ ? 0 : 1, cx = d == DX ? 0 : d == DZ ? 1 : 2, cy = d == DY ? 0 : 2;
-  return Face1{F.q[R][cz] + idx, F.q[R][cx] + idx, F.q[R][cy] + idx, stride, F.co, L, dl};
-}
-
-// PML round R (pml1 for the z, x, y components in turn: own dimension unscaled, then
-// the cross dimensions scaled; pml1_all's order) of the thread's 4 cells; hz / hx / hy
-// say which faces hold them.  Loads first, then the recursions, then the stores.
-template <int R>
-__device__ __forceinline__ void pml1_4(const Face1 &fz, const Face1 &fx, const Face1 &fy, bool hz, bool hx, bool hy,
-                                       bool cross, bool ycross, bool do_y, float (&pz)[4], float (&px)[4],
-                                       float (&py)[4]) {
-  const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 zz = z4, zx = z4, zy = z4, xz = z4, xx = z4, xy = z4, yz = z4, yx = z4, yy = z4;  // [face][component]
-  const bool zyc = do_y && ycross;
-  if (hz) {
-    zz = ld4(fz.zc);
-    if (cross) zx = ld4(fz.xc);
-    if (zyc) zy = ld4(fz.yc);
+// PML round R of a tile's cells: pml1 of the three derivative components.
+template <int R, int TX, bool CROSS>
+struct TilePml : TileFaces<R> {
+  using TileFaces<R>::fx;
+  using TileFaces<R>::fz;
+  __device__ __forceinline__ void ahead(const PmlDev &P, const Grid3 &g, int ix, int iz4, int y, int k) const {
+    this->template prefetch<CROSS ? 3 : 1>(P, g, ix, iz4, y, k, P.f[DX][0].cs, P.f[DY][0].cs, P.f[DZ][0].cs);
   }
-  if (hx) {
-    xx = ld4(fx.xc);
-    if (cross) xz = ld4(fx.zc);
-    if (zyc) xy = ld4(fx.yc);
-  }
-  if (hy) {
-    if (do_y) yy = ld4(fy.yc);
-    if (cross) yz = ld4(fy.zc), yx = ld4(fy.xc);
-  }
-  const float *cox = fx.co + fx.L * 6, *coy = fy.co + fy.L * 6;
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    const float *coz = fz.co + (fz.L + c * fz.dl) * 6;
-    float m;
-    if (hz) m = cmp4(zz, c), pml_round(coz, pz[c], &m), set4(zz, c, m);
-    if (cross) {
-      if (hx) m = cmp4(xz, c), pml_round(cox + 3, pz[c], &m), set4(xz, c, m);
-      if (hy) m = cmp4(yz, c), pml_round(coy + 3, pz[c], &m), set4(yz, c, m);
-    }
-    if (hx) m = cmp4(xx, c), pml_round(cox, px[c], &m), set4(xx, c, m);
-    if (cross) {
-      if (hz) m = cmp4(zx, c), pml_round(coz + 3, px[c], &m), set4(zx, c, m);
-      if (hy) m = cmp4(yx, c), pml_round(coy + 3, px[c], &m), set4(yx, c, m);
-    }
+  // pml1 of the z, x and y components in turn (own dimension unscaled, then the
+  // cross dimensions scaled: pml1_all's order), component by component so that
+  // at most two components' memory is held: the next one's loads are issued
+  // before a component's recursions.  Memory component k of a face belongs to
+  // the derivative component: z faces z x y, x faces x z y, y faces y z x.
+  __device__ __forceinline__ void apply(const PmlCo<TX, 6> &s, const PmlDev &P, const Grid3 &g, int tzq, int tx, int ix,
+                                        int iz4, int iy, bool do_y, float (&pz)[4], float (&px)[4],
+                                        float (&py)[4]) const {
+    const float *coy = nullptr;
+    float *fy = this->yface(P, g, ix, iz4, iy, coy);
+    if (!fx && !fz && !fy) return;
+    const long long cx = P.f[DX][0].cs, cz = P.f[DZ][0].cs, cy = P.f[DY][0].cs;
+    float4 zz, xz, yz, xx, zx, yx, yy, zy, xy;  // [face][component]
+    if (fz) zz = ld4(fz);
+    if (CROSS && fx) xz = ld4(fx + cx);
+    if (CROSS && fy) yz = ld4(fy + cy);
+    if (fx) xx = ld4(fx);
+    if (CROSS && fz) zx = ld4(fz + cz);
+    if (CROSS && fy) yx = ld4(fy + 2 * cy);
+    if (fz) round4z(s.z, tzq, 0, pz, zz), st4(fz, zz);
+    if (CROSS && fx) round4(&s.x[tx][3], pz, xz), st4(fx + cx, xz);
+    if (CROSS && fy) round4(coy + 3, pz, yz), st4(fy + cy, yz);
     if (do_y) {
-      if (hy) m = cmp4(yy, c), pml_round(coy, py[c], &m), set4(yy, c, m);
-      if (ycross) {
-        if (hz) m = cmp4(zy, c), pml_round(coz + 3, py[c], &m), set4(zy, c, m);
-        if (hx) m = cmp4(xy, c), pml_round(cox + 3, py[c], &m), set4(xy, c, m);
-      }
+      if (fy) yy = ld4(fy);
+      if (CROSS && fz) zy = ld4(fz + 2 * cz);
+      if (CROSS && fx) xy = ld4(fx + 2 * cx);
     }
-  }
-  if (hz) {
-    st4(fz.zc, zz);
-    if (cross) st4(fz.xc, zx);
-    if (zyc) st4(fz.yc, zy);
-  }
-  if (hx) {
-    st4(fx.xc, xx);
-    if (cross) st4(fx.zc, xz);
-    if (zyc) st4(fx.yc, xy);
-  }
-  if (hy) {
-    if (do_y) st4(fy.yc, yy);
-    if (cross) st4(fy.zc, yz), st4(fy.xc, yx);
-  }
-}
-
-// Per-thread PML state of a tile marching y from y0: the x and z faces of the thread's
-// cells (fixed over the planes; z faces a multiple of 4 cells wide) and the y face of a
-// plane.
-template <int R>
-struct TilePml {
-  Face1 fx{}, fz{};
-  bool hx = false, hz = false;
-  __device__ __forceinline__ void init(const PmlDev &P, const Grid3 &g, int ix, int iz4, int y0, bool act) {
-    const int nx = g.nx, nz = g.nz;
-    if (act && (ix < P.f[DX][0].w || ix >= nx - P.f[DX][1].w)) {
-      const int s = ix < P.f[DX][0].w ? 0 : 1;
-      const PmlFace &F = P.f[DX][s];
-      const int w = F.w;
-      const long long idx = ((long long)y0 * w + (s ? ix - (nx - w) : ix)) * nz + iz4;
-      fx = face1<R>(F, DX, idx, (long long)w * nz, s ? nx - 1 - ix : ix, 0);
-      hx = true;
-    }
-    if (act && (iz4 < P.f[DZ][0].w || iz4 >= nz - P.f[DZ][1].w)) {
-      const int s = iz4 < P.f[DZ][0].w ? 0 : 1;
-      const PmlFace &F = P.f[DZ][s];
-      const int w = F.w;
-      const long long idx = ((long long)y0 * nx + ix) * w + (s ? iz4 - (nz - w) : iz4);
-      fz = face1<R>(F, DZ, idx, (long long)nx * w, s ? nz - 1 - iz4 : iz4, s ? -1 : 1);
-      hz = true;
-    }
-  }
-  // the y face holding plane iy (hy = false when none)
-  __device__ __forceinline__ Face1 yface(const PmlDev &P, const Grid3 &g, int ix, int iz4, int iy, bool &hy) const {
-    hy = iy < P.f[DY][0].w || iy >= g.ny - P.f[DY][1].w;
-    if (!hy) return Face1{};
-    const int s = iy < P.f[DY][0].w ? 0 : 1;
-    const PmlFace &F = P.f[DY][s];
-    const long long idx = ((long long)(s ? iy - (g.ny - F.w) : iy) * g.nx + ix) * g.nz + iz4;
-    return face1<R>(F, DY, idx, 0, s ? g.ny - 1 - iy : iy, 0);
-  }
-  __device__ __forceinline__ void advance() {
-    if (hx) fx.zc += fx.stride, fx.xc += fx.stride, fx.yc += fx.stride;
-    if (hz) fz.zc += fz.stride, fz.xc += fz.stride, fz.yc += fz.stride;
-  }
-  // L1 prefetch of the x / z face memory k planes ahead and of the y face of plane y
-  __device__ __forceinline__ void prefetch(const PmlDev &P, const Grid3 &g, int ix, int iz4, int y, int k,
-                                           bool cross, bool yc) const {
-    auto pf = [](const float *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(p))); };
-    if (hx) {
-      pf(fx.xc + k * fx.stride);
-      if (cross) pf(fx.zc + k * fx.stride);
-      if (yc) pf(fx.yc + k * fx.stride);
-    }
-    if (hz) {
-      pf(fz.zc + k * fz.stride);
-      if (cross) pf(fz.xc + k * fz.stride);
-      if (yc) pf(fz.yc + k * fz.stride);
-    }
-    bool hy;
-    const Face1 fy = yface(P, g, ix, iz4, y, hy);
-    if (hy) {
-      pf(fy.yc);
-      if (cross) pf(fy.zc), pf(fy.xc);
+    if (fx) round4(s.x[tx], px, xx), st4(fx, xx);
+    if (CROSS && fz) round4z(s.z, tzq, 3, px, zx), st4(fz + cz, zx);
+    if (CROSS && fy) round4(coy + 3, px, yx), st4(fy + 2 * cy, yx);
+    if (do_y) {
+      if (fy) round4(coy, py, yy), st4(fy, yy);
+      if (CROSS && fz) round4z(s.z, tzq, 3, py, zy), st4(fz + 2 * cz, zy);
+      if (CROSS && fx) round4(&s.x[tx][3], py, xy), st4(fx + 2 * cx, xy);
     }
   }
 };
+
+// Tiles by PML content: none, faces without cross terms (pml3d off), all
+enum { TILE_INT = 0, TILE_PML1 = 1, TILE_PML3 = 2 };
+// resident PML tiles per SM the register allocation aims at
+constexpr int kEdgeCtas = 4;
 
 // ---- pass 1: gradient -----------------------------------------------------------
 template <int TX, int P, int NM>
@@ -183,12 +82,13 @@ struct __align__(128) Grad4Smem {
   static constexpr int SB = P + 1;  // planes iy .. iy+P of the anisotropy parameters
   float4 a[SA][HX][10];
   float4 m[SB][NM][TX][8];
+  PmlCo<TX, 6> co;  // PML tiles
   uint64_t bar_a[SA];
   uint64_t bar_b[SB];
 };
 
-template <int TX, int P, int MODEL, bool EDGE>
-__global__ void __launch_bounds__(8 * TX, EDGE ? 384 / (8 * TX) : 0)
+template <int TX, int P, int MODEL, int EDGE>
+__global__ void __launch_bounds__(8 * TX, EDGE ? kEdgeCtas : 0)
     grad4_k(const __grid_constant__ GradArgs a, const Tile4 *__restrict__ tiles, const __grid_constant__ Grad4Maps mp,
             int *err) {
   constexpr int NM = MODEL == 3 ? 4 : MODEL == 2 ? 2 : 1;
@@ -207,9 +107,6 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? 384 / (8 * TX) : 0)
   const bool producer = tzq == 0 && tx == 0;
   const long long col = (long long)ix * nz + iz4;
   const bool do_y = ny > 1;
-  const bool cross = a.pml3d != 0, ycross = a.pml3d != 0 && ny > 1;
-  const int zl = a.pml.f[DZ][0].w, zh = a.pml.f[DZ][1].w;
-  const bool z4ok = zl % 4 == 0 && zh % 4 == 0;
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 
   auto issue_a = [&](int p) {
@@ -237,6 +134,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? 384 / (8 * TX) : 0)
     for (int k = 0; k < SB; k++) mbar_init(&s.bar_b[k], 1);
     mbar_fence_init();
   }
+  if constexpr (EDGE != 0) fill_pml_co(s.co, a.pml, g, iz0, ix0, tzq, tx);
   __syncthreads();
   int last_a = y0 - 1, last_b = y0 - 1;  // last planes the producer issued
   if (producer) {
@@ -251,13 +149,11 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? 384 / (8 * TX) : 0)
     const int y = y0 - R4 + k;
     q[k] = act && y >= 0 && y < ny ? __ldg(w1g + y * nxz4 + col4) : zero4;
   }
-  TilePml<0> pm;
-  if constexpr (EDGE) {
-    if (z4ok) {
-      pm.init(a.pml, g, ix, iz4, y0, act);
-      if (act)
-        for (int y = y0; y < min(y0 + 2, y1); y++) pm.prefetch(a.pml, g, ix, iz4, y, y - y0, cross, do_y && ycross);
-    }
+  TilePml<0, TX, EDGE == TILE_PML3> pm;
+  if constexpr (EDGE != 0) {
+    pm.init(a.pml, g, ix, iz4, y0, act);
+    if (act)
+      for (int y = y0; y < min(y0 + 2, y1); y++) pm.ahead(a.pml, g, ix, iz4, y, y - y0);
   }
   bool ok = true;
 #pragma unroll 1
@@ -266,8 +162,8 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? 384 / (8 * TX) : 0)
       if (iy + R4 + P < y1 + R4) issue_a(iy + R4 + P), last_a = iy + R4 + P;
       if (iy + P < y1) issue_b(iy + P), last_b = iy + P;
     }
-    if constexpr (EDGE) {
-      if (z4ok && act && iy + 2 < y1) pm.prefetch(a.pml, g, ix, iz4, iy + 2, 2, cross, do_y && ycross);
+    if constexpr (EDGE != 0) {
+      if (act && iy + 2 < y1) pm.ahead(a.pml, g, ix, iz4, iy + 2, 2);
     }
     const int r0 = iy - y0, sa0 = r0 % SA, sa4 = (r0 + R4) % SA, sb = r0 % SB;
     if (r0 < R4) ok = ok && mbar_wait(&s.bar_a[sa0], (uint32_t)((r0 / SA) & 1), err);
@@ -291,18 +187,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? 384 / (8 * TX) : 0)
       }
       const long long i0 = (long long)iy * g.nxz + col;
       if (a.io.store | a.io.ic) fused_io4(a.io, g, i0, ix, iy, iz4, col, u4);
-      if constexpr (EDGE) {
-        if (z4ok) {
-          bool hy;
-          const Face1 fy = pm.yface(a.pml, g, ix, iz4, iy, hy);
-          if (pm.hx || pm.hz || hy) pml1_4<0>(pm.fz, pm.fx, fy, pm.hz, pm.hx, hy, cross, ycross, do_y, gz, gx, gy);
-        } else {
-#pragma unroll
-          for (int c = 0; c < 4; c++)
-            if (in_pml(a.pml, g, ix, iy, iz4 + c))
-              pml1_all<0>(a.pml, g, a.pml3d, do_y, ix, iy, iz4 + c, gz[c], gx[c], gy[c]);
-        }
-      }
+      if constexpr (EDGE != 0) pm.apply(s.co, a.pml, g, tzq, tx, ix, iz4, iy, do_y, gz, gx, gy);
       if (MODEL == 2 || MODEL == 3) {
         float4 mv[4];
 #pragma unroll
@@ -318,7 +203,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? 384 / (8 * TX) : 0)
       st4(a.pz + i0, make_float4(gz[0], gz[1], gz[2], gz[3]));
       if (do_y) st4(a.py + i0, make_float4(gy[0], gy[1], gy[2], gy[3]));
     }
-    if constexpr (EDGE) pm.advance();
+    if constexpr (EDGE != 0) pm.advance();
     __syncthreads();  // every thread is done with the stages the producer refills next
 #pragma unroll
     for (int k = 0; k < 2 * R4; k++) q[k] = q[k + 1];
@@ -341,6 +226,7 @@ struct __align__(128) Div4Smem {
   float4 px[SB][TX + 2 * R4][8];
   float4 pz[SB][TX][10];
   float4 w[SB][3][TX][8];  // w0, (v dt)^2, w1
+  PmlCo<TX, 6> co;         // PML tiles
   uint64_t bar_a[SA];
   uint64_t bar_b[SB];
 };
@@ -364,8 +250,8 @@ constexpr size_t div4_smem() {
 
 // QR: 0 the Q update loads its own operands; 1 / 2 ring B also carries the Q
 // memory (FP32 / BF16) and 1/Q of its planes (MODE 2, order <= kDiv4QMax)
-template <int TX, int P, int MODE, bool EDGE, int QR>
-__global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 384 / (8 * TX) : 0)
+template <int TX, int P, int MODE, int EDGE, int QR>
+__global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? kEdgeCtas : 0)
     div4_k(const __grid_constant__ DivArgs a, const Tile4 *__restrict__ tiles, const __grid_constant__ Div4Maps mp,
            int *err) {
   using S = Div4Smem<TX, P>;
@@ -387,9 +273,6 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 384 / (8 * TX) : 0
   const bool producer = tzq == 0 && tx == 0;
   const long long col = (long long)ix * nz + iz4;
   const bool do_y = ny > 1;
-  const bool cross = a.pml3d != 0, ycross = a.pml3d != 0 && ny > 1;
-  const int zl = a.pml.f[DZ][0].w, zh = a.pml.f[DZ][1].w;
-  const bool z4ok = zl % 4 == 0 && zh % 4 == 0;
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
 
   // ring-A plane p (>= y0 + 4) lives in stage (p - y0 - 4) % SA, phase ((p - y0 - 4) / SA) & 1
@@ -422,6 +305,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 384 / (8 * TX) : 0
     for (int k = 0; k < SB; k++) mbar_init(&s.bar_b[k], 1);
     mbar_fence_init();
   }
+  if constexpr (EDGE != 0) fill_pml_co(s.co, a.pml, g, iz0, ix0, tzq, tx);
   __syncthreads();
   // ring A carries planes y0+4 .. y1+3 only (the queue starts with planes
   // y0-4 .. y0+3 read from global memory), so every copy it gets is waited for
@@ -438,13 +322,11 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 384 / (8 * TX) : 0
     const int y = y0 - R4 + k;
     q[k] = do_y && act && y >= 0 && y < ny ? __ldg(pyg + y * nxz4 + col4) : zero4;
   }
-  TilePml<1> pm;
-  if constexpr (EDGE) {
-    if (z4ok) {
-      pm.init(a.pml, g, ix, iz4, y0, act);
-      if (act)
-        for (int y = y0; y < min(y0 + 2, y1); y++) pm.prefetch(a.pml, g, ix, iz4, y, y - y0, cross, do_y && ycross);
-    }
+  TilePml<1, TX, EDGE == TILE_PML3> pm;
+  if constexpr (EDGE != 0) {
+    pm.init(a.pml, g, ix, iz4, y0, act);
+    if (act)
+      for (int y = y0; y < min(y0 + 2, y1); y++) pm.ahead(a.pml, g, ix, iz4, y, y - y0);
   }
   bool ok = true;
 #pragma unroll 1
@@ -453,8 +335,8 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 384 / (8 * TX) : 0
       if (iy + R4 + P < y1 + R4) issue_a(iy + R4 + P), last_a = iy + R4 + P;
       if (iy + P < y1) issue_b(iy + P), last_b = iy + P;
     }
-    if constexpr (EDGE) {
-      if (z4ok && act && iy + 2 < y1) pm.prefetch(a.pml, g, ix, iz4, iy + 2, 2, cross, do_y && ycross);
+    if constexpr (EDGE != 0) {
+      if (act && iy + 2 < y1) pm.ahead(a.pml, g, ix, iz4, iy + 2, 2);
     }
     const int r0 = iy - y0, sa4 = r0 % SA, sb = r0 % SB;
     ok = ok && mbar_wait(&s.bar_a[sa4], (uint32_t)((r0 / SA) & 1), err);
@@ -475,18 +357,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 384 / (8 * TX) : 0
         }
       }
       const long long i0 = (long long)iy * g.nxz + col;
-      if constexpr (EDGE) {
-        if (z4ok) {
-          bool hy;
-          const Face1 fy = pm.yface(a.pml, g, ix, iz4, iy, hy);
-          if (pm.hx || pm.hz || hy) pml1_4<1>(pm.fz, pm.fx, fy, pm.hz, pm.hx, hy, cross, ycross, do_y, dz, dx, dy);
-        } else {
-#pragma unroll
-          for (int c = 0; c < 4; c++)
-            if (in_pml(a.pml, g, ix, iy, iz4 + c))
-              pml1_all<1>(a.pml, g, a.pml3d, do_y, ix, iy, iz4 + c, dz[c], dx[c], dy[c]);
-        }
-      }
+      if constexpr (EDGE != 0) pm.apply(s.co, a.pml, g, tzq, tx, ix, iz4, iy, do_y, dz, dx, dy);
       const float4 cw0 = s.w[sb][0][tx][tzq], cvel = s.w[sb][1][tx][tzq], cw1 = s.w[sb][2][tx][tzq];
       float4 t4, out4;
 #pragma unroll
@@ -505,7 +376,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 384 / (8 * TX) : 0
       }
       st4(a.w0 + i0, out4);
     }
-    if constexpr (EDGE) pm.advance();
+    if constexpr (EDGE != 0) pm.advance();
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 2 * R4; k++) q[k] = q[k + 1];
@@ -523,12 +394,12 @@ size_t grad4_smem() {
   return sizeof(Grad4Smem<TX, P, MODEL == 3 ? 4 : MODEL == 2 ? 2 : 1>);
 }
 
-template <int TX, int P, int MODEL, bool EDGE>
+template <int TX, int P, int MODEL, int EDGE>
 bool grad4_attr1() {
   return cudaFuncSetAttribute(grad4_k<TX, P, MODEL, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)grad4_smem<TX, P, MODEL>()) == cudaSuccess;
 }
-template <int TX, int P, int MODE, bool EDGE, int QR = 0>
+template <int TX, int P, int MODE, int EDGE, int QR = 0>
 bool div4_attr1() {
   return cudaFuncSetAttribute(div4_k<TX, P, MODE, EDGE, QR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)div4_smem<TX, P, QR>()) == cudaSuccess;
@@ -538,21 +409,20 @@ constexpr int kTX = kAniso4TX, kP = 2;
 
 }  // namespace
 
-bool aniso4_init() {
-  bool ok = true;
-  ok &= grad4_attr1<kTX, kP, 2, false>() && grad4_attr1<kTX, kP, 2, true>();
-  ok &= grad4_attr1<kTX, kP, 3, false>() && grad4_attr1<kTX, kP, 3, true>();
-  ok &= div4_attr1<kTX, kP, 0, false>() && div4_attr1<kTX, kP, 0, true>();
-  ok &= div4_attr1<kTX, kP, 1, false>() && div4_attr1<kTX, kP, 1, true>();
-  ok &= div4_attr1<kTX, kP, 2, false>() && div4_attr1<kTX, kP, 2, true>();
-  ok &= div4_attr1<kTX, kP, 2, false, 1>() && div4_attr1<kTX, kP, 2, true, 1>();
-  ok &= div4_attr1<kTX, kP, 2, false, 2>() && div4_attr1<kTX, kP, 2, true, 2>();
-  return ok;
+namespace {
+template <int EDGE>
+bool aniso4_attr() {
+  return grad4_attr1<kTX, kP, 2, EDGE>() && grad4_attr1<kTX, kP, 3, EDGE>() && div4_attr1<kTX, kP, 0, EDGE>() &&
+         div4_attr1<kTX, kP, 1, EDGE>() && div4_attr1<kTX, kP, 2, EDGE>() && div4_attr1<kTX, kP, 2, EDGE, 1>() &&
+         div4_attr1<kTX, kP, 2, EDGE, 2>();
 }
+}  // namespace
+
+bool aniso4_init() { return aniso4_attr<TILE_INT>() && aniso4_attr<TILE_PML1>() && aniso4_attr<TILE_PML3>(); }
 
 int aniso4_ctas_per_sm() {
   int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, div4_k<kTX, kP, 1, false, 0>, 8 * kTX, div4_smem<kTX, kP, 0>());
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, div4_k<kTX, kP, 1, TILE_INT, 0>, 8 * kTX, div4_smem<kTX, kP, 0>());
   return n > 0 ? n : 1;
 }
 
@@ -560,14 +430,18 @@ void launch_grad4(const GradArgs &a, const Tile4 *tiles, int ntiles, bool edge, 
                   int *err, cudaStream_t st) {
   if (ntiles <= 0) return;
   const dim3 block(8, kTX);
+  const int e = !edge ? TILE_INT : a.pml3d ? TILE_PML3 : TILE_PML1;
 #define G_(MD, E) grad4_k<kTX, kP, MD, E><<<ntiles, block, grad4_smem<kTX, kP, MD>(), st>>>(a, tiles, m, err)
+#define E_(MD)                          \
+  if (e == TILE_INT) G_(MD, TILE_INT);  \
+  else if (e == TILE_PML1) G_(MD, TILE_PML1); \
+  else G_(MD, TILE_PML3)
   if (model == 3) {
-    if (edge) G_(3, true);
-    else G_(3, false);
+    E_(3);
   } else {
-    if (edge) G_(2, true);
-    else G_(2, false);
+    E_(2);
   }
+#undef E_
 #undef G_
 }
 
@@ -575,23 +449,24 @@ void launch_div4(const DivArgs &a, const Tile4 *tiles, int ntiles, bool edge, in
                  cudaStream_t st) {
   if (ntiles <= 0) return;
   const dim3 block(8, kTX);
+  const int e = !edge ? TILE_INT : a.pml3d ? TILE_PML3 : TILE_PML1;
 #define D_(MD, E, QR) div4_k<kTX, kP, MD, E, QR><<<ntiles, block, div4_smem<kTX, kP, QR>(), st>>>(a, tiles, m, err)
+#define E_(MD, QR)                              \
+  if (e == TILE_INT) D_(MD, TILE_INT, QR);      \
+  else if (e == TILE_PML1) D_(MD, TILE_PML1, QR); \
+  else D_(MD, TILE_PML3, QR)
   if (mode == 0) {
-    if (edge) D_(0, true, 0);
-    else D_(0, false, 0);
+    E_(0, 0);
   } else if (mode == 1) {
-    if (edge) D_(1, true, 0);
-    else D_(1, false, 0);
+    E_(1, 0);
   } else if (m.qring == 1) {
-    if (edge) D_(2, true, 1);
-    else D_(2, false, 1);
+    E_(2, 1);
   } else if (m.qring == 2) {
-    if (edge) D_(2, true, 2);
-    else D_(2, false, 2);
+    E_(2, 2);
   } else {
-    if (edge) D_(2, true, 0);
-    else D_(2, false, 0);
+    E_(2, 0);
   }
+#undef E_
 #undef D_
 }
 

@@ -18,7 +18,7 @@
 #include <type_traits>
 
 #include "kernel_api.h"
-#include "rtm_device.cuh"
+#include "pml4.cuh"
 #include "tma.cuh"
 
 namespace rtm {
@@ -306,26 +306,16 @@ struct __align__(128) Iso4Smem {
   float4 a[SA][HX][10];
   float4 w0[SB][TX][8];
   float4 vel[SB][TX][8];
+  PmlCo<TX, 3> co;  // PML tiles
   uint64_t bar_a[SA];
   uint64_t bar_b[SB];
 };
 
-__device__ __forceinline__ void prefetch_l1(const void *p) {
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(p)));
-}
-
-// L1 prefetch of the per-cell operands besides the stencil input that the
-// thread's 4 cells of plane iy read: PML face memory, Q variables, imaging
-// condition (image, compensation, source snapshot)
+// L1 prefetch of the operands besides the stencil input and the PML memory
+// that the thread's 4 cells of plane iy read: Q variables, imaging condition
+// (image, compensation, source snapshot)
 template <int MODE>
-__device__ __forceinline__ void iso4_prefetch(const IsoArgs &a, const Grid3 &g, bool pml, int ix, int iy, int iz4,
-                                              long long col) {
-  if (pml)
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      const Face4 f = face4(a.pml, g, d, ix, iy, iz4);
-      if (f.q1) prefetch_l1(f.q1), prefetch_l1(f.q2);
-    }
+__device__ __forceinline__ void iso4_prefetch(const IsoArgs &a, const Grid3 &g, int iy, long long col) {
   const long long i = (long long)iy * g.nxz + col;
   if (MODE == 2) {
     const long long n = (long long)g.ny * g.nxz;
@@ -366,64 +356,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
   const bool producer = tzq == 0 && tx == 0;
   const long long col = (long long)ix * nz + iz4;
   const bool do_y = ny > 2;
-  const int zl = a.pml.f[DZ][0].w, zh = a.pml.f[DZ][1].w, xl = a.pml.f[DX][0].w, xh = a.pml.f[DX][1].w,
-            yl = a.pml.f[DY][0].w, yh = a.pml.f[DY][1].w;
-  // interior tiles hold no PML cell (the tile table guarantees it)
-  const bool x_edge = EDGE && (ix < xl || ix >= nx - xh);
-  const bool z_edge = EDGE && (iz4 < zl || iz4 + 3 >= nz - zh);
-  const bool z4ok = zl % 4 == 0 && zh % 4 == 0;
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto y_edge_at = [&](int y) { return EDGE && (y < yl || y >= ny - yh); };
-  // PML tiles with z faces a multiple of 4 cells wide: the x and z faces of
-  // the thread's 4 cells are fixed over the tile's planes; their round-0 /
-  // round-1 memory (one float4 per array, z fastest) advances by a constant
-  // stride per plane and their recursion constants stay in registers
-  const bool vpml = EDGE && z4ok;
-  float *qx1 = nullptr, *qx2 = nullptr, *qz1 = nullptr, *qz2 = nullptr;
-  long long stx = 0, stz = 0;
-  float cx[3] = {0.f, 0.f, 0.f}, cz[4][3] = {};
-  if (vpml && act && x_edge) {
-    const int sd = ix < xl ? 0 : 1;
-    const PmlFace &F = a.pml.f[DX][sd];
-    const int w = F.w, L = sd ? nx - 1 - ix : ix;
-    const long long idx = ((long long)y0 * w + (sd ? ix - (nx - w) : ix)) * nz + iz4;
-    qx1 = F.q[0][0] + idx, qx2 = F.q[1][0] + idx, stx = (long long)w * nz;
-#pragma unroll
-    for (int k = 0; k < 3; k++) cx[k] = F.co[L * 6 + k];
-  }
-  if (vpml && act && z_edge) {
-    const int sd = iz4 < zl ? 0 : 1;
-    const PmlFace &F = a.pml.f[DZ][sd];
-    const int w = F.w;
-    const long long idx = ((long long)y0 * nx + ix) * w + (sd ? iz4 - (nz - w) : iz4);
-    qz1 = F.q[0][0] + idx, qz2 = F.q[1][0] + idx, stz = (long long)nx * w;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int L = sd ? nz - 1 - (iz4 + c) : iz4 + c;
-#pragma unroll
-      for (int k = 0; k < 3; k++) cz[c][k] = F.co[L * 6 + k];
-    }
-  }
-  // the y face of plane y (memory of the thread's cells, recursion constants)
-  auto yface = [&](int y, float *&q1, float *&q2, const float *&co) {
-    const int sd = y < yl ? 0 : 1;
-    const PmlFace &F = a.pml.f[DY][sd];
-    const long long idx = ((long long)(sd ? y - (ny - F.w) : y) * nx + ix) * nz + iz4;
-    q1 = F.q[0][0] + idx, q2 = F.q[1][0] + idx, co = F.co + (sd ? ny - 1 - y : y) * 6;
-  };
-  // L1 prefetch of the face memory of plane y, k planes beyond the one the
-  // x / z pointers are at
-  auto pml_prefetch = [&](int y, int k) {
-    if (qx1) prefetch_l1(qx1 + k * stx), prefetch_l1(qx2 + k * stx);
-    if (qz1) prefetch_l1(qz1 + k * stz), prefetch_l1(qz2 + k * stz);
-    if ((PML3D || do_y) && y_edge_at(y)) {
-      float *q1, *q2;
-      const float *co;
-      yface(y, q1, q2, co);
-      prefetch_l1(q1), prefetch_l1(q2);
-    }
-  };
-
   // plane p (y0 <= p) lives in stage (p - y0) % S of its ring, phase ((p - y0) / S) & 1
   auto issue_a = [&](int p) {
     const int st = (p - y0) % SA;
@@ -446,6 +379,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
     for (int k = 0; k < SB; k++) mbar_init(&s.bar_b[k], 1);
     mbar_fence_init();
   }
+  if constexpr (EDGE) fill_pml_co(s.co, a.pml, g, iz0, ix0, tzq, tx);
   __syncthreads();
   int last_a = y0 - 1, last_b = y0 - 1;  // last planes the producer issued
   if (producer) {
@@ -461,10 +395,14 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
     const int y = y0 - R4 + k;
     q[k] = act && y >= 0 && y < ny ? __ldg(w1g + y * nxz4 + col4) : zero4;
   }
+  // the round-1 memory of a face is one round stride (its component stride) on
+  TileFaces<0> pm;
+  const long long dx = a.pml.f[DX][0].cs, dy = a.pml.f[DY][0].cs, dz = a.pml.f[DZ][0].cs;
+  if constexpr (EDGE) pm.init(a.pml, g, ix, iz4, y0, act);
   if (act)
     for (int y = y0; y < min(y0 + 2, y1); y++) {
-      iso4_prefetch<MODE>(a, g, !vpml && (x_edge || z_edge || y_edge_at(y)), ix, y, iz4, col);
-      if (vpml) pml_prefetch(y, y - y0);
+      iso4_prefetch<MODE>(a, g, y, col);
+      if constexpr (EDGE) pm.prefetch<2>(a.pml, g, ix, iz4, y, y - y0, dx, dy, dz);
     }
   bool ok = true;
 #pragma unroll 1
@@ -474,28 +412,8 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
       if (iy + P < y1) issue_b(iy + P), last_b = iy + P;
     }
     if (act && iy + 2 < y1) {
-      iso4_prefetch<MODE>(a, g, !vpml && (x_edge || z_edge || y_edge_at(iy + 2)), ix, iy + 2, iz4, col);
-      if (vpml) pml_prefetch(iy + 2, 2);
-    }
-    // PML face memory of this plane, loaded before the waits and the stencil
-    // so that its latency overlaps them (PML tiles only)
-    const bool yf = (PML3D || do_y) && y_edge_at(iy);
-    float4 z1, z2, x1, x2, y1, y2;
-    float *qy1 = nullptr, *qy2 = nullptr;
-    float cy[3] = {0.f, 0.f, 0.f};
-    if constexpr (EDGE) {
-      if (vpml && act) {
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        z1 = z2 = x1 = x2 = y1 = y2 = z4;
-        if (qz1) z1 = *reinterpret_cast<const float4 *>(qz1), z2 = *reinterpret_cast<const float4 *>(qz2);
-        if (qx1) x1 = *reinterpret_cast<const float4 *>(qx1), x2 = *reinterpret_cast<const float4 *>(qx2);
-        if (yf) {
-          const float *cyp;
-          yface(iy, qy1, qy2, cyp);
-          y1 = *reinterpret_cast<const float4 *>(qy1), y2 = *reinterpret_cast<const float4 *>(qy2);
-          cy[0] = cyp[0], cy[1] = cyp[1], cy[2] = cyp[2];
-        }
-      }
+      iso4_prefetch<MODE>(a, g, iy + 2, col);
+      if constexpr (EDGE) pm.prefetch<2>(a.pml, g, ix, iz4, iy + 2, 2, dx, dy, dz);
     }
     const int r0 = iy - y0, sa0 = r0 % SA, sa4 = (r0 + R4) % SA, sb = r0 % SB;
     if (r0 < R4) ok = ok && mbar_wait(&s.bar_a[sa0], (uint32_t)((r0 / SA) & 1), err);
@@ -529,47 +447,34 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
         lyv[c] = ly;
       }
       float v[4];
-      const bool y_edge = y_edge_at(iy);
-      bool pml_done = false;
       if constexpr (EDGE) {
-        if (vpml && (qx1 || qz1 || yf)) {
-          // pml2_dim's rounds per cell in the order z, x, y
-          pml_done = true;
+        // pml2_dim's two rounds per face in the order z, x, y
+        const float *coy = nullptr;
+        float *fy = (PML3D || do_y) ? pm.yface(a.pml, g, ix, iz4, iy, coy) : nullptr;
+        float4 z1, z2, x1, x2, y1, y2;
+        if (pm.fz) z1 = ld4(pm.fz), z2 = ld4(pm.fz + dz);
+        if (pm.fx) x1 = ld4(pm.fx), x2 = ld4(pm.fx + dx);
+        if (fy) y1 = ld4(fy), y2 = ld4(fy + dy);
+        if (PML3D)
 #pragma unroll
-          for (int c = 0; c < 4; c++) {
-            float pz = PML3D ? lzv[c] + lxv[c] + lyv[c] : lzv[c], px = lxv[c], py = lyv[c];
-            float m;
-            if (qz1) {
-              m = comp(z1, c), pml_round(cz[c], pz, &m), setc(z1, c, m);
-              m = comp(z2, c), pml_round(cz[c], pz, &m), setc(z2, c, m);
-            }
-            float &pxr = PML3D ? pz : px;
-            if (qx1) {
-              m = comp(x1, c), pml_round(cx, pxr, &m), setc(x1, c, m);
-              m = comp(x2, c), pml_round(cx, pxr, &m), setc(x2, c, m);
-            }
-            float &pyr = PML3D ? pz : py;
-            if (yf) {
-              m = comp(y1, c), pml_round(cy, pyr, &m), setc(y1, c, m);
-              m = comp(y2, c), pml_round(cy, pyr, &m), setc(y2, c, m);
-            }
-            v[c] = PML3D ? pz : pz + px + py;
-          }
-          if (qz1) *reinterpret_cast<float4 *>(qz1) = z1, *reinterpret_cast<float4 *>(qz2) = z2;
-          if (qx1) *reinterpret_cast<float4 *>(qx1) = x1, *reinterpret_cast<float4 *>(qx2) = x2;
-          if (yf) *reinterpret_cast<float4 *>(qy1) = y1, *reinterpret_cast<float4 *>(qy2) = y2;
-        } else if (!z4ok && (x_edge || y_edge || z_edge)) {
-          pml_done = true;
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            const int iz = iz4 + c;
-            if (x_edge || y_edge || iz < zl || iz >= nz - zh)
-              v[c] = iso4_pml_cell<PML3D>(a.pml, g, lzv[c], lxv[c], lyv[c], do_y, ix, iy, iz);
-            else v[c] = lzv[c] + lxv[c] + lyv[c];
-          }
+          for (int c = 0; c < 4; c++) v[c] = lzv[c] + lxv[c] + lyv[c];
+        if (pm.fz) {
+          float(&p)[4] = PML3D ? v : lzv;
+          round4z(s.co.z, tzq, 0, p, z1), round4z(s.co.z, tzq, 0, p, z2);
+          st4(pm.fz, z1), st4(pm.fz + dz, z2);
+        }
+        if (pm.fx) {
+          float(&p)[4] = PML3D ? v : lxv;
+          round4(s.co.x[tx], p, x1), round4(s.co.x[tx], p, x2);
+          st4(pm.fx, x1), st4(pm.fx + dx, x2);
+        }
+        if (fy) {
+          float(&p)[4] = PML3D ? v : lyv;
+          round4(coy, p, y1), round4(coy, p, y2);
+          st4(fy, y1), st4(fy + dy, y2);
         }
       }
-      if (!pml_done)
+      if (!(EDGE && PML3D))
 #pragma unroll
         for (int c = 0; c < 4; c++) v[c] = lzv[c] + lxv[c] + lyv[c];
       const long long i0 = (long long)iy * g.nxz + col;
@@ -584,8 +489,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
       else out4 = q_update4(a.q, i0, (long long)ny * g.nxz, t4, u4);
       reinterpret_cast<float4 *>(a.w0)[i0 / 4] = out4;
     }
-    if (qx1) qx1 += stx, qx2 += stx;
-    if (qz1) qz1 += stz, qz2 += stz;
+    if constexpr (EDGE) pm.advance();
     __syncthreads();  // every thread is done with the stages the producer refills next
 #pragma unroll
     for (int k = 0; k < 2 * R4; k++) q[k] = q[k + 1];

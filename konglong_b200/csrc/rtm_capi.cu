@@ -527,29 +527,42 @@ static int setup_pml(Engine *h) {
   const double dd[3] = {h->d.dx, h->d.dy, h->d.dz};
   const bool second = h->lap_iso();
   const int ncomp = (!c.pml3d || second) ? 1 : 3;
-  for (int dim = 0; dim < 3; dim++)
+  for (int dim = 0; dim < 3; dim++) {
+    int w[2];
     for (int s = 0; s < 2; s++) {
-      PmlFace &F = h->pml.f[dim][s];
-      F = PmlFace{};
-      int w = c.nbnd[2 * dim + s];
-      bool on = w > 1 && !(dim == DZ && s == SIDE_LO && !c.top_pml);
-      if (!on) continue;
-      if (w * 2 > nn[dim] && !(nn[dim] == 1)) {
+      w[s] = c.nbnd[2 * dim + s];
+      if (w[s] <= 1 || (dim == DZ && s == SIDE_LO && !c.top_pml)) w[s] = 0;
+      if (w[s] * 2 > nn[dim] && !(nn[dim] == 1)) {
         h->err = "PML wider than half the grid";
         return RTM_ERR_ARG;
       }
+    }
+    int wp[2] = {w[0], w[1]};  // layers with the z faces' padding
+    if (dim == DZ && nn[dim] % 4 == 0) {
+      const int r[2] = {(w[0] + 3) / 4 * 4, (w[1] + 3) / 4 * 4};
+      if (r[0] + r[1] <= nn[dim]) wp[0] = r[0], wp[1] = r[1];
+    }
+    const long long plane = dim == DX ? (long long)h->d.ny * h->d.nz
+                                      : dim == DY ? (long long)h->d.nx * h->d.nz : (long long)h->d.nx * h->d.ny;
+    for (int s = 0; s < 2; s++) {
+      PmlFace &F = h->pml.f[dim][s];
+      F = PmlFace{};
+      F.cs = plane * std::max(wp[0], wp[1]);
+      if (!w[s]) continue;
       std::vector<float> co;
-      pml_profile(w, dd[dim], h->d.dt, c.vmax, c.pml_eps, c.pml3d_scaler, co);
+      pml_profile(w[s], dd[dim], h->d.dt, c.vmax, c.pml_eps, c.pml3d_scaler, co);
+      for (int L = w[s]; L < wp[s]; L++) co.insert(co.end(), {1.f, 0.f, 1.f, 1.f, 0.f, 1.f});
       float *dco;
       TRY(h->alloc(dco, co.size()));
       CK(cudaMemcpy(dco, co.data(), co.size() * 4, cudaMemcpyHostToDevice));
-      F.w = w;
+      F.w = wp[s];
       F.co = dco;
-      long long plane = dim == DX ? (long long)h->d.ny * h->d.nz
-                                  : dim == DY ? (long long)h->d.nx * h->d.nz : (long long)h->d.nx * h->d.ny;
+      float *q;
+      TRY(h->alloc(q, (size_t)F.cs * ncomp * 2));
       for (int r = 0; r < 2; r++)
-        for (int k = 0; k < ncomp; k++) TRY(h->alloc(F.q[r][k], (size_t)plane * w));
+        for (int k = 0; k < ncomp; k++) F.q[r][k] = q + (r * ncomp + k) * F.cs;
     }
+  }
   return RTM_OK;
 }
 
@@ -1666,17 +1679,19 @@ int rtm_create(const rtm_dims *d, const rtm_config *c, rtm_handle **out) {
   cudaMemcpy(h->one_z, one.data(), 4 * d->nz, cudaMemcpyHostToDevice);
   cudaMemcpy(h->taper_z, one.data(), 4 * d->nz, cudaMemcpyHostToDevice);
   choose_shape(h);
+  // the 4-cell TMA kernels read the z faces as whole float4s
+  const bool z4 = h->pml.f[DZ][0].w % 4 == 0 && h->pml.f[DZ][1].w % 4 == 0;
   h->use_tma = (c->kernel_variant == 0 || c->kernel_variant == 2) && tma_supported(d->nz) && iso_tma_init();
   if (h->lap_iso() && d->nz % 4 == 0 &&
       (c->kernel_variant == 0 || c->kernel_variant == 3 || c->kernel_variant == 4)) {
-    h->iso4 = c->kernel_variant != 4 && tma_supported(d->nz) && iso_tma4_init() ? 2 : 1;
+    h->iso4 = c->kernel_variant != 4 && z4 && tma_supported(d->nz) && iso_tma4_init() ? 2 : 1;
     h->v4_yseg = yseg_iso4(h);
     if (h->iso4 == 2 && (rc = iso4_tiles(h))) return fail(rc);
   }
   if (c->engine == RTM_ENGINE_FD8 && !h->lap_iso() && (rc = fd8_tiles(h))) return fail(rc);
   // the 4-cell passes carry no density term: a density model runs the one-cell passes
   if (c->engine == RTM_ENGINE_FD8 && !h->lap_iso() && !c->use_rho && !c->state_fp16 && d->nz % 4 == 0 &&
-      (c->kernel_variant == 0 || c->kernel_variant == 3 || c->kernel_variant == 7) && tma_supported(d->nz) &&
+      (c->kernel_variant == 0 || c->kernel_variant == 3 || c->kernel_variant == 7) && z4 && tma_supported(d->nz) &&
       aniso4_init()) {
     h->aniso4 = 1;
     h->an4_yseg = yseg_an4(h);

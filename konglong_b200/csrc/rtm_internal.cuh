@@ -20,8 +20,15 @@ enum { SIDE_LO = 0, SIDE_HI = 1 };
 // layer L counted from the outer edge, the recursion constants of
 // bgprtm/PML.cpp:126-134 for damping g (k = 0..2: (1-g)/(1+g), 2g/(1-g^2),
 // 1/(1-g)) and for g * pml3d_scaler (k = 3..5), built in FP64.
+// The z faces of a grid with nz % 4 == 0 are padded to a multiple of 4 layers
+// with undamped ones (constants 1, 0, 1: their memory stays zero and p passes
+// through), so that the 4-cell kernels read whole float4s for every PML width;
+// only where both padded faces do not fit nz are they left as they are.
+// The arrays follow each other, round 0's components then round 1's, cs floats
+// apart (the same on both sides).
 struct PmlFace {
   int w;            // layer count, 0 = no PML on this face
+  long long cs;     // array stride
   const float *co;  // [w][6]
   float *q[2][3];   // [round][component]
 };
