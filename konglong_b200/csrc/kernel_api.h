@@ -212,6 +212,12 @@ struct CfdPlanDev {
   // Toeplitz interior have converged in FP32; c0 > c1 when there is no such run
   int c0, c1;
   float lmc[4], buc[4], rdc;
+  // tile kernels: quads of rows [k0, k1) have constant factors as pivot rows in
+  // both recurrences (k0 == k1: none); tables by pivot row, zero-padded to a
+  // multiple of 4 rows: tl [.][4] the multipliers to the next four rows, tu [.][4]
+  // the upper-factor entries of the four rows before, tr [.] the reciprocal pivots
+  int k0, k1;
+  const float *tl, *tu, *tr;
   float a[60];  // copy of am, read from the kernel-parameter (constant) bank
   // segment-parallel solve: nseg segments of seglen rows (the last one takes
   // the remainder, >= 8 rows); [n][4] tables: hf = response of the forward
@@ -225,11 +231,14 @@ struct CfdPlanDev {
 int cfd_init();
 // TMA box of the x / y line kernels: nb boxes of R rows (R <= 256) per tile
 void cfd_tma_box(int n, int *R, int *nb);
-// raw derivative of `in` along axis (0 x, 1 y, 2 z) into `out` (no PML).  For
-// x / y, tensor maps of in / out with box (32, R, 1) / (32, 1, R) select the
-// TMA tile kernel (null: plain loads and stores); err receives wait timeouts.
-void launch_cfd_deriv(int axis, const CfdPlanDev &p, const float *in, float *out, int nx, int ny, int nz,
-                      const CUtensorMap *tin, const CUtensorMap *tout, int *err, cudaStream_t st);
+// raw derivative of `in` along axis (0 x, 1 y, 2 z) into `out` (no PML) by the
+// shared-memory tile kernels (kernels_cfd_tile.cu).  For x / y, tensor maps of
+// in / out with box (32, R, 1) / (32, 1, R) select TMA tile moves (null: plain
+// loads and stores); err receives wait timeouts.  False when a line does not
+// fit (nothing launched).
+bool cfd_tile_init();
+bool launch_cfd_tile(int axis, const CfdPlanDev &p, const float *in, float *out, int nx, int ny, int nz,
+                     const CUtensorMap *tin, const CUtensorMap *tout, int *err, cudaStream_t st);
 // x / y derivative by the register-streamed kernel (no shared memory)
 // pipelined persistent x / y line solves over TMA tiles (one CTA per SM, a
 // ring of tile buffers, right-hand side fused into the forward pass); false

@@ -2,21 +2,17 @@
 // sm_100a.  A derivative along one axis solves B f' = A f for every grid line:
 // the 11-point right-hand side (banmul_*, bgprtm/FdEngine_cfd.cpp:164-201,
 // 304-327), the forward elimination of the band LU and the back substitution
-// (banbks_*, bgprtm/FdEngine_cfd.cpp:203-302, 328-356).  A CTA stages 32 lines
-// in shared memory (one HBM read and one write per cell):
-//   phase 1  all four warps form the right-hand sides of a quarter of every
-//            line each, in place (embarrassingly parallel along the line);
-//   phase 2  one warp (lane = line) runs the two sequential recurrences in
-//            register chunks of 8 points: the chunk's operands are loaded
-//            together and the next chunk is prefetched, so the dependency
-//            chain is one FMA per point in elimination, FMA + multiply in
-//            back substitution.
+// (banbks_*, bgprtm/FdEngine_cfd.cpp:203-302, 328-356).  The default line solves
+// are the tile kernels of kernels_cfd_tile.cu; here are the other forms of
+// kernel_variant (register-streamed lines, the pipelined persistent ring, the z
+// solve carrying the epilogue, the segment-parallel pipeline) and the epilogues.
 // The PML / scaling / accumulation steps of FdEngine_cfd::d{x,y,z}1_2D and
 // KernelCPU::TTI run as pointwise epilogues afterwards.
 #include <type_traits>
 
 #include <algorithm>
 
+#include "cfd_rows.cuh"
 #include "kernel_api.h"
 #include "rtm_device.cuh"
 #include "tma.cuh"
@@ -29,39 +25,6 @@ constexpr int kChunk = 8;  // points per register chunk (both phases)
 // prefetch depth (chunks) of the streamed x / y kernel with 32- / 64-bit line
 // offsets: the deepest that fits 128 registers without spilling
 constexpr int kStreamD = 3, kStreamDWide = 2;
-
-// One right-hand-side row of the 11-band A with every rounding explicit, so
-// that each line kernel (staged, streamed, pipelined) gives the same bits:
-// interior rows sum_d a[54 + d] (x[i + d] - x[i - d]), d = 1 .. 5, and the
-// one-sided rows within 5 of a line end (banmul_dev_z_c,
-// bgprtm/FdEngine_cfd.cpp:304-327) accumulated in the reference order.
-struct RhsCoef {
-  float c1, c2, c3, c4, c5;
-};
-__device__ __forceinline__ float rhs_interior(const RhsCoef &c, float m5, float m4, float m3, float m2, float m1,
-                                              float p1, float p2, float p3, float p4, float p5) {
-  float t = __fmul_rn(c.c1, __fsub_rn(p1, m1));
-  t = __fmaf_rn(c.c2, __fsub_rn(p2, m2), t);
-  t = __fmaf_rn(c.c3, __fsub_rn(p3, m3), t);
-  t = __fmaf_rn(c.c4, __fsub_rn(p4, m4), t);
-  return __fmaf_rn(c.c5, __fsub_rn(p5, m5), t);
-}
-// row i < 5 from x[i - 5 + j], j = 0 .. 10 (x[j] here)
-__device__ __forceinline__ float rhs_low(const float (&a)[60], int i, const float *x) {
-  float v = 0.f;
-#pragma unroll
-  for (int j = 0; j < 11; j++)
-    if (j >= 5 - i) v = __fmaf_rn(a[j * 5 + i], x[j], v);
-  return v;
-}
-// row i = n - t, t = 1 .. 5, from x[i - 5 + j], j = 0 .. 10
-__device__ __forceinline__ float rhs_high(const float (&a)[60], int t, const float *x) {
-  float v = 0.f;
-#pragma unroll
-  for (int j = 0; j < 11; j++)
-    if (j < t + 5) v = __fmaf_rn(-a[t + 49 - 5 * j], x[j], v);
-  return v;
-}
 
 // Phase 1: right-hand sides of positions [p0, p1) of one line (element i at
 // L[i * S]), in place, C outputs per chunk from a window of C + 10 inputs
@@ -303,63 +266,6 @@ __device__ __forceinline__ void cfd_tile_compute(const CfdPlanDev &p, float *L, 
   if (warp == 0 && lane < nl) cfd_solve<S, kChunk>(p, L, n);
 }
 
-// 32 lines per CTA staged through shared memory; warp 0 walks the lines
-// (lane = line), all warps move data.  x / y lines (STRIDED): element i of
-// line l at base + l + i*es, smem [i][32]; z lines: line l at base + l*n + i,
-// smem [l][n+1] (bank-conflict free), filled by asynchronous 4-byte copies.
-// One HBM read and one write per cell.
-template <bool STRIDED>
-__global__ void __launch_bounds__(128) cfd_lines_k(CfdPlanDev p, const float *__restrict__ in, float *__restrict__ out,
-                                                   int nz, long long es, long long other_stride, int n_other,
-                                                   long long nlines) {
-  extern __shared__ float sm[];
-  const int n = p.n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  constexpr int U = 16;  // independent loads in flight per thread during staging
-  long long base;
-  int nl;
-  if (STRIDED) {
-    const int izc = blockIdx.x, o = blockIdx.y;
-    const int iz0 = izc * 32;
-    nl = min(32, nz - iz0);
-    base = (long long)o * other_stride + iz0;
-    // rows i of 32 lines: warp w stages rows w*U .. w*U+U-1, then every nw*U rows
-    for (int i0 = warp * U; i0 < n; i0 += nw * U) {
-      float v[U];
-#pragma unroll
-      for (int k = 0; k < U; k++) {
-        const int i = i0 + k;
-        v[k] = (i < n && lane < nl) ? __ldcg(in + base + lane + (long long)i * es) : 0.f;
-      }
-#pragma unroll
-      for (int k = 0; k < U; k++)
-        if (i0 + k < n) sm[(i0 + k) * 32 + lane] = v[k];
-    }
-  } else {
-    const long long l0 = (long long)blockIdx.x * 32;
-    nl = (int)min(32LL, nlines - l0);
-    base = l0 * n;
-    for (int l = warp; l < nl; l += nw) {
-      const float *src = in + base + (long long)l * n;
-      float *dst = sm + l * (n + 1);
-#pragma unroll 4
-      for (int i = lane; i < n; i += 32) cp_async4(dst + i, src + i);
-    }
-    cp_async_wait_all();
-  }
-  constexpr int S = STRIDED ? 32 : 1;
-  __syncthreads();
-  cfd_tile_compute<S>(p, STRIDED ? sm + lane : sm + lane * (n + 1), n, nl, lane, warp, nw);
-  __syncthreads();
-  if (STRIDED) {
-    for (int i = warp; i < n; i += nw)
-      if (lane < nl) __stcg(out + base + lane + (long long)i * es, sm[i * 32 + lane]);
-  } else {
-    for (int l = warp; l < nl; l += nw)
-      for (int i = lane; i < n; i += 32) __stcg(out + base + (long long)l * n + i, sm[l * (n + 1) + i]);
-  }
-}
-
 // x / y lines streamed through registers, no shared memory: lane = z line,
 // one warp per 32 z of one line set (element i of a line at X[i * es]).
 // Forward: the 11-point right-hand side (one-sided rows at both ends) fused
@@ -559,48 +465,6 @@ __global__ void __launch_bounds__(128, 4) cfd_stream_k(const CfdPlanDev p, const
         }
       }
     }
-  }
-}
-
-// x / y lines with TMA tile moves: the 32 (z) x n tile arrives as nb boxes of
-// R rows on one mbarrier and leaves as nb bulk tensor stores.  Rows past n in
-// the last box and z >= nz are zero-filled on load and clipped on store.
-// Shared memory: 128 B for the barrier, then the tile [nb*R][32].
-template <int AXIS>
-__global__ void __launch_bounds__(128) cfd_lines_tma_k(CfdPlanDev p, const __grid_constant__ CUtensorMap tin,
-                                                       const __grid_constant__ CUtensorMap tout, int nz, int R, int nb,
-                                                       int *err) {
-  extern __shared__ __align__(128) unsigned char smraw[];
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smraw);
-  float *sm = reinterpret_cast<float *>(smraw + 128);
-  const int n = p.n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int iz0 = blockIdx.x * 32, o = blockIdx.y;
-  const int nl = min(32, nz - iz0);
-  if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    mbar_expect_tx(bar, (uint32_t)nb * (uint32_t)R * 32u * 4u);
-    for (int b = 0; b < nb; b++) {
-      if (AXIS == DX) tma_load_3d(sm + (size_t)b * R * 32, &tin, bar, iz0, b * R, o);
-      else tma_load_3d(sm + (size_t)b * R * 32, &tin, bar, iz0, o, b * R);
-    }
-  }
-  const bool ok = __syncthreads_and(mbar_wait(bar, 0, err));
-  if (!ok) return;
-  cfd_tile_compute<32>(p, sm + lane, n, nl, lane, warp, nw);
-  fence_proxy_async();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int b = 0; b < nb; b++) {
-      if (AXIS == DX) tma_store_3d(&tout, sm + (size_t)b * R * 32, iz0, b * R, o);
-      else tma_store_3d(&tout, sm + (size_t)b * R * 32, iz0, o, b * R);
-    }
-    bulk_commit();
-    bulk_wait_read();
   }
 }
 
@@ -1019,30 +883,6 @@ void cfd_tma_box(int n, int *R, int *nb) {
   *R = (n + *nb - 1) / *nb;
 }
 
-void launch_cfd_deriv(int axis, const CfdPlanDev &p, const float *in, float *out, int nx, int ny, int nz,
-                      const CUtensorMap *tin, const CUtensorMap *tout, int *err, cudaStream_t st) {
-  const long long nxz = (long long)nx * nz;
-  if (axis == DZ) {
-    const long long nlines = (long long)nx * ny;
-    const size_t smem = (size_t)32 * (nz + 1) * sizeof(float);
-    cfd_lines_k<false><<<(unsigned)((nlines + 31) / 32), 128, smem, st>>>(p, in, out, nz, 1, 0, 0, nlines);
-    return;
-  }
-  const int n = axis == DX ? nx : ny;
-  dim3 grid((nz + 31) / 32, axis == DX ? ny : nx);
-  if (tin && tout) {
-    int R, nb;
-    cfd_tma_box(n, &R, &nb);
-    const size_t smem = 128 + (size_t)nb * R * 32 * sizeof(float);
-    if (axis == DX) cfd_lines_tma_k<DX><<<grid, 128, smem, st>>>(p, *tin, *tout, nz, R, nb, err);
-    else cfd_lines_tma_k<DY><<<grid, 128, smem, st>>>(p, *tin, *tout, nz, R, nb, err);
-    return;
-  }
-  const size_t smem = (size_t)32 * n * sizeof(float);
-  if (axis == DX) cfd_lines_k<true><<<grid, 128, smem, st>>>(p, in, out, nz, nz, nxz, ny, 0);
-  else cfd_lines_k<true><<<grid, 128, smem, st>>>(p, in, out, nz, nxz, nz, nx, 0);
-}
-
 static int g_cfd_sms = 0;  // SM count of the device cfd_init ran on
 
 bool launch_cfd_deriv_pipe(int axis, const CfdPlanDev &p, int nx, int ny, int nz, const CUtensorMap *tin,
@@ -1075,10 +915,7 @@ void launch_cfd_deriv_stream(int axis, const CfdPlanDev &p, const float *in, flo
 
 int cfd_init() {
   const int mx = 227 * 1024;
-  bool ok = cudaFuncSetAttribute(cfd_lines_k<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;
-  ok = ok && cudaFuncSetAttribute(cfd_lines_k<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;
-  ok = ok && cudaFuncSetAttribute(cfd_lines_tma_k<DX>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;
-  ok = ok && cudaFuncSetAttribute(cfd_lines_tma_k<DY>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;
+  bool ok = cfd_tile_init();
   ok = ok && cudaFuncSetAttribute(cfd_pipe_k<DX>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;
   ok = ok && cudaFuncSetAttribute(cfd_pipe_k<DY>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;
   ok = ok && cudaFuncSetAttribute(cfd_zgrad_k, cudaFuncAttributeMaxDynamicSharedMemorySize, mx) == cudaSuccess;

@@ -125,12 +125,6 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, uint32_t 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_u32(dst)),
-               "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
 
 // D_acc[m][j] = sum_k A[m][k] D[j][k] for the 128 m of this CTA (MODE 0: z
 // lines, MODE 1: x / y columns).  Bg holds D's TF32 parts pre-arranged per K

@@ -220,7 +220,7 @@ static int check_launch(Engine *h, const char *what) {
   if (e != cudaSuccess) return cuda_fail(e, what, h);
   if (h->fft_err) {
     h->fft_err = 0;
-    h->err = std::string(what) + ": cuFFT / cuBLAS execution failed";
+    h->err = std::string(what) + ": line operator (cuFFT / cuBLAS / compact FD) execution failed";
     return RTM_ERR_CUDA;
   }
   return RTM_OK;
@@ -517,8 +517,11 @@ static void cfd_deriv(Engine *h, int axis, int sgn, const float *in, float *out)
   if (tma && h->cfd_pipe &&
       launch_cfd_deriv_pipe(axis, h->cfd[axis][sgn], d.nx, d.ny, d.nz, &mi, &mo, h->dflag, h->st))
     return;
-  launch_cfd_deriv(axis, h->cfd[axis][sgn], in, out, d.nx, d.ny, d.nz, tma ? &mi : nullptr, tma ? &mo : nullptr,
-                   h->dflag, h->st);
+  if (!launch_cfd_tile(axis, h->cfd[axis][sgn], in, out, d.nx, d.ny, d.nz, tma ? &mi : nullptr, tma ? &mo : nullptr,
+                       h->dflag, h->st)) {
+    if (axis == DZ) h->fft_err = 1;  // a single z line exceeds shared memory
+    else launch_cfd_deriv_stream(axis, h->cfd[axis][sgn], in, out, d.nx, d.ny, d.nz, h->st);
+  }
 }
 
 static int setup_pml(Engine *h) {
@@ -1619,9 +1622,30 @@ int rtm_create(const rtm_dims *d, const rtm_config *c, rtm_handle **out) {
         cudaMemcpy(dbl, bl.data(), bl.size() * 4, cudaMemcpyHostToDevice);
         cudaMemcpy(dam, am.data(), am.size() * 4, cudaMemcpyHostToDevice);
         cudaMemcpy(drd, rd.data(), rd.size() * 4, cudaMemcpyHostToDevice);
-        CfdPlanDev pd{nn[a], dbu, dbl, dam, drd, dlm, 1, 0, {0, 0, 0, 0}, {0, 0, 0, 0}, 0.f, {}};
+        CfdPlanDev pd{};
+        pd.n = nn[a], pd.bu = dbu, pd.bl = dbl, pd.am = dam, pd.rdiag = drd, pd.lm = dlm;
         for (int k = 0; k < 60; k++) pd.a[k] = am[k];
         cfd_constant_run(nn[a], lm, bu, rd, pd);
+        {  // the tile kernels' factors by pivot row
+          const int n = nn[a], n4 = (n + 3) / 4 * 4;
+          pd.k0 = (pd.c0 + 4 + 3) / 4 * 4, pd.k1 = (pd.c1 - 3) / 4 * 4;
+          if (pd.c0 > pd.c1 || pd.k1 <= pd.k0) pd.k0 = pd.k1 = 0;
+          std::vector<float> tl(4 * (size_t)n4, 0.f), tu(4 * (size_t)n4, 0.f), tr(n4, 0.f);
+          for (int i = 0; i < n; i++) {
+            tr[i] = rd[i];
+            for (int k = 0; k < 4; k++) {
+              if (i + 1 + k < n) tl[(size_t)i * 4 + k] = bl[(size_t)i * 4 + k];
+              if (i - 1 - k >= 0) tu[(size_t)i * 4 + k] = bu[(size_t)(i - 1 - k) * 4 + k];
+            }
+          }
+          float *dtl, *dtu, *dtr;
+          if ((rc = h->alloc(dtl, tl.size())) || (rc = h->alloc(dtu, tu.size())) || (rc = h->alloc(dtr, tr.size())))
+            return fail(rc);
+          cudaMemcpy(dtl, tl.data(), tl.size() * 4, cudaMemcpyHostToDevice);
+          cudaMemcpy(dtu, tu.data(), tu.size() * 4, cudaMemcpyHostToDevice);
+          cudaMemcpy(dtr, tr.data(), tr.size() * 4, cudaMemcpyHostToDevice);
+          pd.tl = dtl, pd.tu = dtu, pd.tr = dtr;
+        }
         {  // segment layout and correction tables of the segment-parallel solve
           std::vector<float> hf, gb, hb;
           cfd_seg_layout(nn[a], pd.nseg, pd.seglen);
@@ -1710,7 +1734,7 @@ int rtm_create(const rtm_dims *d, const rtm_config *c, rtm_handle **out) {
                   d->ny <= cfd_seg_max_n(DY) && d->nz <= cfd_seg_max_n(DZ) && cfd_seg_init() == 0;
   h->cfd_zfuse = c->kernel_variant == 9;
   h->cfd_pipe = c->kernel_variant == 10;
-  if (c->kernel_variant == 0 || c->kernel_variant == 9 || c->kernel_variant == 10) h->cfd_xy = h->cfd_tma ? 1 : 0;
+  if (c->kernel_variant == 0 || c->kernel_variant == 9 || c->kernel_variant == 10) h->cfd_xy = h->cfd_tma ? 1 : 2;
   else if (c->kernel_variant == 5) h->cfd_xy = 0;
   else if (c->kernel_variant == 6 && h->cfd_seg_ok) h->cfd_xy = 4;
   else if (c->kernel_variant == 8 && h->cfd_seg_ok) h->cfd_xy = h->cfd_tma ? 3 : 4;
@@ -2616,7 +2640,7 @@ int rtm_autotune(rtm_handle *h, int steps, int *choice) {
       cands.push_back({0, 0, 0, h->tma_shape, h->tx, 4});
     }
     cands.push_back({0, 0, 0, h->tma_shape, h->tx, 0});
-    if (h->cfd_tma) cands.push_back({0, 0, 0, h->tma_shape, h->tx, 1});
+    cands.push_back({0, 0, 0, h->tma_shape, h->tx, h->cfd_tma ? 1 : 2});
   }
   if (cands.empty()) {
     if (choice) *choice = 0;
