@@ -234,11 +234,11 @@ void cfd_tma_box(int n, int *R, int *nb);
 // raw derivative of `in` along axis (0 x, 1 y, 2 z) into `out` (no PML) by the
 // shared-memory tile kernels (kernels_cfd_tile.cu).  For x / y, tensor maps of
 // in / out with box (32, R, 1) / (32, 1, R) select TMA tile moves (null: plain
-// loads and stores); err receives wait timeouts.  False when a line does not
-// fit (nothing launched).
+// loads and stores); sms: SMs of the device; err receives wait timeouts.  False
+// when a line does not fit (nothing launched).
 bool cfd_tile_init();
 bool launch_cfd_tile(int axis, const CfdPlanDev &p, const float *in, float *out, int nx, int ny, int nz,
-                     const CUtensorMap *tin, const CUtensorMap *tout, int *err, cudaStream_t st);
+                     const CUtensorMap *tin, const CUtensorMap *tout, int sms, int *err, cudaStream_t st);
 // x / y derivative by the register-streamed kernel (no shared memory)
 // pipelined persistent x / y line solves over TMA tiles (one CTA per SM, a
 // ring of tile buffers, right-hand side fused into the forward pass); false

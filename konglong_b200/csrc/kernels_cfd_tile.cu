@@ -8,11 +8,12 @@
 //
 // What bounds it: shared memory caps the lines in flight (three 512-point tiles
 // a SM), so the launch takes (tiles / resident tiles) x (latency of one tile),
-// and a tile's latency is the serial work of its warps.  Measured on a 512-point
-// tile before this form: load 5 k cycles, right-hand sides 10 k, elimination
-// 12.7 k, back substitution 15.7 k, store 5 k, at 3-4 cycles per instruction of
-// a lone warp.  So every phase is written for the fewest instructions on the
-// critical warp:
+// and a tile's latency is the serial work of its warps.  Cycles of a 512-point
+// tile, before this form and now: load 5 k / 4 k, right-hand sides 10.5 k / 5-7 k,
+// elimination 12.5 k / 5.2 k, back substitution 15.7 k / 8.3 k, store 5 k / 2.5 k;
+// a launch at 512 x 512 x 400: x / y lines 400 -> 240 us, z lines 410 -> 210 us
+// (HBM copy rate: 130 us).  Every phase is written for the fewest instructions
+// on its critical warp:
 //   - lines live in shared memory as row quads (4 consecutive rows of a line in
 //     one float4), so the recurrences move a quad per load / store instead of a
 //     row; x / y tiles arrive row by row, and the right-hand-side pass, which
@@ -22,12 +23,19 @@
 //   - each pivot is taken off the four following rows as soon as it is final
 //     (the row's terms still arrive oldest pivot first, one FMA each, so the
 //     bits are those of the row-by-row form): the row-to-row chain is one FMA
-//     (elimination) or a multiply and an FMA (back substitution);
+//     (elimination, 7.9 cycles a row alone on an SM, 18 before) or a multiply and
+//     an FMA (back substitution, 12 cycles, 21 before);
 //   - three quads are loaded ahead; the factors of the Toeplitz interior (rows
 //     k0 .. k1 - 1, bitwise constant) come from the parameter bank, the others
 //     from a table staged in shared memory while the tile loads (from global
-//     memory these ~84 rows cost a third of both recurrences);
-//   - every resident CTA solves on a different scheduler.
+//     memory these ~89 rows cost a third of both recurrences).  Loading a quad's
+//     table rows one quad ahead was slower (z lines 232 us): the copies cost
+//     more than the wait;
+//   - resident CTAs solve on different schedulers (285 -> 259 us);
+//   - eight warps form the right-hand sides of long lines, four of short ones,
+//     whose CTAs fill the SM (the line at kLongLine points);
+//   - the tile that a resident CTA's successor will load is prefetched into L2
+//     (250 -> 240 us).
 #include <algorithm>
 
 #include "cfd_rows.cuh"
@@ -55,6 +63,8 @@ struct TileArgs {
   int lines, pitch;        // lines: per tile (<= 32), floats per line in shared memory
   int tab;                 // table rows
   int off;                 // byte offset of the tile
+  int sms;                 // SMs of the device (CTAs of a wave)
+  int ahead;               // CTAs resident at once: the tile that many on is prefetched into L2
 };
 
 // One lane's line in the tile: raw rows and quads
@@ -64,83 +74,90 @@ struct Line {
   float4 *q;
   __device__ __forceinline__ float &row(int i) const { return r[ROWS ? i * 32 : i]; }
   __device__ __forceinline__ float4 &quad(int k) const { return q[ROWS ? k * 32 : k]; }
-  // 8 raw rows from i (a multiple of 8), zero from row n on
-  __device__ __forceinline__ void load8(float (&v)[8], int i, int n) const {
-    if (i + 8 <= n) {
-      if (ROWS) {
+  // 8 raw rows from i (a multiple of 8); the tile has room past its last row
+  __device__ __forceinline__ void load8(float (&v)[8], int i) const {
+    if (ROWS) {
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = row(i + k);
-      } else {
-        const float4 a = quad(i / 4), b = quad(i / 4 + 1);
-        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
-      }
+      for (int k = 0; k < 8; k++) v[k] = row(i + k);
     } else {
-#pragma unroll
-      for (int k = 0; k < 8; k++) v[k] = i + k < n ? row(i + k) : 0.f;
+      const float4 a = quad(i / 4), b = quad(i / 4 + 1);
+      v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
     }
   }
+  // one value of row i in quad form
+  __device__ __forceinline__ float &elem(int i) const { return reinterpret_cast<float *>(&quad(i / 4))[i % 4]; }
 };
 
 // Phase 1.  Warp w takes a run of 8-row chunks; the rows of the neighbouring
 // runs that its windows reach are read before the barrier, so the runs can be
-// rewritten in place as quads.  Rows from n up to the next multiple of 4
-// become zero.  act: the lane holds a line.
+// rewritten in place as quads.  The loop forms every row as an interior one;
+// the one-sided rows of the line's ends and the zero rows from n up to the next
+// multiple of 4 are written over afterwards (selecting them inside the loop
+// doubled its time).  act: the lane holds a line.
 template <bool ROWS>
-__device__ __forceinline__ void tile_rhs(const CfdPlanDev &p, const Line<ROWS> &L, int warp, bool act) {
+__device__ __forceinline__ void tile_rhs(const CfdPlanDev &p, const Line<ROWS> &L, int warp, int nw, bool act) {
   const int n = p.n, n4 = (n + 3) / 4 * 4;
-  const int run = ((n4 + 7) / 8 + 3) / 4 * 8;
+  const int run = ((n4 + 7) / 8 + nw - 1) / nw * 8;
   const int p0 = min(n4, warp * run), p1 = min(n4, p0 + run);
   const bool own = act && p0 < p1;
   float prev[5], post[5], cur[8];
+  // one-sided rows, every coefficient index a constant (indexed reads of the
+  // parameter bank are slow): rows 0 .. 4 by the first run, rows n - 5 .. n - 1
+  // by the runs that reach them (never the first: n >= 16)
+  const bool lo = p0 == 0, hi = !lo && p1 > n - 5;
+  float ends[5];
   if (own) {
+    if (lo || hi) {
+      float x[16];  // lo: rows -5 .. 10; hi: rows n - 11 .. n - 1
+#pragma unroll
+      for (int k = 0; k < 16; k++) x[k] = lo ? (k < 5 ? 0.f : L.row(k - 5)) : (k < 11 ? L.row(n - 11 + k) : 0.f);
+#pragma unroll
+      for (int k = 0; k < 5; k++) ends[k] = lo ? rhs_low(p.a, k, x + k) : rhs_high(p.a, 5 - k, x + 1 + k);
+    }
 #pragma unroll
     for (int k = 0; k < 5; k++) {
       prev[k] = p0 - 5 + k >= 0 ? L.row(p0 - 5 + k) : 0.f;
       post[k] = p1 + k < n ? L.row(p1 + k) : 0.f;
     }
-    L.load8(cur, p0, n);
+    L.load8(cur, p0);
   }
   __syncthreads();
   if (!own) return;
   const RhsCoef rc{p.a[55], p.a[56], p.a[57], p.a[58], p.a[59]};
-#pragma unroll 1
-  for (int i0 = p0; i0 < p1; i0 += 8) {
-    float next[8];
-    if (i0 + 8 < p1) {
-      L.load8(next, i0 + 8, n);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; k++) next[k] = k < 5 ? post[k] : 0.f;
-    }
-    float w[18];  // rows i0 - 5 .. i0 + 12
+  // rows i0 .. i0 + 7 from prev (i0 - 5 ..), cur and next (i0 + 8 ..)
+  auto chunk = [&](int i0, const float *next, bool two) {
+    float w[18];
 #pragma unroll
     for (int k = 0; k < 18; k++) w[k] = k < 5 ? prev[k] : k < 13 ? cur[k - 5] : next[k - 13];
     float v[8];
-    if (i0 >= 5 && i0 + 8 <= n - 5) {
 #pragma unroll
-      for (int k = 0; k < 8; k++)
-        v[k] = rhs_interior(rc, w[k], w[k + 1], w[k + 2], w[k + 3], w[k + 4], w[k + 6], w[k + 7], w[k + 8], w[k + 9],
-                            w[k + 10]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int i = i0 + k;
-        if (i >= n) v[k] = 0.f;
-        else if (i < 5) v[k] = rhs_low(p.a, i, w + k);
-        else if (i >= n - 5) v[k] = rhs_high(p.a, n - i, w + k);
-        else
-          v[k] = rhs_interior(rc, w[k], w[k + 1], w[k + 2], w[k + 3], w[k + 4], w[k + 6], w[k + 7], w[k + 8], w[k + 9],
-                              w[k + 10]);
-      }
-    }
+    for (int k = 0; k < 8; k++)
+      v[k] = rhs_interior(rc, w[k], w[k + 1], w[k + 2], w[k + 3], w[k + 4], w[k + 6], w[k + 7], w[k + 8], w[k + 9],
+                          w[k + 10]);
     if (ROWS) __syncwarp();  // a quad row replaces four rows of other lanes
     L.quad(i0 / 4) = make_float4(v[0], v[1], v[2], v[3]);
-    if (i0 + 4 < n4) L.quad(i0 / 4 + 1) = make_float4(v[4], v[5], v[6], v[7]);
+    if (two) L.quad(i0 / 4 + 1) = make_float4(v[4], v[5], v[6], v[7]);
+  };
+  int i0 = p0;
+#pragma unroll 1
+  for (; i0 + 8 < p1; i0 += 8) {
+    float next[8];
+    L.load8(next, i0 + 8);
+    chunk(i0, next, true);
 #pragma unroll
     for (int k = 0; k < 5; k++) prev[k] = cur[k + 3];
 #pragma unroll
     for (int k = 0; k < 8; k++) cur[k] = next[k];
   }
+  chunk(i0, post, i0 + 4 < n4);
+  if (lo || hi)
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+      const int i = lo ? k : n - 5 + k;
+      if (i >= p0 && i < p1) L.elem(i) = ends[k];
+    }
+  if (p1 == n4)
+    for (int i = n; i < n4; i++) L.elem(i) = 0.f;
 }
 
 // Factors of the rows outside [k0, k1), in shared memory: per pivot row the
@@ -220,19 +237,9 @@ __device__ __forceinline__ void tile_solve(const CfdPlanDev &p, const TileTab &t
   bwd_quads<ROWS, false>(L, tab.u + ta, tab.rd + ta, uc, p.rdc, 0, qa, c, d, e);
 }
 
-// The warp of a four-warp CTA that solves its tile.  A CTA's warps sit on the
-// SM's four schedulers in warp-slot order, so with warp 0 solving in every CTA
-// the resident solvers would share one scheduler; the CTA's slot (the hardware
-// warp index of its warp 0) spreads them.  Only a hint: any warp may solve.
-__device__ __forceinline__ int solver_warp() {
-  unsigned w;
-  asm volatile("mov.u32 %0, %%warpid;" : "=r"(w));
-  return __syncthreads_count(threadIdx.x < ((w >> 2) & 3u));  // true for threads of warp 0 only
-}
-
-// registers for six resident CTAs: tiles of lines up to ~250 points
+// registers for three resident CTAs of 256 threads or six of 128
 template <int IO>
-__global__ void __launch_bounds__(128, 6) cfd_tile_k(const __grid_constant__ CfdPlanDev p,
+__global__ void __launch_bounds__(256, 3) cfd_tile_k(const __grid_constant__ CfdPlanDev p,
                                                      const __grid_constant__ CUtensorMap tin,
                                                      const __grid_constant__ CUtensorMap tout,
                                                      const __grid_constant__ TileArgs a, int *err) {
@@ -251,16 +258,27 @@ __global__ void __launch_bounds__(128, 6) cfd_tile_k(const __grid_constant__ Cfd
     if (threadIdx.x == 0) {
       mbar_init(bar, 1);
       mbar_fence_init();
+      // the tile that one of the resident CTAs' successors will load
+      const long long nx_ = (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x + a.ahead;
       if (IO == IO_ROWS_TMA) {
         mbar_expect_tx(bar, (uint32_t)a.nb * (uint32_t)a.R * 32u * 4u);
         for (int b = 0; b < a.nb; b++) {
           if (a.axis == DX) tma_load_3d(sm + (size_t)b * a.R * 32, &tin, bar, iz0, b * a.R, o);
           else tma_load_3d(sm + (size_t)b * a.R * 32, &tin, bar, iz0, o, b * a.R);
         }
+        const int zn = (int)(nx_ % gridDim.x) * 32, on = (int)(nx_ / gridDim.x);
+        if (on < (int)gridDim.y)
+          for (int b = 0; b < a.nb; b++) {
+            if (a.axis == DX) tma_prefetch_3d(&tin, zn, b * a.R, on);
+            else tma_prefetch_3d(&tin, zn, on, b * a.R);
+          }
       } else {
         mbar_expect_tx(bar, (uint32_t)nl * (uint32_t)n * 4u);
         for (int l = 0; l < nl; l++)
           bulk_load(sm + (size_t)l * a.pitch, a.in + base + (long long)l * n, (uint32_t)n * 4u, bar);
+        const long long ln = nx_ * a.lines;
+        if (ln < a.nlines)
+          bulk_prefetch(a.in + ln * n, (uint32_t)min((long long)a.lines, a.nlines - ln) * (uint32_t)n * 4u);
       }
     }
   } else if (IO == IO_ROWS) {
@@ -283,7 +301,12 @@ __global__ void __launch_bounds__(128, 6) cfd_tile_k(const __grid_constant__ Cfd
     tu[k] = __ldg(reinterpret_cast<const float4 *>(p.tu) + i);
     tr[k] = __ldg(p.tr + i);
   }
-  const int sw = solver_warp();  // a barrier: the mbarrier is initialised
+  // The solving warp.  Warp k of every CTA issues from scheduler k of its SM, so
+  // one fixed warp would put all resident solvers on one scheduler (the fourth
+  // of the right-hand sides that shares it then took twice as long, as did the
+  // solvers); CTAs that are resident together differ in their wave, mostly.
+  const int sw = (int)((blockIdx.x + (long long)blockIdx.y * gridDim.x) / a.sms) & 3;
+  __syncthreads();  // the mbarrier is initialised
   if (ASYNC) {
     if (!__syncthreads_and(mbar_wait(bar, 0, err))) {
       if (threadIdx.x == 0) mbar_drain(bar, 0);
@@ -297,7 +320,7 @@ __global__ void __launch_bounds__(128, 6) cfd_tile_k(const __grid_constant__ Cfd
   L.r = ROWS ? sm + lane : sm + lane * a.pitch;
   L.q = ROWS ? reinterpret_cast<float4 *>(sm) + lane : reinterpret_cast<float4 *>(sm + lane * a.pitch);
   const bool act = ROWS || lane < nl;  // rows: lanes past nz hold zeros
-  tile_rhs<ROWS>(p, L, warp, act);
+  tile_rhs<ROWS>(p, L, warp, nw, act);
   __syncthreads();
   if (warp == sw && act) tile_solve<ROWS>(p, TileTab{tl, tu, tr}, L);
   if (ASYNC) {
@@ -329,9 +352,15 @@ __global__ void __launch_bounds__(128, 6) cfd_tile_k(const __grid_constant__ Cfd
 }
 
 constexpr size_t kTileSmem = 227 * 1024;
+constexpr int kLongLine = 250;
 
 // byte offset of the tile after the barrier and the factor table of `tab` rows
 int tile_off(int tab) { return (128 + tab * 36 + 127) / 128 * 128; }
+
+// CTAs of `threads` threads and `smem` bytes resident on the device at once
+int tiles_ahead(int sms, int threads, size_t smem) {
+  return sms * (int)std::max<size_t>(1, std::min<size_t>(768 / threads, (228 * 1024) / (smem + 1024)));
+}
 
 template <int IO>
 bool tile_attr() {
@@ -346,34 +375,40 @@ bool cfd_tile_init() {
 }
 
 bool launch_cfd_tile(int axis, const CfdPlanDev &p, const float *in, float *out, int nx, int ny, int nz,
-                     const CUtensorMap *tin, const CUtensorMap *tout, int *err, cudaStream_t st) {
+                     const CUtensorMap *tin, const CUtensorMap *tout, int sms, int *err, cudaStream_t st) {
   const int n4 = (p.n + 3) / 4 * 4;
   TileArgs a{};
-  a.in = in, a.out = out, a.nz = nz, a.axis = axis;
+  a.in = in, a.out = out, a.nz = nz, a.axis = axis, a.sms = sms;
   a.tab = p.k0 + n4 - p.k1;
   a.off = tile_off(a.tab);
   const CUtensorMap none{};
+  const int threads = p.n > kLongLine ? 256 : 128;
   if (axis == DZ) {
     a.nlines = (long long)nx * ny;
     // lines 4 floats (mod 32) apart: a quad load of eight lanes meets every bank once
     a.pitch = n4 + (36 - n4 % 32) % 32;
-    for (a.lines = 32; a.lines > 1 && a.off + (size_t)a.lines * a.pitch * 4 > kTileSmem;) a.lines /= 2;
-    const size_t smem = a.off + (size_t)a.lines * a.pitch * 4;
+    // (a chunk read past n4 reaches up to 4 floats beyond the last line)
+    auto bytes = [&](int lines) { return a.off + ((size_t)lines * a.pitch + 4) * 4; };
+    for (a.lines = 32; a.lines > 1 && bytes(a.lines) > kTileSmem;) a.lines /= 2;
+    const size_t smem = bytes(a.lines);
     if (smem > kTileSmem) return false;
     const unsigned grid = (unsigned)((a.nlines + a.lines - 1) / a.lines);
-    if (nz % 4 == 0) cfd_tile_k<IO_LINES_BULK><<<grid, 128, smem, st>>>(p, none, none, a, err);
-    else cfd_tile_k<IO_LINES><<<grid, 128, smem, st>>>(p, none, none, a, err);
+    a.ahead = tiles_ahead(sms, threads, smem);
+    if (nz % 4 == 0) cfd_tile_k<IO_LINES_BULK><<<grid, threads, smem, st>>>(p, none, none, a, err);
+    else cfd_tile_k<IO_LINES><<<grid, threads, smem, st>>>(p, none, none, a, err);
     return true;
   }
   const long long nxz = (long long)nx * nz;
   a.es = axis == DX ? nz : nxz, a.other = axis == DX ? nxz : nz;
   cfd_tma_box(p.n, &a.R, &a.nb);
-  const int rows = std::max(n4, (tin ? a.nb * a.R + 3 : 0) / 4 * 4);
+  // (a chunk read past n4 reaches up to 4 rows beyond)
+  const int rows = std::max(n4 + 4, (tin ? a.nb * a.R + 3 : 0) / 4 * 4);
   const size_t smem = a.off + (size_t)rows * 128;
   if (smem > kTileSmem) return false;
   const dim3 grid((nz + 31) / 32, axis == DX ? ny : nx);
-  if (tin && tout) cfd_tile_k<IO_ROWS_TMA><<<grid, 128, smem, st>>>(p, *tin, *tout, a, err);
-  else cfd_tile_k<IO_ROWS><<<grid, 128, smem, st>>>(p, none, none, a, err);
+  a.ahead = tiles_ahead(sms, threads, smem);
+  if (tin && tout) cfd_tile_k<IO_ROWS_TMA><<<grid, threads, smem, st>>>(p, *tin, *tout, a, err);
+  else cfd_tile_k<IO_ROWS><<<grid, threads, smem, st>>>(p, none, none, a, err);
   return true;
 }
 

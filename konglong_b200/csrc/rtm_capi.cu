@@ -55,7 +55,7 @@ struct Engine {
   // every other configuration takes the two first-derivative passes
   // (bgprtm/KernelCPU.cpp:125-174)
   bool lap_iso() const { return c.engine == RTM_ENGINE_FD8 && c.model_type == RTM_ISO && !c.use_rho; }
-  int device = 0;
+  int device = 0, sms = 148;
   cudaStream_t st = nullptr;
   long long n = 0, nxz = 0;
   std::string err;
@@ -518,7 +518,7 @@ static void cfd_deriv(Engine *h, int axis, int sgn, const float *in, float *out)
       launch_cfd_deriv_pipe(axis, h->cfd[axis][sgn], d.nx, d.ny, d.nz, &mi, &mo, h->dflag, h->st))
     return;
   if (!launch_cfd_tile(axis, h->cfd[axis][sgn], in, out, d.nx, d.ny, d.nz, tma ? &mi : nullptr, tma ? &mo : nullptr,
-                       h->dflag, h->st)) {
+                       h->sms, h->dflag, h->st)) {
     if (axis == DZ) h->fft_err = 1;  // a single z line exceeds shared memory
     else launch_cfd_deriv_stream(axis, h->cfd[axis][sgn], in, out, d.nx, d.ny, d.nz, h->st);
   }
@@ -1549,6 +1549,7 @@ int rtm_create(const rtm_dims *d, const rtm_config *c, rtm_handle **out) {
     cudaGetLastError();
     return fail(RTM_ERR_CUDA);
   }
+  if (cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess || h->sms < 1) h->sms = 148;
   // a blocking stream: its work waits for earlier legacy-stream work, so the
   // set-up uploads below (pageable cudaMemcpy, whose DMA may still be running
   // when the call returns) land before any kernel of the engine reads them

@@ -88,6 +88,16 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void 
                "r"(smem_u32(src)), "r"(cz), "r"(cx), "r"(cy)
                : "memory");
 }
+// L2 prefetch of a tiled box / of a plain run (address and size multiples of 16 bytes)
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int cz, int cx, int cy) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"((uint64_t)map), "r"(cz),
+               "r"(cx), "r"(cy)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_prefetch(const void *src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(src)), "r"(bytes) : "memory");
+}
+
 // plain bulk copies: addresses and size multiples of 16 bytes
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
