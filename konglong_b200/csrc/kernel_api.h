@@ -289,7 +289,10 @@ struct CfdGradEpiArgs {  // PML round 1 + scaling on raw gradients, in place
   FusedIo io;
   const float *w1;
 };
+// pml_only: the cells of the PML faces alone
 void launch_cfd_grad_epilogue(const CfdGradEpiArgs &a, cudaStream_t st, bool pml_only = false);
+// one launch over the grid (kernels_cfd_epi.cu); opposite PML faces must not overlap
+void launch_cfd_grad_epi(const CfdGradEpiArgs &a, bool pml_only, cudaStream_t st);
 
 struct CfdDivEpiArgs {  // PML round 2 on raw divergence parts + update
   int nx, ny, nz, pml3d, mode;
@@ -305,6 +308,7 @@ struct CfdDivEpiArgs {  // PML round 2 on raw divergence parts + update
   QDev q;
 };
 void launch_cfd_div_epilogue(const CfdDivEpiArgs &a, cudaStream_t st, bool pml_only = false);
+void launch_cfd_div_epi(const CfdDivEpiArgs &a, bool pml_only, cudaStream_t st);
 // the z line solve of `in` fused with the gradient / divergence epilogue (the
 // raw z part stays in shared memory; the x / y parts come from a.gx, a.gy /
 // a.dx, a.dy)

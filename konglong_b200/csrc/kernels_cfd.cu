@@ -12,6 +12,7 @@
 
 #include <algorithm>
 
+#include "cfd_epi.cuh"
 #include "cfd_rows.cuh"
 #include "kernel_api.h"
 #include "rtm_device.cuh"
@@ -642,24 +643,13 @@ __global__ void __launch_bounds__(256, 1) cfd_pipe_k(CfdPlanDev p, const __grid_
   }
 }
 
-// Cell regions of the pointwise epilogues.  The PML cells form six disjoint
-// boxes (y bands over the whole xz plane, x bands inside the y interior, z
-// bands inside both); the rest is the interior box.  Each box is one launch
-// of a 3-D grid: interior cells run without PML code, PML cells gather every
-// PML memory value of the cell first (pml1_all).
+// Cell regions of the line solves that carry an epilogue and of the epilogues
+// of grids whose PML faces overlap (the others: kernels_cfd_epi.cu).  The PML
+// cells form six disjoint boxes (y bands over the whole xz plane, x bands inside
+// the y interior, z bands inside both); the rest is the interior box.
 struct EpiBox {
   int z0, z1, x0, x1, y0, y1;
 };
-
-// density division and VTI / TTI scaling of one cell's gradients after PML
-// round 1 (KernelCPU::ScalarVTI / ScalarTTI), every rounding explicit so that
-// each kernel inlining it gives the same bits
-__device__ __forceinline__ void grad_finish(const CfdGradEpiArgs &a, bool do_y, float &gx, float &gy, float &gz,
-                                            float ep, float dl, float ax, float ay, float r) {
-  if (a.rho) divide_rho(r, do_y, gx, gy, gz);
-  if (a.model == 3) aniso_scale<3>(make_float4(ep, dl, ax, ay), gx, gy, gz);
-  else if (a.model == 2) aniso_scale<2>(make_float4(ep, dl, 0.f, 0.f), gx, gy, gz);
-}
 
 // PML round 1 + VTI / TTI scaling of the raw gradients of one cell, in place
 // (pml1 on each component, then grad_finish)
@@ -676,24 +666,6 @@ __device__ __forceinline__ void grad_cell(const CfdGradEpiArgs &a, const Grid3 &
   a.gz[i] = gz;
   a.gx[i] = gx;
   if (do_y) a.gy[i] = gy;
-}
-
-// accumulation w0 - vel (dx + dz + dy) (with density in the engine's form)
-// and the update of MODE 0 (none) or 1 (leapfrog)
-template <int MODE>
-__device__ __forceinline__ float div_finish(const CfdDivEpiArgs &a, float dxv, float dyv, float dzv, float vel,
-                                            float w0, float w1, float r) {
-  float t;
-  if (a.rho) {
-    t = a.rho_form == 2   ? div_accumulate_rho<2>(w0, vel, r, dxv, dzv, dyv)
-        : a.rho_form == 1 ? div_accumulate_rho<1>(w0, vel, r, dxv, dzv, dyv)
-                          : div_accumulate_rho<0>(w0, vel, r, dxv, dzv, dyv);
-  } else {
-    t = __fmaf_rn(-dxv, vel, w0);
-    t = __fmaf_rn(-dzv, vel, t);
-    t = __fmaf_rn(-dyv, vel, t);
-  }
-  return MODE == 1 ? __fsub_rn(__fadd_rn(w1, w1), t) : t;
 }
 
 // PML round 2 on the raw divergence parts of one cell, then
@@ -837,29 +809,22 @@ __global__ void __launch_bounds__(128) cfd_zdiv_k(CfdPlanDev p, const float *__r
 }
 
 // one box: block (32 z, 8 x), grid (z tiles, x tiles, y count) from (z0, x0, y0);
-// MASK (bit 2*d + s) lists the PML faces that can hold the box's cells
-template <bool PML, int MASK>
+// PML cells gather every memory value of their faces first (pml1_all)
+template <bool PML>
 __global__ void __launch_bounds__(256) cfd_grad_box_k(CfdGradEpiArgs a, EpiBox b) {
   const Grid3 g{a.nx, a.ny, a.nz, (long long)a.nx * a.nz};
   const int iz = b.z0 + blockIdx.x * 32 + threadIdx.x, ix = b.x0 + blockIdx.y * 8 + threadIdx.y, iy = b.y0 + blockIdx.z;
-  if (iz < b.z1 && ix < b.x1) grad_cell<PML, MASK>(a, g, ix, iy, iz);
+  if (iz < b.z1 && ix < b.x1) grad_cell<PML, 63>(a, g, ix, iy, iz);
 }
-template <bool PML, int MASK, int MODE>
+template <bool PML, int MODE>
 __global__ void __launch_bounds__(256) cfd_div_box_k(CfdDivEpiArgs a, EpiBox b) {
   const Grid3 g{a.nx, a.ny, a.nz, (long long)a.nx * a.nz};
   const int iz = b.z0 + blockIdx.x * 32 + threadIdx.x, ix = b.x0 + blockIdx.y * 8 + threadIdx.y, iy = b.y0 + blockIdx.z;
-  if (iz < b.z1 && ix < b.x1) div_cell<PML, MASK, MODE>(a, g, ix, iy, iz);
+  if (iz < b.z1 && ix < b.x1) div_cell<PML, 63, MODE>(a, g, ix, iy, iz);
 }
 
-// face masks of the PML boxes: y band (its y face, any x / z face), x band
-// (its x face, any z face), z band (its z face)
-constexpr int kZL = 1 << (2 * DZ), kZH = 2 << (2 * DZ), kXL = 1 << (2 * DX), kXH = 2 << (2 * DX),
-              kYL = 1 << (2 * DY), kYH = 2 << (2 * DY);
-constexpr int kBoxMask[7] = {0, kYL | kXL | kXH | kZL | kZH, kYH | kXL | kXH | kZL | kZH, kXL | kZL | kZH,
-                             kXH | kZL | kZH, kZL, kZH};
-
-// interior box [0] and the six PML boxes [1..6] (kBoxMask order; empty boxes
-// have z1 <= z0)
+// interior box [0] and the six PML boxes [1..6] (y bands, x bands, z bands;
+// empty boxes have z1 <= z0)
 void epi_boxes(const PmlDev &P, int nx, int ny, int nz, EpiBox *out) {
   const int zl = min(P.f[DZ][0].w, nz), zh = min(P.f[DZ][1].w, nz - zl);
   const int xl = min(P.f[DX][0].w, nx), xh = min(P.f[DX][1].w, nx - xl);
@@ -927,14 +892,6 @@ int cfd_init() {
   return ok ? 0 : -1;
 }
 
-template <int K, typename F>
-static void each_box(const EpiBox *bx, F &&f) {
-  if constexpr (K < 7) {
-    if (!box_empty(bx[K])) f(std::integral_constant<int, K>{});
-    each_box<K + 1>(bx, f);
-  }
-}
-
 // lo and hi layers of one dimension overlap (small grids): a cell of a band
 // box can then also lie in the opposite face, so every box takes all faces
 static bool pml_overlap(const PmlDev &P, int nx, int ny, int nz) {
@@ -942,36 +899,34 @@ static bool pml_overlap(const PmlDev &P, int nx, int ny, int nz) {
 }
 
 void launch_cfd_grad_epilogue(const CfdGradEpiArgs &a, cudaStream_t st, bool pml_only) {
+  if (!pml_overlap(a.pml, a.nx, a.ny, a.nz)) return launch_cfd_grad_epi(a, pml_only, st);
   EpiBox bx[7];
   epi_boxes(a.pml, a.nx, a.ny, a.nz, bx);
-  if (pml_only) bx[0].z1 = bx[0].z0;
-  const bool all = pml_overlap(a.pml, a.nx, a.ny, a.nz);
-  each_box<0>(bx, [&](auto k) {
-    constexpr int K = decltype(k)::value;
-    const dim3 g = box_grid(bx[K]), block(32, 8);
-    if (K > 0 && all) cfd_grad_box_k<true, 63><<<g, block, 0, st>>>(a, bx[K]);
-    else cfd_grad_box_k<(K > 0), kBoxMask[K]><<<g, block, 0, st>>>(a, bx[K]);
-  });
+  for (int k = pml_only ? 1 : 0; k < 7; k++) {
+    if (box_empty(bx[k])) continue;
+    const dim3 g = box_grid(bx[k]), block(32, 8);
+    if (k) cfd_grad_box_k<true><<<g, block, 0, st>>>(a, bx[k]);
+    else cfd_grad_box_k<false><<<g, block, 0, st>>>(a, bx[k]);
+  }
 }
 
-template <int K, int MODE>
-static void div_box(const CfdDivEpiArgs &a, const EpiBox &b, bool all, cudaStream_t st) {
+template <int MODE>
+static void div_box(const CfdDivEpiArgs &a, const EpiBox &b, bool pml, cudaStream_t st) {
   const dim3 g = box_grid(b), block(32, 8);
-  if (K > 0 && all) cfd_div_box_k<true, 63, MODE><<<g, block, 0, st>>>(a, b);
-  else cfd_div_box_k<(K > 0), kBoxMask[K], MODE><<<g, block, 0, st>>>(a, b);
+  if (pml) cfd_div_box_k<true, MODE><<<g, block, 0, st>>>(a, b);
+  else cfd_div_box_k<false, MODE><<<g, block, 0, st>>>(a, b);
 }
 
 void launch_cfd_div_epilogue(const CfdDivEpiArgs &a, cudaStream_t st, bool pml_only) {
+  if (!pml_overlap(a.pml, a.nx, a.ny, a.nz)) return launch_cfd_div_epi(a, pml_only, st);
   EpiBox bx[7];
   epi_boxes(a.pml, a.nx, a.ny, a.nz, bx);
-  if (pml_only) bx[0].z1 = bx[0].z0;
-  const bool all = pml_overlap(a.pml, a.nx, a.ny, a.nz);
-  each_box<0>(bx, [&](auto k) {
-    constexpr int K = decltype(k)::value;
-    if (a.mode == 0) div_box<K, 0>(a, bx[K], all, st);
-    else if (a.mode == 1) div_box<K, 1>(a, bx[K], all, st);
-    else div_box<K, 2>(a, bx[K], all, st);
-  });
+  for (int k = pml_only ? 1 : 0; k < 7; k++) {
+    if (box_empty(bx[k])) continue;
+    if (a.mode == 0) div_box<0>(a, bx[k], k > 0, st);
+    else if (a.mode == 1) div_box<1>(a, bx[k], k > 0, st);
+    else div_box<2>(a, bx[k], k > 0, st);
+  }
 }
 
 void launch_cfd_zgrad(const CfdPlanDev &p, const float *in, const CfdGradEpiArgs &a, cudaStream_t st) {

@@ -560,6 +560,15 @@ static int setup_pml(Engine *h) {
       CK(cudaMemcpy(dco, co.data(), co.size() * 4, cudaMemcpyHostToDevice));
       F.w = wp[s];
       F.co = dco;
+      if (dim == DZ) {
+        std::vector<float> cz(co.size());
+        for (int i = 0; i < wp[s]; i++)
+          for (int k = 0; k < 6; k++) cz[(size_t)k * wp[s] + i] = co[(size_t)(s ? wp[s] - 1 - i : i) * 6 + k];
+        float *dcz;
+        TRY(h->alloc(dcz, cz.size()));
+        CK(cudaMemcpy(dcz, cz.data(), cz.size() * 4, cudaMemcpyHostToDevice));
+        F.cz = dcz;
+      }
       float *q;
       TRY(h->alloc(q, (size_t)F.cs * ncomp * 2));
       for (int r = 0; r < 2; r++)

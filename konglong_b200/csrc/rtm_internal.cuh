@@ -30,6 +30,7 @@ struct PmlFace {
   int w;            // layer count, 0 = no PML on this face
   long long cs;     // array stride
   const float *co;  // [w][6]
+  const float *cz;  // z faces: the constants [6][w] by cell along z (the high face's layers reversed)
   float *q[2][3];   // [round][component]
 };
 
