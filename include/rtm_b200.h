@@ -392,7 +392,7 @@ int rtm_illum_compensate(rtm_handle *h, int smooth_xy, int smooth_z, float amp_d
 
 /* Propagator::modelling loop (bgprtm/Propagator.cpp:1099-1153): for it in
  * [0, nts): kernel, update2nd, inject(it + it_shift), extract(it / ntratio)
- * when it % ntratio == 0, swap.  Fused kernels; time loop in a CUDA graph. */
+ * when it % ntratio == 0, swap.  Fused kernels, launched step by step. */
 int rtm_modelling(rtm_handle *h, int nts, int it_shift, int ntratio);
 
 /* Propagator::migration loop (bgprtm/Propagator.cpp:1210-1255).
@@ -484,7 +484,7 @@ int rtm_set_compressor_fallback(rtm_handle *h, float tau, float max_fraction);
  * tiles of every active shot) or all VTI, or all TTI (each step two persistent
  * kernels, the gradient and the divergence pass of the one-cell kernels; no
  * density, FP32 state), then one batched injection and one batched extraction
- * launch; the time loop runs as CUDA graphs.  Each handle must have its model,
+ * launch.  Each handle must have its model,
  * injection (and, optionally, extraction) set and be reset.
  * No reference counterpart: bgprtm runs one shot per process
  * (bgprtm/Propagator.cpp:1054-1260 per shot). */
@@ -554,7 +554,7 @@ enum {
   RTM_K_CFD_XF = 13,   /* compact FD, segment-parallel: fused x kernel (x divergence part, accumulation, update) */
   RTM_NKINDS = 14
 };
-/* on = 1: the time loops run eagerly (no CUDA graph) with CUDA events around
+/* on = 1: the time loops run with CUDA events around
  * every launch, and the per-kind device time accumulates; on = 0 resets. */
 int rtm_profile(rtm_handle *h, int on);
 /* ms[RTM_NKINDS], count[RTM_NKINDS]: accumulated device time and launches. */

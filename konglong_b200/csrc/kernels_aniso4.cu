@@ -15,6 +15,7 @@
 #include <type_traits>
 
 #include "kernel_api.h"
+#include "launch.cuh"
 #include "pml4.cuh"
 #include "tma.cuh"
 
@@ -134,8 +135,10 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? kEdgeCtas : 0)
     for (int k = 0; k < SB; k++) mbar_init(&s.bar_b[k], 1);
     mbar_fence_init();
   }
+  dep_launch();
   if constexpr (EDGE != 0) fill_pml_co(s.co, a.pml, g, iz0, ix0, tzq, tx);
   __syncthreads();
+  dep_wait();
   int last_a = y0 - 1, last_b = y0 - 1;  // last planes the producer issued
   if (producer) {
     for (int p = y0; p < min(y0 + R4 + P, y1 + R4); p++) issue_a(p), last_a = p;
@@ -305,8 +308,10 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? kEdgeCtas : 0)
     for (int k = 0; k < SB; k++) mbar_init(&s.bar_b[k], 1);
     mbar_fence_init();
   }
+  dep_launch();
   if constexpr (EDGE != 0) fill_pml_co(s.co, a.pml, g, iz0, ix0, tzq, tx);
   __syncthreads();
+  dep_wait();
   // ring A carries planes y0+4 .. y1+3 only (the queue starts with planes
   // y0-4 .. y0+3 read from global memory), so every copy it gets is waited for
   int last_a = y0 + R4 - 1, last_b = y0 - 1;
@@ -431,7 +436,7 @@ void launch_grad4(const GradArgs &a, const Tile4 *tiles, int ntiles, bool edge, 
   if (ntiles <= 0) return;
   const dim3 block(8, kTX);
   const int e = !edge ? TILE_INT : a.pml3d ? TILE_PML3 : TILE_PML1;
-#define G_(MD, E) grad4_k<kTX, kP, MD, E><<<ntiles, block, grad4_smem<kTX, kP, MD>(), st>>>(a, tiles, m, err)
+#define G_(MD, E) launch_dep(grad4_k<kTX, kP, MD, E>, ntiles, block, grad4_smem<kTX, kP, MD>(), st, a, tiles, m, err)
 #define E_(MD)                          \
   if (e == TILE_INT) G_(MD, TILE_INT);  \
   else if (e == TILE_PML1) G_(MD, TILE_PML1); \
@@ -450,7 +455,7 @@ void launch_div4(const DivArgs &a, const Tile4 *tiles, int ntiles, bool edge, in
   if (ntiles <= 0) return;
   const dim3 block(8, kTX);
   const int e = !edge ? TILE_INT : a.pml3d ? TILE_PML3 : TILE_PML1;
-#define D_(MD, E, QR) div4_k<kTX, kP, MD, E, QR><<<ntiles, block, div4_smem<kTX, kP, QR>(), st>>>(a, tiles, m, err)
+#define D_(MD, E, QR) launch_dep(div4_k<kTX, kP, MD, E, QR>, ntiles, block, div4_smem<kTX, kP, QR>(), st, a, tiles, m, err)
 #define E_(MD, QR)                              \
   if (e == TILE_INT) D_(MD, TILE_INT, QR);      \
   else if (e == TILE_PML1) D_(MD, TILE_PML1, QR); \

@@ -40,6 +40,7 @@
 
 #include "cfd_rows.cuh"
 #include "kernel_api.h"
+#include "launch.cuh"
 #include "rtm_device.cuh"
 #include "tma.cuh"
 
@@ -254,6 +255,8 @@ __global__ void __launch_bounds__(256, 3) cfd_tile_k(const __grid_constant__ Cfd
   const long long l0 = (long long)blockIdx.x * a.lines;           // lines
   const int nl = ROWS ? min(32, a.nz - iz0) : (int)min((long long)a.lines, a.nlines - l0);
   const long long base = ROWS ? (long long)o * a.other + iz0 : l0 * n;
+  dep_launch();
+  dep_wait();
   if (ASYNC) {
     if (threadIdx.x == 0) {
       mbar_init(bar, 1);
@@ -394,8 +397,8 @@ bool launch_cfd_tile(int axis, const CfdPlanDev &p, const float *in, float *out,
     if (smem > kTileSmem) return false;
     const unsigned grid = (unsigned)((a.nlines + a.lines - 1) / a.lines);
     a.ahead = tiles_ahead(sms, threads, smem);
-    if (nz % 4 == 0) cfd_tile_k<IO_LINES_BULK><<<grid, threads, smem, st>>>(p, none, none, a, err);
-    else cfd_tile_k<IO_LINES><<<grid, threads, smem, st>>>(p, none, none, a, err);
+    if (nz % 4 == 0) launch_dep(cfd_tile_k<IO_LINES_BULK>, grid, threads, smem, st, p, none, none, a, err);
+    else launch_dep(cfd_tile_k<IO_LINES>, grid, threads, smem, st, p, none, none, a, err);
     return true;
   }
   const long long nxz = (long long)nx * nz;
@@ -407,8 +410,8 @@ bool launch_cfd_tile(int axis, const CfdPlanDev &p, const float *in, float *out,
   if (smem > kTileSmem) return false;
   const dim3 grid((nz + 31) / 32, axis == DX ? ny : nx);
   a.ahead = tiles_ahead(sms, threads, smem);
-  if (tin && tout) cfd_tile_k<IO_ROWS_TMA><<<grid, threads, smem, st>>>(p, *tin, *tout, a, err);
-  else cfd_tile_k<IO_ROWS><<<grid, threads, smem, st>>>(p, none, none, a, err);
+  if (tin && tout) launch_dep(cfd_tile_k<IO_ROWS_TMA>, grid, threads, smem, st, p, *tin, *tout, a, err);
+  else launch_dep(cfd_tile_k<IO_ROWS>, grid, threads, smem, st, p, none, none, a, err);
   return true;
 }
 

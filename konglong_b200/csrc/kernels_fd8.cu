@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include "kernel_api.h"
+#include "launch.cuh"
 #include "rtm_device.cuh"
 
 namespace rtm {
@@ -186,6 +187,8 @@ __device__ __forceinline__ void iso_tile(const IsoArgs &a, const float *__restri
 template <int TX, int MODE, bool PML3D>
 __global__ void __launch_bounds__(TZ *TX) iso_fd8_step(IsoArgs a) {
   __shared__ float tile[TX + 2 * R][TZ + 2 * R];
+  dep_launch();
+  dep_wait();
   iso_tile<TX, MODE, PML3D>(a, a.w1, a.w0, blockIdx.x, blockIdx.y, blockIdx.z, tile);
 }
 
@@ -198,6 +201,8 @@ template <int TX, bool PML3D>
 __global__ void __launch_bounds__(TZ *TX) iso_fd8_batch(const IsoBatchShot *__restrict__ shots,
                                                          const int *__restrict__ start, int nactive, int total, int it) {
   __shared__ float tile[TX + 2 * R][TZ + 2 * R];
+  dep_launch();
+  dep_wait();
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
     int lo = 0, hi = nactive - 1;
     while (lo < hi) {
@@ -284,6 +289,8 @@ template <int TX, int MODEL, bool F16, bool EDGE>
 __global__ void __launch_bounds__(TZ *TX) grad_fd8(GradArgs a, const Tile4 *__restrict__ tiles) {
   __shared__ float tile[TX + 2 * R][TZ + 2 * R];
   const Tile4 tl = tiles[blockIdx.x];
+  dep_launch();
+  dep_wait();
   grad_tile<TX, MODEL, F16, EDGE>(a, a.w1, tl.bz, tl.bx, tl.y0, tl.y1, tile);
 }
 
@@ -396,6 +403,8 @@ __global__ void __launch_bounds__(TZ *TX) div_fd8(DivArgs a, const Tile4 *__rest
   __shared__ float tpx[TX + 2 * R][TZ];
   __shared__ float tpz[TX][TZ + 2 * R];
   const Tile4 tl = tiles[blockIdx.x];
+  dep_launch();
+  dep_wait();
   div_tile<TX, MODE, F16, EDGE>(a, a.w1, a.w0, tl.bz, tl.bx, tl.y0, tl.y1, tpx, tpz);
 }
 
@@ -408,6 +417,8 @@ __global__ void __launch_bounds__(TZ *TX) grad_fd8_batch(const AnisoBatchShot *_
                                                           const int *__restrict__ start, int nactive, int total,
                                                           int it) {
   __shared__ float tile[TX + 2 * R][TZ + 2 * R];
+  dep_launch();
+  dep_wait();
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
     int lo = 0, hi = nactive - 1;
     while (lo < hi) {
@@ -428,6 +439,8 @@ __global__ void __launch_bounds__(TZ *TX) div_fd8_batch(const AnisoBatchShot *__
                                                          const int *__restrict__ start, int nactive, int total, int it) {
   __shared__ float tpx[TX + 2 * R][TZ];
   __shared__ float tpz[TX][TZ + 2 * R];
+  dep_launch();
+  dep_wait();
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
     int lo = 0, hi = nactive - 1;
     while (lo < hi) {
@@ -452,7 +465,7 @@ static dim3 fd_grid(int nx, int ny, int nz, int tx, int yseg) {
 template <int TX>
 static void iso_launch_tx(const IsoArgs &a, int mode, int pml3d, cudaStream_t st) {
   dim3 grid = fd_grid(a.nx, a.ny, a.nz, TX, a.yseg), block(TZ, TX);
-#define ISO_L(M, P) iso_fd8_step<TX, M, P><<<grid, block, 0, st>>>(a)
+#define ISO_L(M, P) launch_dep(iso_fd8_step<TX, M, P>, grid, block, 0, st, a)
   if (pml3d) {
     if (mode == 0) ISO_L(0, true);
     else if (mode == 1) ISO_L(1, true);
@@ -475,8 +488,8 @@ template <int TX>
 static void iso_batch_tx(const IsoBatchShot *shots, const int *start, int nactive, int total, int it, int pml3d,
                          int ctas, cudaStream_t st) {
   const unsigned grid = (unsigned)std::max(1, std::min(total, ctas));
-  if (pml3d) iso_fd8_batch<TX, true><<<grid, dim3(TZ, TX), 0, st>>>(shots, start, nactive, total, it);
-  else iso_fd8_batch<TX, false><<<grid, dim3(TZ, TX), 0, st>>>(shots, start, nactive, total, it);
+  if (pml3d) launch_dep(iso_fd8_batch<TX, true>, grid, dim3(TZ, TX), 0, st, shots, start, nactive, total, it);
+  else launch_dep(iso_fd8_batch<TX, false>, grid, dim3(TZ, TX), 0, st, shots, start, nactive, total, it);
 }
 
 void launch_iso_fd8_batch(const IsoBatchShot *shots, const int *start, int nactive, int total, int it, int pml3d,
@@ -503,9 +516,9 @@ void launch_aniso_fd8_batch(const AnisoBatchShot *shots, const int *start, int n
   if (total <= 0 || nactive <= 0) return;
   const unsigned grid = (unsigned)std::max(1, std::min(total, ctas));
   const dim3 block(TZ, kAnisoBatchTX);
-  if (model == 3) grad_fd8_batch<kAnisoBatchTX, 3><<<grid, block, 0, st>>>(shots, start, nactive, total, it);
-  else grad_fd8_batch<kAnisoBatchTX, 2><<<grid, block, 0, st>>>(shots, start, nactive, total, it);
-  div_fd8_batch<kAnisoBatchTX><<<grid, block, 0, st>>>(shots, start, nactive, total, it);
+  if (model == 3) launch_dep(grad_fd8_batch<kAnisoBatchTX, 3>, grid, block, 0, st, shots, start, nactive, total, it);
+  else launch_dep(grad_fd8_batch<kAnisoBatchTX, 2>, grid, block, 0, st, shots, start, nactive, total, it);
+  launch_dep(div_fd8_batch<kAnisoBatchTX>, grid, block, 0, st, shots, start, nactive, total, it);
 }
 
 int aniso_batch_ctas_per_sm() {
@@ -518,9 +531,9 @@ int aniso_batch_ctas_per_sm() {
 template <int TX, bool F16, bool EDGE>
 static void grad_launch_tx(const GradArgs &a, const Tile4 *tiles, int n, int model, cudaStream_t st) {
   const dim3 block(TZ, TX);
-  if (model == 3) grad_fd8<TX, 3, F16, EDGE><<<n, block, 0, st>>>(a, tiles);
-  else if (model == 2) grad_fd8<TX, 2, F16, EDGE><<<n, block, 0, st>>>(a, tiles);
-  else grad_fd8<TX, 1, F16, EDGE><<<n, block, 0, st>>>(a, tiles);
+  if (model == 3) launch_dep(grad_fd8<TX, 3, F16, EDGE>, n, block, 0, st, a, tiles);
+  else if (model == 2) launch_dep(grad_fd8<TX, 2, F16, EDGE>, n, block, 0, st, a, tiles);
+  else launch_dep(grad_fd8<TX, 1, F16, EDGE>, n, block, 0, st, a, tiles);
 }
 
 template <bool F16, bool EDGE>
@@ -545,9 +558,9 @@ void launch_grad_fd8(const GradArgs &a, const Tile4 *tiles, int ntiles, bool edg
 template <int TX, bool F16, bool EDGE>
 static void div_launch_tx(const DivArgs &a, const Tile4 *tiles, int n, int mode, cudaStream_t st) {
   const dim3 block(TZ, TX);
-  if (mode == 0) div_fd8<TX, 0, F16, EDGE><<<n, block, 0, st>>>(a, tiles);
-  else if (mode == 1) div_fd8<TX, 1, F16, EDGE><<<n, block, 0, st>>>(a, tiles);
-  else div_fd8<TX, 2, F16, EDGE><<<n, block, 0, st>>>(a, tiles);
+  if (mode == 0) launch_dep(div_fd8<TX, 0, F16, EDGE>, n, block, 0, st, a, tiles);
+  else if (mode == 1) launch_dep(div_fd8<TX, 1, F16, EDGE>, n, block, 0, st, a, tiles);
+  else launch_dep(div_fd8<TX, 2, F16, EDGE>, n, block, 0, st, a, tiles);
 }
 
 template <bool F16, bool EDGE>

@@ -8,6 +8,7 @@
 #include <algorithm>
 
 #include "kernel_api.h"
+#include "launch.cuh"
 #include "rtm_device.cuh"
 
 namespace rtm {
@@ -29,13 +30,15 @@ __global__ void update2nd_q_k(float *__restrict__ w0, const float *__restrict__ 
 // one CTA per (trace, y tap), threads over the x-z taps (z fastest)
 __global__ void inject_scatter_k(TraceDev t, int it, float *__restrict__ w0, const float *__restrict__ vel, int nx,
                                  int nz) {
+  dep_launch();
   const int r = t.ids ? t.ids[blockIdx.x] : blockIdx.x;
   const int *o = t.off + 3 * r, *l = t.len + 3 * r;
   const int lx = l[0], lz = l[2];
   const int iy = blockIdx.y;
-  if (iy >= l[1]) return;
   const float val = t.traces[(long long)r * t.nt + it] * t.scaler;
   const int ntap = lx * lz;
+  dep_wait();
+  if (iy >= l[1]) return;
   for (int k = threadIdx.x; k < ntap; k += blockDim.x) {
     const int iz = k % lz, ix = k / lz;
     const float cy = val * t.ky[(long long)r * t.ly + iy];
@@ -60,12 +63,13 @@ constexpr int kInjTile = kGroupTile, kInjChunk = 32, kInjSplit = 4, kInjRows = k
 __global__ void __launch_bounds__(256) inject_group_k(GroupDev g, TraceDev t, int it, float *__restrict__ w0,
                                                       const float *__restrict__ vel, int nx, int ny, int nz) {
   constexpr int CELLS = kInjRows * kInjTile;
+  dep_launch();
   __shared__ float s_xy[CELLS], s_kx[kInjChunk][kInjTile], s_ky[kInjChunk][kInjRows];
   __shared__ int4 s_box[kInjChunk];
   const int tile = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;  // 8 warps
   const int x0 = g.tile_xy[2 * tile], y0 = g.tile_xy[2 * tile + 1] + blockIdx.y * kInjRows;
   const int b = g.tile_ptr[tile], e = g.tile_ptr[tile + 1];
-  if (y0 >= ny) return;
+  if (y0 >= ny) return dep_wait();
   const int c = threadIdx.x, lx = c % kInjTile, ly = c / kInjTile;
   float acc = 0.f;
   for (int k0 = b; k0 < e; k0 += kInjChunk) {
@@ -112,6 +116,7 @@ __global__ void __launch_bounds__(256) inject_group_k(GroupDev g, TraceDev t, in
       }
   }
   if (c < CELLS) s_xy[c] = acc;
+  dep_wait();  // only constants and samples were read so far
   __syncthreads();
   const int lz = g.lz;
 #pragma unroll 4
@@ -175,6 +180,8 @@ __device__ __forceinline__ float extract_box(const TraceDev &t, int r, const flo
 // one warp per receiver over its kernel box
 __global__ void extract_direct_k(TraceDev t, const float *__restrict__ w0, float *__restrict__ out, int jt, int nt_out,
                                  int nx, int nz) {
+  dep_launch();
+  dep_wait();
   const int k0 = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
   if (k0 >= (t.ids ? t.nids : t.ntr)) return;
@@ -196,6 +203,8 @@ __global__ void __launch_bounds__(256) extract_zplane_k(GroupDev g, const float 
   const int ix = g.tile_xy[2 * tile] + c % T, iy = g.tile_xy[2 * tile + 1] + c / T;
   const bool in = c < T * T && ix < nx && iy < ny;
   float acc = 0.f;
+  dep_launch();
+  dep_wait();
   if (in) {
     const float *p = w0 + ((long long)iy * nx + ix) * nz + g.offz;
 #pragma unroll 5
@@ -215,12 +224,14 @@ __global__ void __launch_bounds__(256) extract_xy_k(GroupDev g, TraceDev t, cons
                                                     float *__restrict__ out, int jt, int nt_out, int nx) {
   const int m = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
-  if (m >= g.ntr) return;
+  dep_launch();
+  if (m >= g.ntr) return dep_wait();
   const int4 rec = g.members[m];
   const int lx = rec.z, ly = rec.w;
   const float *kx = t.kx + (long long)rec.x * t.lx, *ky = t.ky + (long long)rec.x * t.ly;
   const float *p = plane + rec.y;
   float acc = 0.f;
+  dep_wait();
   if (lx > 0) {
     int iy = lane / lx, ix = lane - iy * lx;
     const int sy = 32 / lx, sx = 32 - sy * lx;
@@ -246,6 +257,8 @@ __global__ void __launch_bounds__(256) extract_xy_k(GroupDev g, TraceDev t, cons
 
 // per-slab max |w| (one CTA per y slab)
 __global__ void slab_max_k(const float *__restrict__ w, float *__restrict__ slab, uint16_t *c16, int fmt, long long nxz) {
+  dep_launch();
+  dep_wait();
   const int iy = blockIdx.x;
   const float *p = w + (long long)iy * nxz;
   float m = 0.f;
@@ -357,12 +370,14 @@ void launch_inject_scatter(const TraceDev &t, int it, float *w0, const float *ve
   (void)ny;
   const int cnt = t.ids ? t.nids : t.ntr;
   if (cnt <= 0 || it < 0 || it >= t.nt) return;
-  inject_scatter_k<<<dim3(cnt, t.ly), 256, 0, st>>>(t, it, w0, vel, nx, nz);
+  launch_dep(inject_scatter_k, dim3(cnt, t.ly), 256, 0, st, t, it, w0, vel, nx, nz);
 }
 
 // Batched injection: block (trace, y row of its kernel, shot); the same
 // scatter as inject_scatter_k into the step output of each shot.
 __global__ void batch_inject_k(const IsoBatchShot *__restrict__ shots, int it_src, int it) {
+  dep_launch();
+  dep_wait();
   const IsoBatchShot &S = shots[blockIdx.z];
   const TraceDev &t = S.inj;
   const int r = blockIdx.x;
@@ -387,6 +402,8 @@ __global__ void batch_inject_k(const IsoBatchShot *__restrict__ shots, int it_sr
 
 // Batched extraction: a warp per receiver (extract_direct_k), blockIdx.y = shot.
 __global__ void batch_extract_k(const IsoBatchShot *__restrict__ shots, int jt, int it) {
+  dep_launch();
+  dep_wait();
   const IsoBatchShot &S = shots[blockIdx.y];
   const TraceDev &t = S.ext;
   const int r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
@@ -401,12 +418,12 @@ __global__ void batch_extract_k(const IsoBatchShot *__restrict__ shots, int jt, 
 void launch_batch_inject(const IsoBatchShot *shots, int nactive, int max_ntr, int max_ly, int it_src, int it,
                          cudaStream_t st) {
   if (nactive <= 0 || max_ntr <= 0 || max_ly <= 0) return;
-  batch_inject_k<<<dim3(max_ntr, max_ly, nactive), 256, 0, st>>>(shots, it_src, it);
+  launch_dep(batch_inject_k, dim3(max_ntr, max_ly, nactive), 256, 0, st, shots, it_src, it);
 }
 
 void launch_batch_extract(const IsoBatchShot *shots, int nactive, int max_ntr, int jt, int it, cudaStream_t st) {
   if (nactive <= 0 || max_ntr <= 0) return;
-  batch_extract_k<<<dim3((max_ntr + 7) / 8, nactive), 256, 0, st>>>(shots, jt, it);
+  launch_dep(batch_extract_k, dim3((max_ntr + 7) / 8, nactive), 256, 0, st, shots, jt, it);
 }
 
 // ---- FP16 wavefield state ----------------------------------------------------
@@ -550,7 +567,7 @@ void launch_inject_group(const GroupDev &gr, const TraceDev &t, int it, float *p
                          int nx, int ny, int nz, cudaStream_t st) {
   (void)plane;
   if (gr.ntiles <= 0 || it < 0 || it >= t.nt) return;
-  inject_group_k<<<dim3(gr.ntiles, kInjSplit), 256, 0, st>>>(gr, t, it, w0, vel, nx, ny, nz);
+  launch_dep(inject_group_k, dim3(gr.ntiles, kInjSplit), 256, 0, st, gr, t, it, w0, vel, nx, ny, nz);
 }
 
 void launch_extract_direct(const TraceDev &t, const float *w0, float *out, int jt, int nt_out, int nx, int ny, int nz,
@@ -558,18 +575,18 @@ void launch_extract_direct(const TraceDev &t, const float *w0, float *out, int j
   (void)ny;
   const int cnt = t.ids ? t.nids : t.ntr;
   if (cnt <= 0 || jt < 0 || jt >= nt_out) return;
-  extract_direct_k<<<(cnt + 7) / 8, 256, 0, st>>>(t, w0, out, jt, nt_out, nx, nz);
+  launch_dep(extract_direct_k, (cnt + 7) / 8, 256, 0, st, t, w0, out, jt, nt_out, nx, nz);
 }
 
 void launch_extract_group(const GroupDev &gr, const TraceDev &t, const float *w0, float *plane, float *out, int jt,
                           int nt_out, int nx, int ny, int nz, cudaStream_t st) {
   if (gr.ntiles <= 0 || jt < 0 || jt >= nt_out) return;
-  extract_zplane_k<<<dim3(gr.ntiles, (gr.tile * gr.tile + 63) / 64), 256, 0, st>>>(gr, w0, plane, nx, ny, nz);
-  extract_xy_k<<<(gr.ntr + 7) / 8, 256, 0, st>>>(gr, t, plane, out, jt, nt_out, nx);
+  launch_dep(extract_zplane_k, dim3(gr.ntiles, (gr.tile * gr.tile + 63) / 64), 256, 0, st, gr, w0, plane, nx, ny, nz);
+  launch_dep(extract_xy_k, (gr.ntr + 7) / 8, 256, 0, st, gr, t, plane, out, jt, nt_out, nx);
 }
 
 void launch_slab_max(const float *w, float *slab, uint16_t *c16_base, int fmt, int nx, int ny, int nz, cudaStream_t st) {
-  slab_max_k<<<ny, 1024, 0, st>>>(w, slab, c16_base, fmt, (long long)nx * nz);
+  launch_dep(slab_max_k, ny, 1024, 0, st, w, slab, c16_base, fmt, (long long)nx * nz);
 }
 
 void launch_fused_io(const FusedIo &io, const float *u, int nx, int ny, int nz, cudaStream_t st) {

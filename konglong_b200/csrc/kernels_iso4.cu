@@ -18,6 +18,7 @@
 #include <type_traits>
 
 #include "kernel_api.h"
+#include "launch.cuh"
 #include "pml4.cuh"
 #include "tma.cuh"
 
@@ -379,8 +380,10 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
     for (int k = 0; k < SB; k++) mbar_init(&s.bar_b[k], 1);
     mbar_fence_init();
   }
+  dep_launch();
   if constexpr (EDGE) fill_pml_co(s.co, a.pml, g, iz0, ix0, tzq, tx);
   __syncthreads();
+  dep_wait();
   int last_a = y0 - 1, last_b = y0 - 1;  // last planes the producer issued
   if (producer) {
     for (int p = y0; p < min(y0 + R4 + P, y1 + R4); p++) issue_a(p), last_a = p;
@@ -507,7 +510,7 @@ template <int TX, int P, bool EDGE>
 void tma4_launch(const IsoArgs &a, const Tile4 *tiles, int ntiles, const CUtensorMap &w1, const CUtensorMap &w0,
                  const CUtensorMap &vel, int *err, int mode, int pml3d, cudaStream_t st) {
   const size_t smem = sizeof(Iso4Smem<TX, P>);
-#define L_(M, P3) iso_fd8_tma4<TX, P, M, P3, EDGE><<<ntiles, dim3(8, TX), smem, st>>>(a, tiles, w1, w0, vel, err)
+#define L_(M, P3) launch_dep(iso_fd8_tma4<TX, P, M, P3, EDGE>, ntiles, dim3(8, TX), smem, st, a, tiles, w1, w0, vel, err)
   if (pml3d) {
     if (mode == 0) L_(0, true);
     else if (mode == 1) L_(1, true);

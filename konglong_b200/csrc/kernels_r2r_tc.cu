@@ -41,6 +41,7 @@
 #include <cstdint>
 
 #include "kernel_api.h"
+#include "launch.cuh"
 #include "rtm_b200.h"
 #include "tma.cuh"
 
@@ -160,6 +161,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const uint32_t ncols = nw <= 32 ? 32 : nw <= 64 ? 64 : nw <= 128 ? 128 : nw <= 256 ? 256 : 512;
   const int nkb = (n + kTcBK - 1) / kTcBK;
 
+  dep_launch();
+  dep_wait();
   if (tid == 0) {
     for (int i = 0; i < S; i++) mbar_init(rawf + i, 33), mbar_init(conv + i, 64), mbar_init(empty + i, 1);
     mbar_init(accf, 1);
@@ -427,7 +430,7 @@ void launch_r2r_tc(int axis, const float *in, float *out, const unsigned char *B
   const int S = tc_stages(npad), mode = axis == 2 ? 0 : 1;
 #define RTM_TC_LAUNCH(MODE, SS) \
   if (mode == MODE && S == SS)                                                                               \
-    r2r_tc_k<MODE, SS><<<(unsigned)tiles, kTcThreads, sm, st>>>(in, out, Bg, n, npad, geo, err);
+    launch_dep(r2r_tc_k<MODE, SS>, (unsigned)tiles, kTcThreads, sm, st, in, out, Bg, n, npad, geo, err);
   RTM_TC_ALL(RTM_TC_LAUNCH)
 #undef RTM_TC_LAUNCH
 }

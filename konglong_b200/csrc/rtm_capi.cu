@@ -1,6 +1,5 @@
 // rtm_capi.cu - the engine behind include/rtm_b200.h: device state of one shot,
-// the time-loop drivers (Propagator::modelling / migration) captured as CUDA
-// graphs, and every extern "C" entry point.  No entry point throws or aborts;
+// the time-loop drivers (Propagator::modelling / migration), and every extern "C" entry point.  No entry point throws or aborts;
 // CUDA failures become RTM_ERR_CUDA with the message kept on the handle.
 #include <cuda_fp16.h>
 
@@ -87,8 +86,8 @@ struct Engine {
   char *snaps = nullptr;
   // snapshot offload (rtm_snapshot_offload): the slots live in pinned host memory and
   // `nstage` device slots (snaps) stage them; slot s uses staging slot s % nstage.
-  // Copies run on st_copy, forked from st by events and joined back before every
-  // graph capture ends; stage_ev[k] marks the last copy into / out of staging slot k.
+  // Copies run on st_copy, forked from st by events and joined back at the end of every
+  // loop; stage_ev[k] marks the last copy into / out of staging slot k.
   float *illum = nullptr;  // source illumination (rtm_illum_setup), accumulated by the imaging condition
   int illum_on = 0;
   // imaging condition (rtm_image_condition): 0 zero-lag correlation fused into the
@@ -1092,53 +1091,28 @@ static int stage_ready(Engine *h, int s) {
   h->stage_wait[k] = false;
   return RTM_OK;
 }
-// join every copy back into st (before a graph capture ends, and after a loop)
+// join every copy back into st (at the end of a loop)
 static int stage_join(Engine *h) {
   if (!h->nstage) return RTM_OK;
   for (int k = 0; k < h->nstage; k++) TRY(stage_ready(h, k));
   return RTM_OK;
 }
 
-// Runs fn(step index) for `count` steps inside CUDA graphs of up to `chunk`
-// steps each, timed with events on the engine's stream; every snapshot copy
-// forked from the engine stream is joined back before a capture ends.
-template <typename F> static int run_graphs(Engine *h, int count, F fn) {
-  const int chunk = 256;
+// Runs fn(step index) for `count` steps, timed with events on the engine's
+// stream.  Plain launches: the host submits a step's 3-12 kernels in less time
+// than the GPU takes for them, and the first starts at once; capturing and
+// instantiating a CUDA graph of a loop that runs once cost 3-4 us per launch
+// before its first kernel could start (601 x 300 line shot of 50 steps: 1.69 ->
+// 1.44 ms, 128^3 shot of 100 steps: 5.2 -> 4.8 ms without it).
+template <typename F> static int run_loop(Engine *h, int count, F fn) {
   h->launches = 0;
   CK(cudaEventRecord(h->ev0, h->st));
-  if (h->prof_on) {  // eager launches bracketed by events (no graph)
-    for (int s = 0; s < count; s++) TRY(fn(s));
-    TRY(stage_join(h));
-    CK(cudaEventRecord(h->ev1, h->st));
-    CK(cudaEventSynchronize(h->ev1));
-    CK(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
-    prof_collect(h);
-    return check_flag(h);
-  }
-  for (int s0 = 0; s0 < count; s0 += chunk) {
-    const int s1 = std::min(count, s0 + chunk);
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
-    int rc = RTM_OK;
-    for (int s = s0; s < s1 && rc == RTM_OK; s++) rc = fn(s);
-    if (rc == RTM_OK) rc = stage_join(h);
-    cudaError_t ec = cudaStreamEndCapture(h->st, &g);
-    if (rc != RTM_OK) {
-      if (g) cudaGraphDestroy(g);
-      return rc;
-    }
-    if (ec != cudaSuccess) return cuda_fail(ec, "cudaStreamEndCapture", h);
-    cudaGraphExec_t ge = nullptr;
-    cudaError_t ei = cudaGraphInstantiate(&ge, g, 0);
-    cudaGraphDestroy(g);
-    if (ei != cudaSuccess) return cuda_fail(ei, "cudaGraphInstantiate", h);
-    cudaError_t el = cudaGraphLaunch(ge, h->st);
-    cudaGraphExecDestroy(ge);
-    if (el != cudaSuccess) return cuda_fail(el, "cudaGraphLaunch", h);
-  }
+  for (int s = 0; s < count; s++) TRY(fn(s));
+  TRY(stage_join(h));
   CK(cudaEventRecord(h->ev1, h->st));
   CK(cudaEventSynchronize(h->ev1));
   CK(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
+  if (h->prof_on) prof_collect(h);
   return check_flag(h);
 }
 
@@ -1376,8 +1350,7 @@ static int batch_upload(rtm_batch *b, const std::vector<int> &order, std::vector
 }
 
 // `count` steps of the shots in `order` (sorted by step count, descending:
-// the active shots of step it are the prefix with nts > it), as CUDA graphs
-// of up to 256 steps.  extract: ntratio > 0 gathers receivers every ntratio steps.
+// the active shots of step it are the prefix with nts > it).  extract: ntratio > 0 gathers receivers every ntratio steps.
 static int batch_run(rtm_batch *b, const std::vector<int> &order, const std::vector<int> &nts_sorted, int count,
                      int it_shift, int ntratio) {
   std::vector<int> start;
@@ -1398,31 +1371,10 @@ static int batch_run(rtm_batch *b, const std::vector<int> &order, const std::vec
     if (ntratio > 0 && it % ntratio == 0) launch_batch_extract(b->d_shots, na, max_ext, it / ntratio, it, b->st);
   };
   if (cudaEventRecord(b->ev0, b->st)) return RTM_ERR_CUDA;
-  for (int s0 = 0; s0 < count; s0 += 256) {
-    const int s1 = std::min(count, s0 + 256);
-    cudaGraph_t g = nullptr;
-    if (cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal)) return RTM_ERR_CUDA;
-    for (int it = s0; it < s1; it++) step(it);
-    cudaError_t ec = cudaStreamEndCapture(b->st, &g);
-    if (ec != cudaSuccess) {
-      b->err = std::string("batch graph capture: ") + cudaGetErrorString(ec);
-      cudaGetLastError();
-      return RTM_ERR_CUDA;
-    }
-    cudaGraphExec_t ge = nullptr;
-    cudaError_t ei = cudaGraphInstantiate(&ge, g, 0);
-    cudaGraphDestroy(g);
-    if (ei != cudaSuccess) {
-      b->err = std::string("batch graph instantiate: ") + cudaGetErrorString(ei);
-      cudaGetLastError();
-      return RTM_ERR_CUDA;
-    }
-    cudaError_t el = cudaGraphLaunch(ge, b->st);
-    cudaGraphExecDestroy(ge);
-    if (el != cudaSuccess) {
-      b->err = std::string("batch graph launch: ") + cudaGetErrorString(el);
-      return RTM_ERR_CUDA;
-    }
+  for (int it = 0; it < count; it++) step(it);
+  if (cudaError_t el = cudaGetLastError()) {
+    b->err = std::string("batch launch: ") + cudaGetErrorString(el);
+    return RTM_ERR_CUDA;
   }
   if (cudaEventRecord(b->ev1, b->st) || cudaEventSynchronize(b->ev1)) {
     b->err = std::string("batch loop: ") + cudaGetErrorString(cudaGetLastError());
@@ -2317,7 +2269,7 @@ int rtm_modelling(rtm_handle *h, int nts, int it_shift, int ntratio) {
   TRY(rtm::ready(h));
   if (nts < 0 || ntratio < 1) return RTM_ERR_ARG;
   const int mode = h->c.use_q ? 2 : 1;
-  return rtm::run_graphs(h, nts, [&](int it) {
+  return rtm::run_loop(h, nts, [&](int it) {
     TRY(rtm::step_kernel(h, mode, rtm::io_none()));
     TRY(rtm::do_inject(h, it + it_shift));
     if (it % ntratio == 0) TRY(rtm::do_extract(h, it / ntratio));
@@ -2340,7 +2292,7 @@ int rtm_migration(rtm_handle *h, int dir, int it_begin, int it_end, int it_shift
   rtm::FusedIo pending = rtm::io_none();
   int pending_slot = -1;  // slot the pending store writes (offload: copied to the host after it)
   const bool off = h->nstage > 0;
-  int rc = rtm::run_graphs(h, count, [&](int s) {
+  int rc = rtm::run_loop(h, count, [&](int s) {
     const int it = it_begin + s * inc;
     TRY(rtm::step_kernel(h, mode, pending));
     if (off && pending.store) TRY(rtm::offload_d2h(h, pending_slot));

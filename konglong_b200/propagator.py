@@ -362,7 +362,7 @@ def checkpoint_slots_for_budget(nts_fwd, interval, slot_bytes, ckpt_bytes, budge
 class Batch:
     """Several ISO FD8 shots stepped together (rtm_batch_*): one persistent
     kernel per time step over every active shot's tiles, batched injection and
-    extraction, the time loop as CUDA graphs.  The shots keep their own state:
+    extraction.  The shots keep their own state:
     after `modelling`, each Propagator holds what its own `modelling` call
     would have produced."""
 
