@@ -346,9 +346,8 @@ def run_small_shots(args, ranks):
     """Batched small-shot workload (64 seeded shots, grids 96-256 per axis,
     500-2000 steps, receivers every step; ISO, or VTI with per-layer Thomsen
     parameters for small_shots_vti): every shot's full modelling run, once per
-    shot with its own CUDA-graph loop (per-shot launches) and once for all
-    shots together (persistent launches per step over every shot, batched
-    I/O).  Metric: shots per second of the batched run."""
+    shot by itself and once for all shots together (each on its own stream,
+    side by side on the device).  Metric: shots per second of the batched run."""
     from konglong_b200 import workloads as W
     from konglong_b200.propagator import Batch, Propagator, spread_coeffs
     from konglong_b200.spec import ISO, VTI
@@ -406,10 +405,10 @@ def run_small_shots(args, ranks):
     nshots = len(shots) * ranks.world
     return {"metric": "shots/s", "value": nshots / (ms * 1e-3), "unit": "shots/s", "ms": ms,
             "per_shot": {"value": len(shots) / (per_ms * 1e-3), "ms": per_ms,
-                         "what": "the same shots, one rtm_modelling (own CUDA-graph loop) per shot"},
+                         "what": "the same shots, one rtm_modelling after the other"},
             "gpts": R.aggregate_gpts(ranks.world, cell_steps, 1, ms),
             "roofline": {"bound": "hbm",
-                         "kernel": ("grad_fd8_batch + div_fd8_batch" if vti else "iso_fd8_batch") +
+                         "kernel": ("grad4_k + div4_k" if vti else "iso_fd8_tma4") +
                                    " (whole batched step)", "achieved": achieved,
                          "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": None,
                          "peak_source": peak_src,

@@ -478,28 +478,25 @@ int rtm_set_compressor(rtm_handle *h, rtm_ae *a);
  * reference (its WaveFieldCompress has no learned code). */
 int rtm_set_compressor_fallback(rtm_handle *h, float tau, float max_fraction);
 
-/* ---- Batched small shots (many shots, one persistent launch per step) ----
+/* ---- Batched small shots (many shots side by side on one device) ----
  * A batch steps several FD8 handles (no Q) of different grids and step counts
- * together: all ISO (each time step one persistent kernel over the column
- * tiles of every active shot) or all VTI, or all TTI (each step two persistent
- * kernels, the gradient and the divergence pass of the one-cell kernels; no
- * density, FP32 state), then one batched injection and one batched extraction
- * launch.  Each handle must have its model,
- * injection (and, optionally, extraction) set and be reset.
+ * together, all ISO, all VTI or all TTI (no density, FP32 state): each shot's
+ * own step, injection and extraction kernels on its own stream, the launches
+ * interleaved step by step, so that small grids share the chip.  Each handle must
+ * have its model, injection (and, optionally, extraction) set and be reset.
  * No reference counterpart: bgprtm runs one shot per process
  * (bgprtm/Propagator.cpp:1054-1260 per shot). */
 typedef struct rtm_batch rtm_batch;
 int rtm_batch_create(rtm_handle *const *shots, int nshots, rtm_batch **out);
 int rtm_batch_destroy(rtm_batch *b);
 /* rtm_modelling(shots[s], nts[s], it_shift, ntratio) for every shot at once:
- * same wavefields and traces (receiver sums may differ in the last bit from a
- * handle's grouped extraction). */
+ * same wavefields and traces. */
 int rtm_batch_modelling(rtm_batch *b, const int *nts, int it_shift, int ntratio);
 /* Device time of the last rtm_batch_modelling (ms). */
 int rtm_batch_last_ms(rtm_batch *b, float *ms);
-/* Times `steps` batched steps for each tile width / y-segment length the
- * batched kernel offers, keeps the fastest and returns its index; zeroes the
- * shots' wavefields, PML memory and traces (as rtm_reset). */
+/* Times `steps` batched steps with the shots' present kernels (0) and with the
+ * ones rtm_autotune chooses for each (1), keeps the faster and returns its index;
+ * zeroes the shots' wavefields, PML memory and traces (as rtm_reset). */
 int rtm_batch_autotune(rtm_batch *b, int steps, int *choice);
 
 /* Failure detection.  rtm_check_finite scans field RTM_FIELD_W0 / W1 / IMAGE on

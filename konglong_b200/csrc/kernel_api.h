@@ -27,16 +27,6 @@ struct IsoArgs {
   QDev q;
 };
 
-// one shot of a batched ISO step (device array): its step arguments, its two
-// wavefield buffers (w1 = wa on even steps) and its tile grid
-struct IsoBatchShot {
-  IsoArgs a;
-  float *wa, *wb;
-  int tiles_z, tiles_x, tiles_y;
-  TraceDev inj, ext;  // source traces (scatter) and receivers (gathered into ext_out)
-  float *ext_out;     // [ext.ntr][ext.nt]
-};
-
 // FP16 wavefield state (per-y-slab scale: value = half * scale[iy])
 struct StateF16 {
   const __half *w1;     // current field, scale s1
@@ -71,21 +61,6 @@ struct DivArgs {
   QDev q;
 };
 
-// one VTI / TTI shot of a batched two-pass step (device array): its pass
-// arguments, its two wavefield buffers (w1 = wa on even steps, as in
-// IsoBatchShot), its tile grid and y segment
-struct AnisoBatchShot {
-  GradArgs g;
-  DivArgs d;
-  float *wa, *wb;
-  int tiles_z, tiles_x, tiles_y, yseg;
-};
-constexpr int kAnisoBatchTX = 8;  // tile width of the batched two-pass kernels
-// one step (both passes) of every active VTI / TTI shot of a batch
-void launch_aniso_fd8_batch(const AnisoBatchShot *shots, const int *start, int nactive, int total, int it, int model,
-                            int ctas, cudaStream_t st);
-int aniso_batch_ctas_per_sm();
-
 // mode: 0 = operator only (w0 -= vel*L), 1 = + leapfrog update, 2 = + Q update
 void launch_iso_fd8(const IsoArgs &a, int mode, int pml3d, int tx, cudaStream_t st);
 // the same step with 4 z cells per thread (float4 rows; nz % 4 == 0), tile
@@ -93,17 +68,6 @@ void launch_iso_fd8(const IsoArgs &a, int mode, int pml3d, int tx, cudaStream_t 
 void launch_iso_fd8_v4(const IsoArgs &a, int mode, int pml3d, int tx, cudaStream_t st);
 // the CTAs per SM launch_iso_fd8_v4 keeps resident (leapfrog mode)
 int iso_v4_ctas_per_sm(int tx, int pml3d);
-// one step of every active shot of a batch (ISO, leapfrog): shots[0..nactive)
-// device array, start[] their first work items (start[nactive] = total)
-void launch_iso_fd8_batch(const IsoBatchShot *shots, const int *start, int nactive, int total, int it, int pml3d,
-                          int tx, int ctas, cudaStream_t st);
-// the CTAs per SM the batched ISO kernel keeps resident at tile width tx
-int iso_batch_ctas_per_sm(int tx, int pml3d);
-// batched source injection at trace sample it_src and receiver extraction at
-// sample jt, into the step-`it` output buffers of shots[0..nactive)
-void launch_batch_inject(const IsoBatchShot *shots, int nactive, int max_ntr, int max_ly, int it_src, int it,
-                         cudaStream_t st);
-void launch_batch_extract(const IsoBatchShot *shots, int nactive, int max_ntr, int jt, int it, cudaStream_t st);
 // one CTA per entry of tiles[0, ntiles) (column tiles of 32 z x tx x cells);
 // non-edge tiles hold no PML cell and run without the PML code
 void launch_grad_fd8(const GradArgs &a, const Tile4 *tiles, int ntiles, bool edge, int model, int tx,

@@ -135,8 +135,8 @@ __global__ void __launch_bounds__(256) inject_group_k(GroupDev g, TraceDev t, in
 // taps, so a load instruction reads eight short contiguous runs and the column
 // indices advance without divisions; kBoxU steps of columns are loaded before
 // the first is summed.  The flat tap index cost two integer divisions a tap
-// (the batch's 3072 receivers of 20^3 taps took 112 us), one step at a time
-// waited on memory for each (65 us).
+// (3072 receivers of 20^3 taps took 112 us), one step at a time waited on memory
+// for each (65 us; now 25).
 constexpr int kBoxZ = 5, kBoxU = 4;
 __device__ __forceinline__ float extract_box(const TraceDev &t, int r, const float *__restrict__ w0, int nx, int nz,
                                              int lane) {
@@ -371,59 +371,6 @@ void launch_inject_scatter(const TraceDev &t, int it, float *w0, const float *ve
   const int cnt = t.ids ? t.nids : t.ntr;
   if (cnt <= 0 || it < 0 || it >= t.nt) return;
   launch_dep(inject_scatter_k, dim3(cnt, t.ly), 256, 0, st, t, it, w0, vel, nx, nz);
-}
-
-// Batched injection: block (trace, y row of its kernel, shot); the same
-// scatter as inject_scatter_k into the step output of each shot.
-__global__ void batch_inject_k(const IsoBatchShot *__restrict__ shots, int it_src, int it) {
-  dep_launch();
-  dep_wait();
-  const IsoBatchShot &S = shots[blockIdx.z];
-  const TraceDev &t = S.inj;
-  const int r = blockIdx.x;
-  if (r >= t.ntr || it_src < 0 || it_src >= t.nt) return;
-  const int *o = t.off + 3 * r, *l = t.len + 3 * r;
-  const int lx = l[0], lz = l[2];
-  const int iy = blockIdx.y;
-  if (iy >= l[1]) return;
-  float *w0 = (it & 1) ? S.wa : S.wb;
-  const float *vel = S.a.vel;
-  const int nx = S.a.nx, nz = S.a.nz;
-  const float val = t.traces[(long long)r * t.nt + it_src] * t.scaler;
-  const int ntap = lx * lz;
-  for (int k = threadIdx.x; k < ntap; k += blockDim.x) {
-    const int iz = k % lz, ix = k / lz;
-    const float cy = val * t.ky[(long long)r * t.ly + iy];
-    const float cx = cy * t.kx[(long long)r * t.lx + ix];
-    const long long c = ((long long)(iy + o[1]) * nx + ix + o[0]) * nz + o[2] + iz;
-    atomicAdd(w0 + c, cx * t.kz[(long long)r * t.lz + iz] * vel[c]);
-  }
-}
-
-// Batched extraction: a warp per receiver (extract_direct_k), blockIdx.y = shot.
-__global__ void batch_extract_k(const IsoBatchShot *__restrict__ shots, int jt, int it) {
-  dep_launch();
-  dep_wait();
-  const IsoBatchShot &S = shots[blockIdx.y];
-  const TraceDev &t = S.ext;
-  const int r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int lane = threadIdx.x & 31;
-  if (r >= t.ntr || jt < 0 || jt >= t.nt) return;
-  const float *w0 = (it & 1) ? S.wa : S.wb;
-  const int nx = S.a.nx, nz = S.a.nz;
-  const float acc = extract_box(t, r, w0, nx, nz, lane);
-  if (lane == 0) S.ext_out[(long long)r * t.nt + jt] = acc;
-}
-
-void launch_batch_inject(const IsoBatchShot *shots, int nactive, int max_ntr, int max_ly, int it_src, int it,
-                         cudaStream_t st) {
-  if (nactive <= 0 || max_ntr <= 0 || max_ly <= 0) return;
-  launch_dep(batch_inject_k, dim3(max_ntr, max_ly, nactive), 256, 0, st, shots, it_src, it);
-}
-
-void launch_batch_extract(const IsoBatchShot *shots, int nactive, int max_ntr, int jt, int it, cudaStream_t st) {
-  if (nactive <= 0 || max_ntr <= 0) return;
-  launch_dep(batch_extract_k, dim3((max_ntr + 7) / 8, nactive), 256, 0, st, shots, jt, it);
 }
 
 // ---- FP16 wavefield state ----------------------------------------------------

@@ -364,6 +364,21 @@ static int iso4_tiles(Engine *h) {
 static int fd8_tiles(Engine *h) { return build_tiles(h, h->t_fd8, h->tx, h->yseg); }
 static int an4_tiles(Engine *h) { return build_tiles(h, h->t_an4, kAniso4TX, h->an4_yseg); }
 
+// the launch shape the autotuner chooses (FD8)
+struct LaunchShape {
+  int iso4, v4_tx, v4_shape, v4_yseg, tma_shape, tx, yseg, aniso4, an4_yseg;
+};
+static LaunchShape launch_shape(const Engine *h) {
+  return {h->iso4, h->v4_tx, h->v4_shape, h->v4_yseg, h->tma_shape, h->tx, h->yseg, h->aniso4, h->an4_yseg};
+}
+static int set_launch_shape(Engine *h, const LaunchShape &s) {
+  h->iso4 = s.iso4, h->v4_tx = s.v4_tx, h->v4_shape = s.v4_shape, h->v4_yseg = s.v4_yseg, h->tma_shape = s.tma_shape;
+  h->tx = s.tx, h->yseg = s.yseg, h->aniso4 = s.aniso4, h->an4_yseg = s.an4_yseg;
+  if (h->iso4 == 2) TRY(iso4_tiles(h));
+  if (h->aniso4) TRY(an4_tiles(h));
+  return h->c.engine == RTM_ENGINE_FD8 && !h->lap_iso() ? fd8_tiles(h) : (int)RTM_OK;
+}
+
 static int yseg_an4(Engine *h) { return yseg_v4(h, kAniso4TX, aniso4_ctas_per_sm()); }
 
 static int yseg_iso4(Engine *h) {
@@ -1262,125 +1277,52 @@ struct rtm_handle : Engine {};
 // ---- batched small shots ----------------------------------------------------
 struct rtm_batch {
   std::vector<rtm::Engine *> shots;
-  int device = 0, pml3d = 0;
-  cudaStream_t st = nullptr;
+  std::vector<cudaEvent_t> done;  // per shot: end of its loop on its own stream
+  int device = 0;
+  cudaStream_t st = nullptr;      // the streams fork from it and join it (timing)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.f;
-  int tx = 8, yseg = 0;  // tile width, y segment (0: whole y extent)
-  rtm::IsoBatchShot *d_shots = nullptr;    // every shot's I/O (and ISO step) arguments
-  rtm::AnisoBatchShot *d_ashots = nullptr;  // VTI / TTI batches: the two passes' arguments
-  int *d_start = nullptr;
-  int cap = 0;
-  int model = RTM_ISO;  // the shots' model type (ISO: one-pass kernel; VTI / TTI: two passes)
-  std::string err;
 };
 
 namespace rtm {
-// tile-shape candidates of the batched kernels: {tile width, y segment (0 =
-// whole y)}; the VTI / TTI passes take those of width kAnisoBatchTX
-static const int kBatchShapes[][2] = {{8, 0}, {8, 32}, {16, 0}, {16, 32}, {8, 16}};
-static const int kBatchNShapes = 5;
-
-// Device table of the shots in `order`, their first work items, and the
-// trace maxima of the batched I/O launches.
-static int batch_upload(rtm_batch *b, const std::vector<int> &order, std::vector<int> &start, int &max_inj,
-                        int &max_ly, int &max_ext) {
-  const int n = (int)order.size();
-  const bool aniso = b->model != RTM_ISO;
-  const int tx = aniso ? kAnisoBatchTX : b->tx;
-  std::vector<IsoBatchShot> hs(n);
-  std::vector<AnisoBatchShot> ha(aniso ? n : 0);
-  start.assign(n + 1, 0);
-  max_inj = max_ly = max_ext = 0;
+// nts[k] steps of every shot, each on its handle's own stream, the launches
+// interleaved step by step.  A small shot leaves most of the chip idle (128^3:
+// 432 PML tiles of a step's 21 us, 88 interior tiles of its 11 us, receiver
+// kernels of a few us); side by side the shots fill it with the kernels that
+// are fastest for each.  One persistent kernel over all shots' tiles, before,
+// could only be a kernel all shots share, the one-cell one: 0.88 ms a step for 12
+// shots of 96 - 160 cells an axis, as long as the shots one after the other.
+// ntratio > 0 records the receivers every ntratio steps.
+static int batch_run(rtm_batch *b, const int *nts, int it_shift, int ntratio) {
+  const int n = (int)b->shots.size();
+  Engine *h = nullptr;  // CK's error text
+  CK(cudaEventRecord(b->ev0, b->st));
+  int most = 0;
   for (int k = 0; k < n; k++) {
-    Engine *h = b->shots[order[k]];
-    const rtm_dims &d = h->d;
-    IsoBatchShot &S = hs[k];
-    IsoArgs &a = S.a;
-    a.nx = d.nx, a.ny = d.ny, a.nz = d.nz;
-    a.yseg = b->yseg > 0 ? std::min(b->yseg, d.ny) : d.ny;
-    a.w1 = h->w1, a.w0 = h->w0, a.vel = h->vel;
-    memcpy(a.c2x, h->c2x, sizeof a.c2x), memcpy(a.c2y, h->c2y, sizeof a.c2y), memcpy(a.c2z, h->c2z, sizeof a.c2z);
-    a.pml = pml_dev(h);
-    a.io = FusedIo{};
-    a.q = QDev{};
-    S.wa = h->w1, S.wb = h->w0;
-    S.tiles_z = (d.nz + 31) / 32, S.tiles_x = (d.nx + tx - 1) / tx, S.tiles_y = (d.ny + a.yseg - 1) / a.yseg;
-    S.inj = h->inj.dev(), S.ext = h->ext.dev(), S.ext_out = h->ext.out;
-    S.inj.ids = nullptr, S.ext.ids = nullptr;
-    if (aniso) {  // the one-cell passes' arguments of the engine's own step (no density, no Q, FP32 state)
-      AnisoBatchShot &A = ha[k];
-      GradArgs &g = A.g;
-      g.nx = d.nx, g.ny = d.ny, g.nz = d.nz, g.yseg = a.yseg, g.pml3d = h->c.pml3d;
-      g.px = h->px, g.py = h->py, g.pz = h->pz;
-      g.eps = h->eps, g.del = h->del, g.pjx = h->pjx, g.pjy = h->pjy;
-      memcpy(g.c1x, h->c1x, sizeof g.c1x), memcpy(g.c1y, h->c1y, sizeof g.c1y), memcpy(g.c1z, h->c1z, sizeof g.c1z);
-      g.pml = pml_dev(h);
-      DivArgs &v = A.d;
-      v.nx = d.nx, v.ny = d.ny, v.nz = d.nz, v.yseg = a.yseg, v.pml3d = h->c.pml3d;
-      v.px = h->px, v.py = h->py, v.pz = h->pz, v.vel = h->vel;
-      memcpy(v.c1x, h->c1x, sizeof v.c1x), memcpy(v.c1y, h->c1y, sizeof v.c1y), memcpy(v.c1z, h->c1z, sizeof v.c1z);
-      v.pml = pml_dev(h);
-      A.wa = S.wa, A.wb = S.wb;
-      A.tiles_z = S.tiles_z, A.tiles_x = S.tiles_x, A.tiles_y = S.tiles_y, A.yseg = a.yseg;
+    CK(cudaStreamWaitEvent(b->shots[k]->st, b->ev0, 0));
+    b->shots[k]->launches = 0;
+    most = std::max(most, nts[k]);
+  }
+  for (int it = 0; it < most; it++)
+    for (int k = 0; k < n; k++) {
+      if (it >= nts[k]) continue;
+      Engine *s = b->shots[k];
+      TRY(step_kernel(s, 1, io_none()));
+      TRY(do_inject(s, it + it_shift));
+      if (ntratio > 0 && it % ntratio == 0) TRY(do_extract(s, it / ntratio));
+      do_swap(s);
     }
-    start[k + 1] = start[k] + S.tiles_z * S.tiles_x * S.tiles_y;
-    max_inj = std::max(max_inj, h->inj.ntr), max_ly = std::max(max_ly, h->inj.ly);
-    max_ext = std::max(max_ext, h->ext.ntr);
+  for (int k = 0; k < n; k++) {
+    CK(cudaEventRecord(b->done[k], b->shots[k]->st));
+    CK(cudaStreamWaitEvent(b->st, b->done[k], 0));
   }
-  if (n > b->cap) {
-    cudaFree(b->d_shots), cudaFree(b->d_ashots), cudaFree(b->d_start);
-    b->d_shots = nullptr, b->d_ashots = nullptr, b->d_start = nullptr, b->cap = 0;
-    if (cudaMalloc(&b->d_shots, n * sizeof(IsoBatchShot)) != cudaSuccess ||
-        (aniso && cudaMalloc(&b->d_ashots, n * sizeof(AnisoBatchShot)) != cudaSuccess) ||
-        cudaMalloc(&b->d_start, (n + 1) * sizeof(int)) != cudaSuccess) {
-      cudaGetLastError();
-      b->err = "batch table allocation failed";
-      return RTM_ERR_NOMEM;
-    }
-    b->cap = n;
+  CK(cudaEventRecord(b->ev1, b->st));
+  CK(cudaEventSynchronize(b->ev1));
+  CK(cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1));
+  for (Engine *s : b->shots) {
+    if (s->prof_on) prof_collect(s);
+    TRY(check_flag(s));
   }
-  if (cudaMemcpyAsync(b->d_shots, hs.data(), n * sizeof(IsoBatchShot), cudaMemcpyHostToDevice, b->st) ||
-      (aniso && cudaMemcpyAsync(b->d_ashots, ha.data(), n * sizeof(AnisoBatchShot), cudaMemcpyHostToDevice, b->st)) ||
-      cudaMemcpyAsync(b->d_start, start.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, b->st)) {
-    b->err = "batch table upload failed";
-    return RTM_ERR_CUDA;
-  }
-  return RTM_OK;
-}
-
-// `count` steps of the shots in `order` (sorted by step count, descending:
-// the active shots of step it are the prefix with nts > it).  extract: ntratio > 0 gathers receivers every ntratio steps.
-static int batch_run(rtm_batch *b, const std::vector<int> &order, const std::vector<int> &nts_sorted, int count,
-                     int it_shift, int ntratio) {
-  std::vector<int> start;
-  int max_inj, max_ly, max_ext;
-  TRY(batch_upload(b, order, start, max_inj, max_ly, max_ext));
-  int num_sms = 0;
-  cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, b->device);
-  const bool aniso = b->model != RTM_ISO;
-  const int grid = (aniso ? aniso_batch_ctas_per_sm() : iso_batch_ctas_per_sm(b->tx, b->pml3d)) *
-                   (num_sms > 0 ? num_sms : 148);
-  const int n = (int)order.size();
-  auto step = [&](int it) {
-    int na = 0;
-    while (na < n && nts_sorted[na] > it) na++;
-    if (aniso) launch_aniso_fd8_batch(b->d_ashots, b->d_start, na, start[na], it, b->model, grid, b->st);
-    else launch_iso_fd8_batch(b->d_shots, b->d_start, na, start[na], it, b->pml3d, b->tx, grid, b->st);
-    launch_batch_inject(b->d_shots, na, max_inj, max_ly, it + it_shift, it, b->st);
-    if (ntratio > 0 && it % ntratio == 0) launch_batch_extract(b->d_shots, na, max_ext, it / ntratio, it, b->st);
-  };
-  if (cudaEventRecord(b->ev0, b->st)) return RTM_ERR_CUDA;
-  for (int it = 0; it < count; it++) step(it);
-  if (cudaError_t el = cudaGetLastError()) {
-    b->err = std::string("batch launch: ") + cudaGetErrorString(el);
-    return RTM_ERR_CUDA;
-  }
-  if (cudaEventRecord(b->ev1, b->st) || cudaEventSynchronize(b->ev1)) {
-    b->err = std::string("batch loop: ") + cudaGetErrorString(cudaGetLastError());
-    return RTM_ERR_CUDA;
-  }
-  cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1);
   return RTM_OK;
 }
 }  // namespace rtm
@@ -2465,7 +2407,7 @@ int rtm_batch_create(rtm_handle *const *shots, int nshots, rtm_batch **out) {
   rtm_batch *b = new rtm_batch();
   for (int k = 0; k < nshots; k++) {
     rtm::Engine *h = shots[k];
-    // every shot ISO on the Laplacian kernel, or every shot FD8 VTI (or TTI) on
+    // every shot ISO on the Laplacian kernels, or every shot FD8 VTI (or TTI) on
     // the two passes, leapfrog without Q or density, FP32 state, one device and
     // PML mode
     const bool iso = h && h->lap_iso();
@@ -2477,10 +2419,15 @@ int rtm_batch_create(rtm_handle *const *shots, int nshots, rtm_batch **out) {
     }
     b->shots.push_back(h);
   }
-  b->device = shots[0]->device, b->pml3d = shots[0]->c.pml3d, b->model = shots[0]->c.model_type;
+  b->device = shots[0]->device;
   cudaSetDevice(b->device);
-  if (cudaStreamCreate(&b->st) || cudaEventCreate(&b->ev0) ||  // blocking: ordered after the set-up uploads
-      cudaEventCreate(&b->ev1)) {
+  bool ok = !cudaStreamCreate(&b->st) && !cudaEventCreate(&b->ev0) && !cudaEventCreate(&b->ev1);
+  for (int k = 0; ok && k < nshots; k++) {
+    cudaEvent_t e = nullptr;
+    ok = !cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+    if (ok) b->done.push_back(e);
+  }
+  if (!ok) {
     cudaGetLastError();
     rtm_batch_destroy(b);
     return RTM_ERR_CUDA;
@@ -2493,7 +2440,7 @@ int rtm_batch_destroy(rtm_batch *b) {
   if (!b) return RTM_ERR_ARG;
   cudaSetDevice(b->device);
   if (b->st) cudaStreamSynchronize(b->st);
-  cudaFree(b->d_shots), cudaFree(b->d_ashots), cudaFree(b->d_start);
+  for (cudaEvent_t e : b->done) cudaEventDestroy(e);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->st) cudaStreamDestroy(b->st);
@@ -2504,24 +2451,9 @@ int rtm_batch_destroy(rtm_batch *b) {
 int rtm_batch_modelling(rtm_batch *b, const int *nts, int it_shift, int ntratio) {
   if (!b || !nts || ntratio < 1) return RTM_ERR_ARG;
   cudaSetDevice(b->device);
-  const int n = (int)b->shots.size();
-  for (int k = 0; k < n; k++)
+  for (size_t k = 0; k < b->shots.size(); k++)
     if (nts[k] < 0) return RTM_ERR_ARG;
-  // every handle's own stream must be idle before the batch stream touches its buffers
-  for (rtm::Engine *h : b->shots) CK(cudaStreamSynchronize(h->st));
-  std::vector<int> order(n);
-  for (int k = 0; k < n; k++) order[k] = k;
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return nts[x] > nts[y]; });
-  std::vector<int> sorted(n);
-  for (int k = 0; k < n; k++) sorted[k] = nts[order[k]];
-  TRY(rtm::batch_run(b, order, sorted, sorted.empty() ? 0 : sorted[0], it_shift, ntratio));
-  // each shot swapped its wavefields once per step
-  for (int k = 0; k < n; k++)
-    if (nts[k] & 1) {
-      std::swap(b->shots[k]->w0, b->shots[k]->w1);
-      b->shots[k]->iq0 = 1 - b->shots[k]->iq0;
-    }
-  return RTM_OK;
+  return rtm::batch_run(b, nts, it_shift, ntratio);
 }
 
 int rtm_batch_last_ms(rtm_batch *b, float *ms) {
@@ -2533,25 +2465,26 @@ int rtm_batch_last_ms(rtm_batch *b, float *ms) {
 int rtm_batch_autotune(rtm_batch *b, int steps, int *choice) {
   if (!b || steps < 1) return RTM_ERR_ARG;
   cudaSetDevice(b->device);
-  const int n = (int)b->shots.size();
-  for (rtm::Engine *h : b->shots) CK(cudaStreamSynchronize(h->st));
-  std::vector<int> order(n), sorted(n, steps);
-  for (int k = 0; k < n; k++) order[k] = k;
-  float best = 1e30f;
-  int bi = 0;
-  for (int c = 0; c < rtm::kBatchNShapes; c++) {
-    if (b->model != RTM_ISO && rtm::kBatchShapes[c][0] != rtm::kAnisoBatchTX) continue;
-    b->tx = rtm::kBatchShapes[c][0], b->yseg = rtm::kBatchShapes[c][1];
-    TRY(rtm::batch_run(b, order, sorted, 1, 0, 0));  // warm-up
-    TRY(rtm::batch_run(b, order, sorted, steps, 0, 0));
-    if (b->last_ms < best) best = b->last_ms, bi = c;
+  const std::vector<int> nts(b->shots.size(), steps);
+  // candidate 0: the shots' present kernels; 1: each shot's own autotuned ones
+  float ms[2] = {0.f, 0.f};
+  std::vector<rtm::LaunchShape> before;
+  for (rtm::Engine *h : b->shots) before.push_back(rtm::launch_shape(h));
+  for (int c = 0; c < 2; c++) {
+    if (c)
+      for (rtm::Engine *h : b->shots) TRY(rtm_autotune(static_cast<rtm_handle *>(h), steps, nullptr));
+    TRY(rtm::batch_run(b, std::vector<int>(nts.size(), 1).data(), 0, 0));  // warm-up
+    TRY(rtm::batch_run(b, nts.data(), 0, 0));
+    ms[c] = b->last_ms;
   }
-  b->tx = rtm::kBatchShapes[bi][0], b->yseg = rtm::kBatchShapes[bi][1];
-  for (rtm::Engine *h : b->shots) {
+  const int best = ms[1] < ms[0] ? 1 : 0;
+  for (size_t k = 0; k < b->shots.size(); k++) {
+    rtm::Engine *h = b->shots[k];
+    if (!best) TRY(rtm::set_launch_shape(h, before[k]));
     TRY(rtm::zero_state(h));
     CK(cudaStreamSynchronize(h->st));
   }
-  if (choice) *choice = bi;
+  if (choice) *choice = best;
   return RTM_OK;
 }
 

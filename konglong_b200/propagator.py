@@ -360,9 +360,8 @@ def checkpoint_slots_for_budget(nts_fwd, interval, slot_bytes, ckpt_bytes, budge
 
 
 class Batch:
-    """Several ISO FD8 shots stepped together (rtm_batch_*): one persistent
-    kernel per time step over every active shot's tiles, batched injection and
-    extraction.  The shots keep their own state:
+    """Several FD8 shots stepped together (rtm_batch_*), each on its own stream,
+    side by side on the device.  The shots keep their own state:
     after `modelling`, each Propagator holds what its own `modelling` call
     would have produced."""
 
@@ -386,7 +385,7 @@ class Batch:
             pass
 
     def autotune(self, steps=5):
-        """Fastest tile shape of the batched kernel (zeroes the shots' state)."""
+        """The faster of the shots' present and autotuned kernels (zeroes the shots' state)."""
         ch = C.c_int(0)
         _lib.check(self.L.rtm_batch_autotune(self.b, steps, C.byref(ch)), "rtm_batch_autotune")
         return ch.value
