@@ -30,7 +30,8 @@ struct TraceSetDev {
   int *ungrouped = nullptr;
   int n_ungrouped = 0;
   std::vector<GroupDev> groups;
-  std::vector<void *> group_allocs;
+  char *mem = nullptr;  // the block that holds all of the above
+  size_t cap = 0;
   TraceDev dev() const {
     TraceDev t{};
     t.ntr = ntr, t.lx = lx, t.ly = ly, t.lz = lz, t.nt = nt;
@@ -82,7 +83,7 @@ struct Engine {
   float *plane = nullptr;
   // snapshots
   int snap_fmt = 0, nslots = 0;
-  size_t slot_bytes = 0;
+  size_t slot_bytes = 0, snaps_bytes = 0;  // of a slot; of the slots' allocation
   char *snaps = nullptr;
   // snapshot offload (rtm_snapshot_offload): the slots live in pinned host memory and
   // `nstage` device slots (snaps) stage them; slot s uses staging slot s % nstage.
@@ -1141,16 +1142,43 @@ static int ready(Engine *h) {
   return RTM_OK;
 }
 
-// Host staging of the traces of a TraceSet and its grouping by z kernel.
+// The device tables of one TraceSet, laid out one behind the other (256-byte
+// aligned) for a single allocation and a single copy.  Every array by itself
+// cost an allocation and a synchronous copy (1.0 ms a set of 2304 receivers).
+struct TableBlock {
+  std::vector<char> host;  // the part that is copied
+  std::vector<std::pair<void **, size_t>> fix;
+  size_t end = 0;
+  size_t reserve(size_t bytes) {
+    const size_t o = end;
+    end = (end + bytes + 255) / 256 * 256;
+    return o;
+  }
+  // p takes the place of count elements of src (at least one element's room)
+  template <typename P, typename T> void add(P *&p, const T *src, size_t count) {
+    const size_t o = reserve(std::max<size_t>(1, count) * sizeof(T));
+    host.resize(end);
+    if (count) memcpy(host.data() + o, src, count * sizeof(T));
+    fix.push_back({(void **)&p, o});
+  }
+};
+
+// Host staging of the traces of a TraceSet and its grouping by z kernel.  The
+// block of the set before is taken again when it fits, unless more than kTableIdle
+// of it would lie idle: a shot's source and its receivers take turns in one set.
+constexpr size_t kTableIdle = size_t(64) << 20;
 static int upload_traces(Engine *h, TraceSetDev &t, int ntr, int lx, int ly, int lz, const int *off3, const int *len3,
                          const float *kx, const float *ky, const float *kz, const float *traces, int nt, float scaler,
                          bool extraction) {
-  for (void *p : {(void *)t.off, (void *)t.len, (void *)t.kx, (void *)t.ky, (void *)t.kz, (void *)t.traces,
-                  (void *)t.out, (void *)t.ungrouped})
-    h->release(p);
-  for (void *p : t.group_allocs) h->release(p);
+  char *mem = t.mem;
+  const size_t cap = t.cap;
   t = TraceSetDev{};
-  if (ntr <= 0) return RTM_OK;
+  t.mem = mem, t.cap = cap;
+  if (ntr <= 0) {
+    h->release(t.mem);
+    t = TraceSetDev{};
+    return RTM_OK;
+  }
   // validate every kernel box against the grid
   for (int r = 0; r < ntr; r++) {
     const int *o = off3 + 3 * r, *l = len3 + 3 * r;
@@ -1161,39 +1189,39 @@ static int upload_traces(Engine *h, TraceSetDev &t, int ntr, int lx, int ly, int
         return RTM_ERR_ARG;
       }
   }
-  t.ntr = ntr, t.lx = lx, t.ly = ly, t.lz = lz, t.nt = nt, t.scaler = scaler;
-  TRY(h->alloc(t.off, 3 * (size_t)ntr));
-  TRY(h->alloc(t.len, 3 * (size_t)ntr));
-  TRY(h->alloc(t.kx, (size_t)ntr * lx));
-  TRY(h->alloc(t.ky, (size_t)ntr * ly));
-  TRY(h->alloc(t.kz, (size_t)ntr * lz));
-  CK(cudaMemcpy(t.off, off3, 12 * (size_t)ntr, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(t.len, len3, 12 * (size_t)ntr, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(t.kx, kx, 4 * (size_t)ntr * lx, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(t.ky, ky, 4 * (size_t)ntr * ly, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(t.kz, kz, 4 * (size_t)ntr * lz, cudaMemcpyHostToDevice));
-  if (!extraction) {
-    TRY(h->alloc(t.traces, (size_t)ntr * nt));
-    CK(cudaMemcpy(t.traces, traces, 4 * (size_t)ntr * nt, cudaMemcpyHostToDevice));
-  } else {
-    TRY(h->alloc(t.out, (size_t)ntr * nt));
-    CK(cudaMemset(t.out, 0, 4 * (size_t)ntr * nt));
-  }
+  TableBlock tab;
+  tab.host.reserve((size_t)ntr * (4 * (6 + lx + ly + lz) + 10 * sizeof(int4)) + 8192);
+  TraceSetDev s;  // the new set; t stays empty if anything fails
+  s.ntr = ntr, s.lx = lx, s.ly = ly, s.lz = lz, s.nt = nt, s.scaler = scaler;
+  tab.add(s.off, off3, 3 * (size_t)ntr);
+  tab.add(s.len, len3, 3 * (size_t)ntr);
+  tab.add(s.kx, kx, (size_t)ntr * lx);
+  tab.add(s.ky, ky, (size_t)ntr * ly);
+  tab.add(s.kz, kz, (size_t)ntr * lz);
   // group traces whose z kernels are identical (first index, length, values)
   std::map<std::vector<uint32_t>, std::vector<int>> by_z;
+  std::vector<int> *same = nullptr;  // the group of the trace before
   for (int r = 0; r < ntr; r++) {
+    const int n = len3[3 * r + 2];
+    if (same && off3[3 * r + 2] == off3[3 * r - 1] && n == len3[3 * r - 1] &&
+        !memcmp(kz + (size_t)r * lz, kz + (size_t)(r - 1) * lz, 4 * (size_t)n)) {
+      same->push_back(r);
+      continue;
+    }
     std::vector<uint32_t> key;
     key.push_back((uint32_t)off3[3 * r + 2]);
-    key.push_back((uint32_t)len3[3 * r + 2]);
-    for (int k = 0; k < len3[3 * r + 2]; k++) {
+    key.push_back((uint32_t)n);
+    for (int k = 0; k < n; k++) {
       uint32_t b;
       memcpy(&b, kz + (size_t)r * lz + k, 4);
       key.push_back(b);
     }
-    by_z[key].push_back(r);
+    same = &by_z[key];
+    same->push_back(r);
   }
   std::vector<int> loose;
   const int T = kGroupTile;
+  s.groups.reserve(by_z.size());  // the table's places are filled in by address
   for (auto &kv : by_z) {
     const std::vector<int> &mem = kv.second;
     // the packed member tables hold 16-bit lengths; longer kernels go trace by trace
@@ -1231,28 +1259,32 @@ static int upload_traces(Engine *h, TraceSetDev &t, int ntr, int lx, int ly, int
         ptr.push_back((int)lst.size());
       }
     g.ntiles = (int)txy.size() / 2;
-    int *dxy, *dp;
-    int4 *dm, *dl;
-    float *dkz;
-    TRY(h->alloc(dm, mem.size()));
-    TRY(h->alloc(dkz, std::max(1, g.lz)));
-    TRY(h->alloc(dxy, std::max<size_t>(2, txy.size())));
-    TRY(h->alloc(dp, ptr.size()));
-    TRY(h->alloc(dl, std::max<size_t>(1, lst.size())));
-    t.group_allocs.insert(t.group_allocs.end(), {(void *)dm, dkz, dxy, dp, dl});
-    CK(cudaMemcpy(dm, recs.data(), sizeof(int4) * recs.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dkz, kz + (size_t)r0 * lz, 4 * g.lz, cudaMemcpyHostToDevice));
-    if (!txy.empty()) CK(cudaMemcpy(dxy, txy.data(), 4 * txy.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dp, ptr.data(), 4 * ptr.size(), cudaMemcpyHostToDevice));
-    if (!lst.empty()) CK(cudaMemcpy(dl, lst.data(), sizeof(int4) * lst.size(), cudaMemcpyHostToDevice));
-    g.members = dm, g.kz = dkz, g.tile_xy = dxy, g.tile_ptr = dp, g.tile_list = dl;
-    t.groups.push_back(g);
+    s.groups.push_back(g);
+    GroupDev &d = s.groups.back();
+    tab.add(d.members, recs.data(), recs.size());
+    tab.add(d.kz, kz + (size_t)r0 * lz, g.lz);
+    tab.add(d.tile_xy, txy.data(), txy.size());
+    tab.add(d.tile_ptr, ptr.data(), ptr.size());
+    tab.add(d.tile_list, lst.data(), lst.size());
   }
-  if (!loose.empty()) {
-    TRY(h->alloc(t.ungrouped, loose.size()));
-    CK(cudaMemcpy(t.ungrouped, loose.data(), 4 * loose.size(), cudaMemcpyHostToDevice));
-    t.n_ungrouped = (int)loose.size();
+  s.n_ungrouped = (int)loose.size();
+  if (!loose.empty()) tab.add(s.ungrouped, loose.data(), loose.size());
+  const size_t tbytes = 4 * (size_t)ntr * nt;  // the traces are copied from where they are
+  tab.fix.push_back({(void **)(extraction ? &s.out : &s.traces), tab.reserve(tbytes)});
+  if (t.cap < tab.end || t.cap - tab.end > kTableIdle) {
+    h->release(t.mem);
+    t.mem = nullptr, t.cap = 0;
+    TRY(h->alloc(t.mem, tab.end));
+    t.cap = tab.end;
   }
+  for (auto &f : tab.fix) *f.first = t.mem + f.second;
+  // on the handle's stream: behind any step that still reads the block's old tables
+  CK(cudaMemcpyAsync(t.mem, tab.host.data(), tab.host.size(), cudaMemcpyHostToDevice, h->st));
+  if (extraction) CK(cudaMemsetAsync(s.out, 0, tbytes, h->st));
+  else CK(cudaMemcpyAsync(s.traces, traces, tbytes, cudaMemcpyHostToDevice, h->st));
+  CK(cudaStreamSynchronize(h->st));
+  s.mem = t.mem, s.cap = t.cap;
+  t = std::move(s);
   if (!t.groups.empty() && !h->plane) TRY(h->alloc(h->plane, (size_t)h->d.nx * h->d.ny));
   return RTM_OK;
 }
@@ -1852,18 +1884,25 @@ int rtm_snapshot_setup(rtm_handle *h, int fmt, int nslots) {
   if (h->st_copy) cudaStreamSynchronize(h->st_copy);
   if (h->host_snaps) cudaFreeHost(h->host_snaps);
   h->host_snaps = nullptr, h->nstage = 0;
+  // slots of the same format and number are taken again (shot after shot in one
+  // handle: freeing and allocating 10 slots of 10 MB took 0.8 ms)
+  const size_t slot = rtm::slot_size(h, fmt);
+  const bool slabs = fmt == RTM_SNAP_C16 || fmt == RTM_SNAP_FP16S;
+  const bool same = h->snaps && h->snap_fmt == fmt && h->nslots == nslots && h->slot_bytes == slot &&
+                    h->snaps_bytes == slot * nslots && (!slabs || h->slabs) && (fmt != RTM_SNAP_AE || h->ae_scratch);
+  h->snap_fmt = fmt, h->nslots = nslots, h->slot0 = 0;
+  h->slot_bytes = slot;
+  h->stored.assign(nslots, 0);
+  if (same) return RTM_OK;
   h->release(h->snaps), h->release(h->slabs), h->release(h->ae_scratch);
   h->snaps = nullptr, h->slabs = nullptr, h->ae_scratch = nullptr;
-  h->snap_fmt = fmt, h->nslots = nslots, h->slot0 = 0;
-  h->slot_bytes = rtm::slot_size(h, fmt);
-  h->stored.assign(nslots, 0);
   if (!nslots) return RTM_OK;
   TRY(h->alloc(h->snaps, h->slot_bytes * nslots));
-  if (fmt == RTM_SNAP_C16 || fmt == RTM_SNAP_FP16S) TRY(h->alloc(h->slabs, (size_t)nslots * h->d.ny));
+  h->snaps_bytes = h->slot_bytes * nslots;
+  if (slabs) TRY(h->alloc(h->slabs, (size_t)nslots * h->d.ny));
   if (fmt == RTM_SNAP_AE) TRY(h->alloc(h->ae_scratch, h->n));
   return RTM_OK;
 }
-
 
 int rtm_checkpoint_setup(rtm_handle *h, int nckpt, size_t *bytes_each) {
   if (!h || nckpt < 0) return RTM_ERR_ARG;
@@ -1948,6 +1987,7 @@ int rtm_snapshot_offload(rtm_handle *h, int nstage) {
   h->release(h->snaps);
   h->snaps = nullptr;
   TRY(h->alloc(h->snaps, h->slot_bytes * nstage));
+  h->snaps_bytes = h->slot_bytes * nstage;
   if (cudaHostAlloc((void **)&h->host_snaps, h->slot_bytes * nslots, cudaHostAllocDefault) != cudaSuccess) {
     h->host_snaps = nullptr;
     h->err = "cudaHostAlloc of " + std::to_string(h->slot_bytes * nslots) + " bytes failed";

@@ -8,6 +8,7 @@ meaning.  Every call goes through the C ABI of include/rtm_b200.h; errors
 raise `RtmError` with the engine's message.  There is no CPU code path.
 """
 import ctypes as C
+import threading
 
 import numpy as np
 
@@ -262,7 +263,9 @@ class Propagator:
 
     # -- field access -------------------------------------------------------------------
     def get(self, field):
-        out = np.zeros(self.n, np.float32)
+        return self._read(field, np.empty(self.n, np.float32))
+
+    def _read(self, field, out):
         self._ck(self.L.rtm_get(self.h, field, out.ctypes.data), "rtm_get")
         return out
 
@@ -285,9 +288,17 @@ class Propagator:
         self.reset()
         self.image_setup(ntaper_t, ntaper_z, edge)
         self.set_injection(rcv, rcv_traces, self.spec.dt_dxyz)
-        self.migration(1, nt - 1, -1, it_shift, interval)
+        # a second host thread faults the result's pages in while the device runs
+        # the loop: a copy into untouched pages takes 8.9 ms for 41 MB, 2.0 ms else
+        image = np.empty(self.n, np.float32)
+        touch = threading.Thread(target=image.fill, args=(0,))
+        touch.start()
+        try:
+            self.migration(1, nt - 1, -1, it_shift, interval)
+        finally:
+            touch.join()
         bwd_ms = self.last_loop_ms
-        return self.get(FIELD_IMAGE), fwd_ms, bwd_ms
+        return self._read(FIELD_IMAGE, image), fwd_ms, bwd_ms
 
     def rtm_shot_checkpointed(self, src: TraceSet, src_traces, rcv: TraceSet, rcv_traces, nt, nts_fwd, interval,
                               seg_slots, snap_fmt=0, ntaper_t=0, ntaper_z=0, edge=1, it_shift=-1):
