@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "launch.cuh"
 #include "rtm_internal.cuh"
 
 struct rtm_ae;
@@ -117,7 +118,7 @@ bool iso_tma4_init();
 int iso_tma4_ctas_per_sm(int shape, int pml3d);
 void launch_iso_fd8_tma4(const IsoArgs &a, const Tile4 *tiles, int ntiles, bool edge, const CUtensorMap &w1,
                          const CUtensorMap &w0, const CUtensorMap &vel, int *err, int mode, int pml3d, int shape,
-                         cudaStream_t st);
+                         const LaunchPair &pair, cudaStream_t st);
 
 // FD8 VTI / TTI passes with 4 z cells per thread and TMA rings
 // (kernels_aniso4.cu), tile width kAniso4TX, nz % 4 == 0, FP32 state
@@ -138,9 +139,9 @@ constexpr int kDiv4QMax = 4;
 bool aniso4_init();         // shared-memory attributes (call outside any capture)
 int aniso4_ctas_per_sm();   // resident CTAs per SM of the interior divergence kernel
 void launch_grad4(const GradArgs &a, const Tile4 *tiles, int ntiles, bool edge, int model, const Grad4Maps &m,
-                  int *err, cudaStream_t st);
+                  int *err, const LaunchPair &pair, cudaStream_t st);
 void launch_div4(const DivArgs &a, const Tile4 *tiles, int ntiles, bool edge, int mode, const Div4Maps &m, int *err,
-                 cudaStream_t st);
+                 const LaunchPair &pair, cudaStream_t st);
 
 // shot illumination compensation: optional box smoothing (half widths hxy, hz),
 // damping factor from the mean (dsum: one double of scratch), image *= factor;

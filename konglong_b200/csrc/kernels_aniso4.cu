@@ -91,7 +91,7 @@ struct __align__(128) Grad4Smem {
 template <int TX, int P, int MODEL, int EDGE>
 __global__ void __launch_bounds__(8 * TX, EDGE ? kEdgeCtas : 0)
     grad4_k(const __grid_constant__ GradArgs a, const Tile4 *__restrict__ tiles, const __grid_constant__ Grad4Maps mp,
-            int *err) {
+            int *err, const LaunchPair pair) {
   constexpr int NM = MODEL == 3 ? 4 : MODEL == 2 ? 2 : 1;
   using S = Grad4Smem<TX, P, NM>;
   constexpr int SA = S::SA, SB = S::SB, HX = S::HX;
@@ -135,10 +135,8 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? kEdgeCtas : 0)
     for (int k = 0; k < SB; k++) mbar_init(&s.bar_b[k], 1);
     mbar_fence_init();
   }
-  dep_launch();
   if constexpr (EDGE != 0) fill_pml_co(s.co, a.pml, g, iz0, ix0, tzq, tx);
-  __syncthreads();
-  dep_wait();
+  pair_begin(pair, producer);
   int last_a = y0 - 1, last_b = y0 - 1;  // last planes the producer issued
   if (producer) {
     for (int p = y0; p < min(y0 + R4 + P, y1 + R4); p++) issue_a(p), last_a = p;
@@ -217,6 +215,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? kEdgeCtas : 0)
     for (int p = max(y0, last_a - SA + 1); p <= last_a; p++) mbar_drain(&s.bar_a[(p - y0) % SA], ((p - y0) / SA) & 1);
     for (int p = max(y0, last_b - SB + 1); p <= last_b; p++) mbar_drain(&s.bar_b[(p - y0) % SB], ((p - y0) / SB) & 1);
   }
+  pair_end(pair);
 }
 
 // ---- pass 2: divergence ---------------------------------------------------------
@@ -256,7 +255,7 @@ constexpr size_t div4_smem() {
 template <int TX, int P, int MODE, int EDGE, int QR>
 __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? kEdgeCtas : 0)
     div4_k(const __grid_constant__ DivArgs a, const Tile4 *__restrict__ tiles, const __grid_constant__ Div4Maps mp,
-           int *err) {
+           int *err, const LaunchPair pair) {
   using S = Div4Smem<TX, P>;
   constexpr int SA = S::SA, SB = S::SB;
   using QT = QType<QR>;
@@ -308,10 +307,8 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? kEdgeCtas : 0)
     for (int k = 0; k < SB; k++) mbar_init(&s.bar_b[k], 1);
     mbar_fence_init();
   }
-  dep_launch();
   if constexpr (EDGE != 0) fill_pml_co(s.co, a.pml, g, iz0, ix0, tzq, tx);
-  __syncthreads();
-  dep_wait();
+  pair_begin(pair, producer);
   // ring A carries planes y0+4 .. y1+3 only (the queue starts with planes
   // y0-4 .. y0+3 read from global memory), so every copy it gets is waited for
   int last_a = y0 + R4 - 1, last_b = y0 - 1;
@@ -391,6 +388,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? kEdgeCtas : 0)
       mbar_drain(&s.bar_a[(p - y0 - R4) % SA], ((p - y0 - R4) / SA) & 1);
     for (int p = max(y0, last_b - SB + 1); p <= last_b; p++) mbar_drain(&s.bar_b[(p - y0) % SB], ((p - y0) / SB) & 1);
   }
+  pair_end(pair);
 }
 
 // ---- host side -------------------------------------------------------------------
@@ -432,11 +430,11 @@ int aniso4_ctas_per_sm() {
 }
 
 void launch_grad4(const GradArgs &a, const Tile4 *tiles, int ntiles, bool edge, int model, const Grad4Maps &m,
-                  int *err, cudaStream_t st) {
+                  int *err, const LaunchPair &pair, cudaStream_t st) {
   if (ntiles <= 0) return;
   const dim3 block(8, kTX);
   const int e = !edge ? TILE_INT : a.pml3d ? TILE_PML3 : TILE_PML1;
-#define G_(MD, E) launch_dep(grad4_k<kTX, kP, MD, E>, ntiles, block, grad4_smem<kTX, kP, MD>(), st, a, tiles, m, err)
+#define G_(MD, E) launch_dep(grad4_k<kTX, kP, MD, E>, ntiles, block, grad4_smem<kTX, kP, MD>(), st, a, tiles, m, err, pair)
 #define E_(MD)                          \
   if (e == TILE_INT) G_(MD, TILE_INT);  \
   else if (e == TILE_PML1) G_(MD, TILE_PML1); \
@@ -451,11 +449,11 @@ void launch_grad4(const GradArgs &a, const Tile4 *tiles, int ntiles, bool edge, 
 }
 
 void launch_div4(const DivArgs &a, const Tile4 *tiles, int ntiles, bool edge, int mode, const Div4Maps &m, int *err,
-                 cudaStream_t st) {
+                 const LaunchPair &pair, cudaStream_t st) {
   if (ntiles <= 0) return;
   const dim3 block(8, kTX);
   const int e = !edge ? TILE_INT : a.pml3d ? TILE_PML3 : TILE_PML1;
-#define D_(MD, E, QR) launch_dep(div4_k<kTX, kP, MD, E, QR>, ntiles, block, div4_smem<kTX, kP, QR>(), st, a, tiles, m, err)
+#define D_(MD, E, QR) launch_dep(div4_k<kTX, kP, MD, E, QR>, ntiles, block, div4_smem<kTX, kP, QR>(), st, a, tiles, m, err, pair)
 #define E_(MD, QR)                              \
   if (e == TILE_INT) D_(MD, TILE_INT, QR);      \
   else if (e == TILE_PML1) D_(MD, TILE_PML1, QR); \

@@ -340,7 +340,8 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
                                                        const Tile4 *__restrict__ tiles,
                                                        const __grid_constant__ CUtensorMap map_w1,
                                                        const __grid_constant__ CUtensorMap map_w0,
-                                                       const __grid_constant__ CUtensorMap map_vel, int *err) {
+                                                       const __grid_constant__ CUtensorMap map_vel, int *err,
+                                                       const LaunchPair pair) {
   using S = Iso4Smem<TX, P>;
   constexpr int SA = S::SA, SB = S::SB, HX = S::HX;
   constexpr uint32_t BYTES_A = HX * 160, BYTES_B = 2 * TX * 128;
@@ -380,10 +381,8 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
     for (int k = 0; k < SB; k++) mbar_init(&s.bar_b[k], 1);
     mbar_fence_init();
   }
-  dep_launch();
   if constexpr (EDGE) fill_pml_co(s.co, a.pml, g, iz0, ix0, tzq, tx);
-  __syncthreads();
-  dep_wait();
+  pair_begin(pair, producer);
   int last_a = y0 - 1, last_b = y0 - 1;  // last planes the producer issued
   if (producer) {
     for (int p = y0; p < min(y0 + R4 + P, y1 + R4); p++) issue_a(p), last_a = p;
@@ -504,13 +503,14 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
     for (int p = max(y0, last_a - SA + 1); p <= last_a; p++) mbar_drain(&s.bar_a[(p - y0) % SA], ((p - y0) / SA) & 1);
     for (int p = max(y0, last_b - SB + 1); p <= last_b; p++) mbar_drain(&s.bar_b[(p - y0) % SB], ((p - y0) / SB) & 1);
   }
+  pair_end(pair);
 }
 
 template <int TX, int P, bool EDGE>
 void tma4_launch(const IsoArgs &a, const Tile4 *tiles, int ntiles, const CUtensorMap &w1, const CUtensorMap &w0,
-                 const CUtensorMap &vel, int *err, int mode, int pml3d, cudaStream_t st) {
+                 const CUtensorMap &vel, int *err, int mode, int pml3d, const LaunchPair &pair, cudaStream_t st) {
   const size_t smem = sizeof(Iso4Smem<TX, P>);
-#define L_(M, P3) launch_dep(iso_fd8_tma4<TX, P, M, P3, EDGE>, ntiles, dim3(8, TX), smem, st, a, tiles, w1, w0, vel, err)
+#define L_(M, P3) launch_dep(iso_fd8_tma4<TX, P, M, P3, EDGE>, ntiles, dim3(8, TX), smem, st, a, tiles, w1, w0, vel, err, pair)
   if (pml3d) {
     if (mode == 0) L_(0, true);
     else if (mode == 1) L_(1, true);
@@ -525,10 +525,10 @@ void tma4_launch(const IsoArgs &a, const Tile4 *tiles, int ntiles, const CUtenso
 
 template <int TX, int P>
 void tma4_shape(const IsoArgs &a, const Tile4 *tiles, int ntiles, bool edge, const CUtensorMap &w1,
-                const CUtensorMap &w0, const CUtensorMap &vel, int *err, int mode, int pml3d, cudaStream_t st) {
+                const CUtensorMap &w0, const CUtensorMap &vel, int *err, int mode, int pml3d, const LaunchPair &pair, cudaStream_t st) {
   if (ntiles <= 0) return;
-  if (edge) tma4_launch<TX, P, true>(a, tiles, ntiles, w1, w0, vel, err, mode, pml3d, st);
-  else tma4_launch<TX, P, false>(a, tiles, ntiles, w1, w0, vel, err, mode, pml3d, st);
+  if (edge) tma4_launch<TX, P, true>(a, tiles, ntiles, w1, w0, vel, err, mode, pml3d, pair, st);
+  else tma4_launch<TX, P, false>(a, tiles, ntiles, w1, w0, vel, err, mode, pml3d, pair, st);
 }
 
 template <int TX, int P, bool EDGE>
@@ -605,10 +605,10 @@ int iso_tma4_ctas_per_sm(int shape, int pml3d) {
 
 void launch_iso_fd8_tma4(const IsoArgs &a, const Tile4 *tiles, int ntiles, bool edge, const CUtensorMap &w1,
                          const CUtensorMap &w0, const CUtensorMap &vel, int *err, int mode, int pml3d, int shape,
-                         cudaStream_t st) {
-  if (shape == 0) tma4_shape<16, 2>(a, tiles, ntiles, edge, w1, w0, vel, err, mode, pml3d, st);
-  else if (shape == 1) tma4_shape<16, 4>(a, tiles, ntiles, edge, w1, w0, vel, err, mode, pml3d, st);
-  else tma4_shape<32, 2>(a, tiles, ntiles, edge, w1, w0, vel, err, mode, pml3d, st);
+                         const LaunchPair &pair, cudaStream_t st) {
+  if (shape == 0) tma4_shape<16, 2>(a, tiles, ntiles, edge, w1, w0, vel, err, mode, pml3d, pair, st);
+  else if (shape == 1) tma4_shape<16, 4>(a, tiles, ntiles, edge, w1, w0, vel, err, mode, pml3d, pair, st);
+  else tma4_shape<32, 2>(a, tiles, ntiles, edge, w1, w0, vel, err, mode, pml3d, pair, st);
 }
 
 }  // namespace rtm

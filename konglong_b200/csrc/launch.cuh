@@ -18,6 +18,50 @@ namespace rtm {
 __device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Two launches of one pass over disjoint tiles (PML tiles, then interior tiles),
+// the second free to run beside the first: the PML tiles come in one or two
+// uneven waves (813 tiles on 592 places: the SMs stood idle for a quarter of the
+// launch), and the interior tiles fill what they leave.  The first launch lets
+// the second in only after its own dep_wait(), so whatever both read is written
+// by then; block 0 says so in `flag` (release / acquire, a number of its own for
+// each pair), and a second launch that does not find its number waits as usual.  The
+// second launch calls dep_wait() as its last act instead of its first: its end
+// then implies the end of the first, and the kernel after it need wait for
+// nothing more.  No launch waits for one behind it: the second is let in when
+// every CTA of the first has its place.
+enum { PAIR_NONE = 0, PAIR_FIRST = 1, PAIR_SECOND = 2 };
+struct LaunchPair {
+  int role;
+  unsigned *flag;
+  unsigned number;
+};
+// in place of dep_launch(); __syncthreads(); dep_wait(): called by every thread,
+// after what the CTA prepares; `lead` is one thread, the one that issues copies
+__device__ __forceinline__ void pair_begin(const LaunchPair &p, bool lead) {
+  if (p.role == PAIR_FIRST) {
+    __syncthreads();
+    dep_wait();
+    if (lead) {
+      if (blockIdx.x == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p.flag), "r"(p.number) : "memory");
+      dep_launch();
+    }
+    return;
+  }
+  dep_launch();
+  int seen = 1;
+  if (p.role == PAIR_SECOND && lead) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.flag) : "memory");
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+    seen = v == p.number;
+  }
+  seen = __syncthreads_and(seen);
+  if (p.role == PAIR_NONE || !seen) dep_wait();
+}
+__device__ __forceinline__ void pair_end(const LaunchPair &p) {
+  if (p.role == PAIR_SECOND) dep_wait();
+}
+
 // k<<<grid, block, smem, st>>>(args...) with the attribute
 template <typename... P, typename... A>
 void launch_dep(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A &...args) {

@@ -124,6 +124,7 @@ struct Engine {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.f;
   int *dflag = nullptr;
+  unsigned *pair_flag = nullptr, pair_no = 0;  // LaunchPair's flag and the last pair's number
   int *nfflag = nullptr;  // result of the non-finite scan (allocated on first use)
   rtm_ae *ae = nullptr;      // learned compressor of RTM_SNAP_AE snapshots
   float ae_fb_tau = 0.f;     // FP16 fallback of learned snapshots: blocks above tau x the largest scale,
@@ -378,6 +379,16 @@ static int set_launch_shape(Engine *h, const LaunchShape &s) {
   if (h->iso4 == 2) TRY(iso4_tiles(h));
   if (h->aniso4) TRY(an4_tiles(h));
   return h->c.engine == RTM_ENGINE_FD8 && !h->lap_iso() ? fd8_tiles(h) : (int)RTM_OK;
+}
+
+// The PML tiles' and the interior tiles' launches of a pass, in that order: side
+// by side (launch.cuh) when there are both.
+static void launch_pair(Engine *h, const TileSet &t, LaunchPair &edge, LaunchPair &inner) {
+  edge = inner = {PAIR_NONE, h->pair_flag, 0};
+  if (!t.n_int || !t.n_edge) return;
+  if (++h->pair_no == 0) h->pair_no = 1;  // 0: the flag's first value
+  edge.role = PAIR_FIRST, inner.role = PAIR_SECOND;
+  edge.number = inner.number = h->pair_no;
 }
 
 static int yseg_an4(Engine *h) { return yseg_v4(h, kAniso4TX, aniso4_ctas_per_sm()); }
@@ -714,9 +725,11 @@ static int step_kernel(Engine *h, int mode, const FusedIo &io) {
         {
           const TileSet &t = h->t_iso;
           KScope k(h, RTM_K_ISO, (t.n_int > 0) + (t.n_edge > 0));
-          launch_iso_fd8_tma4(a, t.d, t.n_int, false, m1, m0, mv, h->dflag, mode, h->c.pml3d, h->v4_shape, h->st);
-          launch_iso_fd8_tma4(a, t.d + t.n_int, t.n_edge, true, m1, m0, mv, h->dflag, mode, h->c.pml3d, h->v4_shape,
+          LaunchPair pe, pi;
+          launch_pair(h, t, pe, pi);
+          launch_iso_fd8_tma4(a, t.d + t.n_int, t.n_edge, true, m1, m0, mv, h->dflag, mode, h->c.pml3d, h->v4_shape, pe,
                               h->st);
+          launch_iso_fd8_tma4(a, t.d, t.n_int, false, m1, m0, mv, h->dflag, mode, h->c.pml3d, h->v4_shape, pi, h->st);
         }
         return check_launch(h, "iso_fd8_tma4");
       }
@@ -777,14 +790,18 @@ static int step_kernel(Engine *h, int mode, const FusedIo &io) {
     if (ok) {
       {
         KScope k(h, RTM_K_GRAD, (t.n_int > 0) + (t.n_edge > 0));
-        launch_grad4(g, t.d, t.n_int, false, h->c.model_type, gm, h->dflag, h->st);
-        launch_grad4(g, t.d + t.n_int, t.n_edge, true, h->c.model_type, gm, h->dflag, h->st);
+        LaunchPair pe, pi;
+        launch_pair(h, t, pe, pi);
+        launch_grad4(g, t.d + t.n_int, t.n_edge, true, h->c.model_type, gm, h->dflag, pe, h->st);
+        launch_grad4(g, t.d, t.n_int, false, h->c.model_type, gm, h->dflag, pi, h->st);
       }
       TRY(check_launch(h, "grad4"));
       {
         KScope k(h, RTM_K_DIV, (t.n_int > 0) + (t.n_edge > 0));
-        launch_div4(v, t.d, t.n_int, false, mode, dm, h->dflag, h->st);
-        launch_div4(v, t.d + t.n_int, t.n_edge, true, mode, dm, h->dflag, h->st);
+        LaunchPair pe, pi;
+        launch_pair(h, t, pe, pi);
+        launch_div4(v, t.d + t.n_int, t.n_edge, true, mode, dm, h->dflag, pe, h->st);
+        launch_div4(v, t.d, t.n_int, false, mode, dm, h->dflag, pi, h->st);
       }
       return check_launch(h, "div4");
     }
@@ -1503,7 +1520,9 @@ int rtm_create(const rtm_dims *d, const rtm_config *c, rtm_handle **out) {
   } else if ((rc = h->alloc(h->w0, h->n)) || (rc = h->alloc(h->w1, h->n))) {
     return fail(rc);
   }
-  if ((rc = h->alloc(h->vel, h->n)) || (rc = h->alloc(h->dflag, 1))) return fail(rc);
+  if ((rc = h->alloc(h->vel, h->n)) || (rc = h->alloc(h->dflag, 1)) || (rc = h->alloc(h->pair_flag, 1)))
+    return fail(rc);
+  cudaMemset(h->pair_flag, 0, sizeof(unsigned));
   const bool first_deriv = !h->lap_iso();
   if (first_deriv) {
     if ((rc = h->alloc(h->px, h->n)) || (rc = h->alloc(h->pz, h->n)) || (d->ny > 1 && (rc = h->alloc(h->py, h->n))))
