@@ -172,14 +172,6 @@ __global__ void adam_k(float *p, const float *g, float *m, float *v, int n, floa
   p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
-// Morton index of cell (x, y, z) of an 8^3 block: bits z0 y0 x0 z1 y1 x1 z2 y2 x2
-__host__ __device__ __forceinline__ int morton8(int x, int y, int z) {
-  int m = 0;
-#pragma unroll
-  for (int b = 0; b < 3; b++) m |= (((z >> b) & 1) << (3 * b)) | (((y >> b) & 1) << (3 * b + 1)) | (((x >> b) & 1) << (3 * b + 2));
-  return m;
-}
-
 }  // namespace
 }  // namespace rtm
 
@@ -190,6 +182,7 @@ struct rtm_ae {
   float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // params, grads, Adam moments
   float *loss = nullptr;
   int step = 0;
+  int wave_enc[2] = {1, 1}, wave_dec[2] = {1, 1};  // CTAs of one wave: cell by cell, 16-byte accesses
   // workspace for `cap` blocks: normalised input, per-layer outputs; training
   // also keeps pre-activations and gradients
   int cap = 0, cap_train = 0;
@@ -286,228 +279,344 @@ void ae_loss_grad(rtm_ae *a, int n) {
 constexpr int kChunkBlocks = 8192;  // blocks per encode / decode pass over a volume
 
 // ---- fused inference over a volume -------------------------------------------
-// One warp per 8^3 block, a CTA of 4 warps per 4 blocks consecutive in z (32 z
-// cells of each x / y row: 128-byte rows in and out).  The CTA stages the
-// encoder (or decoder) weights once as BF16 in shared memory; each warp runs
-// its block through the four layers with the layer outputs in shared memory
-// (BF16: the next layer's operand rounding) and writes only the latent and the
-// scale (or the decoded cells).  Each output element is the same mma.sync
-// chain over k in steps of 16 as in gemm_bf16_k, with the same operand
-// roundings, bias and activation, so the results equal the layer-by-layer
-// path bit for bit.  Rows of a layer beyond its M (8 or 1 per block) and
-// columns beyond K (8 in E1) enter the MMA as zeros.
-constexpr int kFusedWarps = 4;
+// 16 blocks (consecutive in the latents' order, z fastest) are the 16 rows of
+// every MMA, and a CTA's 8 warps are the 8 octants of the blocks (the row index
+// of E2 / D2 within a block).  With a block a row, the 16 x 16 accumulator tile
+// of one layer is, packed to BF16, the A fragment of the next: E1's tile of
+// child j is k step j of E2, E2's tile is E3's operand, E3's tile of octant p is
+// k step p of E4, and likewise D1 .. D4.  Cells go from memory to E1's fragments
+// and from D4's accumulators to memory as float4s, each once; only the blocks'
+// largest |value|, E3's tiles and D1's latents pass through shared memory.
+// One warp per block with the layer outputs in shared memory, before, used 8 or
+// 1 of the 16 rows in five layers of eight and moved every value through shared
+// memory: encode + decode of 400 x 400 x 320 took 904 us, now 91 + 68 us.  The
+// MMAs with full rows take 27 us of tensor time and the volumes 67 us of memory
+// time; what bounds the kernels is issue slots at 16 warps an SM (half of them
+// used) and, decoding, the half-sector stores.
+// Each output element is the same mma.sync chain over k in steps of 16 as in
+// gemm_bf16_k, with the same operand roundings, bias and activation, so the
+// results equal the layer-by-layer path bit for bit.
+constexpr int kAeWarps = 8, kAeRows = 16;
 
-// Row strides (bf16 elements) of the operands in shared memory: K + 8 for a
-// layer's transposed weights and its input rows, so that the 32-bit loads of
-// a fragment's column pairs fall in distinct banks (a row of K + 8 bf16 moves
-// the bank by 4 words: the 8 row groups x 4 column pairs of a fragment cover
-// the 32 banks once).  Rows of E1's input (K = 8) stay unpadded (4 words).
-constexpr int kpad(int k) { return k == 8 ? 8 : k + 8; }
-
-// out(m, n, v) for m < M, n < N: v = act(bias[n] + sum_k A[m][k] W[k][n]),
-// A bf16 [M][LDA] and the weights transposed, Wt bf16 [N][kpad(K)], in shared
-// memory.  Each pair of adjacent columns is one 32-bit load.
-template <int M, int K, int N, int LDA, bool ACT, typename Out>
-__device__ __forceinline__ void warp_layer(const __nv_bfloat16 *A, const __nv_bfloat16 *Wt, const float *bias,
-                                           Out out) {
-  constexpr int LDW = kpad(K);
-  const int lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3;
-  auto a2 = [&](int m, int k) -> uint32_t {
-    return (m < M && k < K) ? *reinterpret_cast<const uint32_t *>(A + m * LDA + k) : 0u;
-  };
-  auto b2 = [&](int k, int n) -> uint32_t {
-    return k < K ? *reinterpret_cast<const uint32_t *>(Wt + n * LDW + k) : 0u;
-  };
-#pragma unroll 1
-  for (int m0 = 0; m0 < M; m0 += 16) {
-#pragma unroll 1
-    for (int n0 = 0; n0 < N; n0 += 8) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int k0 = 0; k0 < K; k0 += 16) {
-        const int r0 = m0 + gr, r1 = r0 + 8, c0 = k0 + 2 * t, c1 = c0 + 8, n = n0 + gr;
-        uint32_t a[4];
-        a[0] = a2(r0, c0);
-        a[1] = a2(r1, c0);
-        a[2] = a2(r0, c1);
-        a[3] = a2(r1, c1);
-        mma_bf16(acc, a, b2(c0, n), b2(c1, n));
-      }
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int m = m0 + gr + (q >= 2 ? 8 : 0), n = n0 + 2 * t + (q & 1);
-        if (m >= M) continue;
-        float v = acc[q] + bias[n];
-        if (ACT) v = v > 0.f ? v : kSlope * v;
-        out(m, n, v);
-      }
-    }
-  }
-}
-
-// transposed, padded weights of a layer and of four consecutive layers
-template <int L> constexpr int wt_size() { return kL_N[L] * kpad(kL_K[L]); }
-template <int L0> constexpr int half_wt() { return wt_size<L0>() + wt_size<L0 + 1>() + wt_size<L0 + 2>() + wt_size<L0 + 3>(); }
-constexpr int half_b(int l0) { return kL_N[l0] + kL_N[l0 + 1] + kL_N[l0 + 2] + kL_N[l0 + 3]; }
-
-// layer L's weights W[k][n] (FP32 master) into Wt[n][kpad(K)] as bf16, its biases as FP32
+// the B fragment of rows [16 ks, 16 ks + 16) and columns [8 nt, 8 nt + 8) of layer L's weights
+// (FP32 master, rounded to BF16); rows beyond K are zeros
 template <int L>
-__device__ __forceinline__ void stage_layer(const float *__restrict__ p, __nv_bfloat16 *wt, float *b) {
-  constexpr int K = kL_K[L], N = kL_N[L], wo = w_off(L);
-  for (int i = threadIdx.x; i < K * N; i += blockDim.x) {
-    const int k = i / N, n = i % N;
-    wt[n * kpad(K) + k] = __float2bfloat16_rn(p[wo + i]);
+__device__ __forceinline__ uint2 b_frag(const float *__restrict__ p, int ks, int nt, int lane) {
+  constexpr int K = kL_K[L], N = kL_N[L];
+  const float *w = p + w_off(L) + nt * 8 + (lane >> 2);
+  const int k = ks * 16 + 2 * (lane & 3);
+  uint2 b;
+  b.x = pack_bf16(w[k * N], w[(k + 1) * N]);
+  b.y = K > 8 ? pack_bf16(w[(k + 8) * N], w[(k + 9) * N]) : 0u;
+  return b;
+}
+// the biases of a lane's columns 2t, 2t + 1 of tile nt and of the tile after it
+template <int L>
+__device__ __forceinline__ float4 b_bias(const float *__restrict__ p, int nt, int lane) {
+  const float *b = p + w_off(L) + kL_K[L] * kL_N[L] + nt * 8 + 2 * (lane & 3);
+  return make_float4(b[0], b[1], b[8], b[9]);
+}
+// (x + bx, y + by) under the leaky ReLU (slope < 1: the larger of v and slope v) as two BF16; the
+// packed FP32 forms round as the scalar ones in half the issue slots
+__device__ __forceinline__ uint32_t act2(float x, float y, float bx, float by) {
+  float vx, vy, sx, sy;
+  asm("{\n .reg .b64 v, b, s;\n"
+      " mov.b64 v, {%4, %5};\n mov.b64 b, {%6, %7};\n mov.b64 s, {%8, %8};\n"
+      " add.rn.f32x2 v, v, b;\n mul.rn.f32x2 s, v, s;\n"
+      " mov.b64 {%0, %1}, v;\n mov.b64 {%2, %3}, s;\n}"
+      : "=f"(vx), "=f"(vy), "=f"(sx), "=f"(sy)
+      : "f"(x), "f"(y), "f"(bx), "f"(by), "f"(kSlope));
+  return pack_bf16(fmaxf(vx, sx), fmaxf(vy, sy));
+}
+// bias and activation of a 16 x 16 accumulator, as the next layer's A fragment
+__device__ __forceinline__ void next_a(uint32_t (&a)[4], const float (&d0)[4], const float (&d1)[4], const float4 &b) {
+  a[0] = act2(d0[0], d0[1], b.x, b.y);
+  a[1] = act2(d0[2], d0[3], b.x, b.y);
+  a[2] = act2(d1[0], d1[1], b.z, b.w);
+  a[3] = act2(d1[2], d1[3], b.z, b.w);
+}
+// The BF16 rounding of v / sc for four cells.  v * (1 / sc) lies within 2 units
+// of the last FP32 place of v / sc, so the two round to the same BF16 unless the
+// 16 bits that go are within 4 of half: then, or when 1 / sc may be subnormal
+// (`far`), the cells are divided.  32 divisions a lane were a third of the
+// encoder's instructions.
+__device__ __forceinline__ uint2 scale4(const float4 &v, float sc, float inv, bool far) {
+  float4 q = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
+  auto low = [](float f) { return (__float_as_uint(f) << 16) + 0x80040000u; };  // <= 8 << 16: near half
+  const unsigned m = min(min(low(q.x), low(q.y)), min(low(q.z), low(q.w)));
+  if (far || m <= 0x80000u) q = make_float4(v.x / sc, v.y / sc, v.z / sc, v.w / sc);
+  return make_uint2(pack_bf16(q.x, q.y), pack_bf16(q.z, q.w));
+}
+
+// A lane's cells of the blocks of one row: octant `oct`, cube cells of column
+// pair t; of child pair c (bits y1, x1) the 4 z cells from (x + 2 x1, y + 2 y1, z)
+// on.  Starts at block `blk` and moves on by `step` blocks.
+struct AeCells {
+  int bz, bx, by, nbz, nbx, nby, sz, sx, sy;
+  __device__ __forceinline__ AeCells(long long blk, long long step, int nbz_, int nbx_, int nby_)
+      : nbz(nbz_), nbx(nbx_), nby(nby_) {
+    const unsigned u = (unsigned)blk, q = u / nbz, v = (unsigned)step, w = v / nbz;
+    bz = (int)(u - q * nbz), bx = (int)(q % nbx), by = (int)(q / nbx);
+    sz = (int)(v - w * nbz), sx = (int)(w % nbx), sy = (int)(w / nbx);
   }
-  for (int i = threadIdx.x; i < N; i += blockDim.x) b[i] = p[wo + K * N + i];
-}
-template <int L0>
-__device__ __forceinline__ void stage_weights(const float *__restrict__ p, __nv_bfloat16 *w, float *b) {
-  constexpr int w1 = wt_size<L0>(), w2 = w1 + wt_size<L0 + 1>(), w3 = w2 + wt_size<L0 + 2>();
-  constexpr int b1 = kL_N[L0], b2 = b1 + kL_N[L0 + 1], b3 = b2 + kL_N[L0 + 2];
-  stage_layer<L0>(p, w, b);
-  stage_layer<L0 + 1>(p, w + w1, b + b1);
-  stage_layer<L0 + 2>(p, w + w2, b + b2);
-  stage_layer<L0 + 3>(p, w + w3, b + b3);
-}
-
-// input row strides: E2 reads E1's output as [8][128], E3 E2's as [8][16],
-// D2 D1's as [8][16], D3 D2's as [8][16], D4 D3's as [64][16]
-constexpr int kLdE2 = kpad(128), kLdE3 = kpad(16), kLdD2 = kpad(16), kLdD3 = kpad(16), kLdD4 = kpad(16);
-
-struct __align__(16) AeEncSmem {
-  __nv_bfloat16 w[half_wt<0>()];
-  float b[half_b(0)];
-  float raw[kFusedWarps][kBlock];           // the blocks' cells, Morton order
-  __nv_bfloat16 x[kFusedWarps][kBlock];     // E1 input [64][8]
-  __nv_bfloat16 h1[kFusedWarps][8 * kLdE2]; // E1 output = E2 input [8][128]
-  __nv_bfloat16 h2[kFusedWarps][8 * kLdE3]; // E2 output = E3 input [8][16]
-  __nv_bfloat16 h3[kFusedWarps][8 * 16];    // E3 output = E4 input [1][128]
+  __device__ __forceinline__ void next() {
+    bz += sz, bx += sx, by += sy;
+    if (bz >= nbz) bz -= nbz, bx++;
+    if (bx >= nbx) bx -= nbx, by++;
+  }
+};
+struct AeRow {
+  int x, y, z;
+  long long o;  // cell offset
+  bool ok;      // there is such a block
+  __device__ __forceinline__ AeRow(const AeCells &k, int nx, int nz, int oct, int t) {
+    x = k.bx * 8 + (oct >> 2) * 4 + (t >> 1);
+    y = k.by * 8 + ((oct >> 1) & 1) * 4 + (t & 1);
+    z = k.bz * 8 + (oct & 1) * 4;
+    ok = k.by < k.nby;
+    o = ((long long)y * nx + x) * nz + z;
+  }
+  __device__ __forceinline__ bool in(int c, int nx, int ny, int nz) const {
+    return ok && x + 2 * (c >> 1) < nx && y + 2 * (c & 1) < ny && z < nz;
+  }
+  __device__ __forceinline__ long long at(int c, int nx, int nz) const {
+    return o + (long long)((c & 1) * nx + (c >> 1)) * 2 * nz;
+  }
 };
 
-// Persistent: each CTA stages the weights once, then takes groups of 4
-// blocks consecutive in z (group g: z group g % nbzg, then x, then y; block
-// bz = 4 (g % nbzg) + warp) until none is left.
-__global__ void __launch_bounds__(32 * kFusedWarps) ae_encode_k(const float *__restrict__ p,
-                                                               const float *__restrict__ vol, int nx, int ny, int nz,
-                                                               __nv_bfloat16 *__restrict__ latent,
-                                                               float *__restrict__ scales) {
-  extern __shared__ __align__(16) unsigned char smem_ae[];
-  AeEncSmem &s = *reinterpret_cast<AeEncSmem *>(smem_ae);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nbz = (nz + 7) / 8, nbx = (nx + 7) / 8, nby = (ny + 7) / 8, nbzg = (nbz + kFusedWarps - 1) / kFusedWarps;
-  const long long ngroups = (long long)nbzg * nbx * nby;
-  stage_weights<0>(p, s.w, s.b);
-  for (long long grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
-  const int bx = (int)((grp / nbzg) % nbx), by = (int)(grp / ((long long)nbzg * nbx)), z0 = (int)(grp % nbzg) * 32;
-  // 32 z x 8 x x 8 y cells: thread -> (z quad, x, y) rows of 128 bytes
-  for (int i = threadIdx.x; i < 8 * 8 * 8; i += blockDim.x) {
-    const int zq = i & 7, xi = (i >> 3) & 7, yj = i >> 6;
-    const int x = bx * 8 + xi, y = by * 8 + yj;
+// VEC: the volume and the latents are 16-byte aligned and nz % 4 == 0; else cell by cell
+template <bool VEC>
+__device__ __forceinline__ float4 ae_load4(const float *__restrict__ vol, const AeRow &k, int c, int nx, int ny, int nz) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (!k.in(c, nx, ny, nz)) return v;
+  const float *s = vol + k.at(c, nx, nz);
+  if (VEC) return __ldg(reinterpret_cast<const float4 *>(s));
+  v.x = s[0];
+  if (k.z + 1 < nz) v.y = s[1];
+  if (k.z + 2 < nz) v.z = s[2];
+  if (k.z + 3 < nz) v.w = s[3];
+  return v;
+}
+
+// Persistent: the weights' fragments are made once, then groups of 16 blocks
+// are taken until none is left, the next group's cells loaded before the last
+// layer of the present one.
+template <bool VEC>
+__global__ void __launch_bounds__(32 * kAeWarps, 2) ae_encode_k(const float *__restrict__ p,
+                                                                const float *__restrict__ vol, int nx, int ny, int nz,
+                                                                __nv_bfloat16 *__restrict__ latent,
+                                                                float *__restrict__ scales) {
+  __shared__ uint4 w2[8][32];                // E2's fragments of k step j, both column tiles
+  __shared__ uint4 h3[kAeWarps][32];         // E3's tile of an octant: E4's A fragment
+  __shared__ float red[kAeWarps][kAeRows];   // largest |value| of a block's octants
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3;
+  const int nbz = (nz + 7) / 8, nbx = (nx + 7) / 8, nby = (ny + 7) / 8;
+  const long long nb = (long long)nbz * nbx * nby, ngroups = (nb + kAeRows - 1) / kAeRows;
+  {
+    const uint2 f0 = b_frag<1>(p, warp, 0, lane), f1 = b_frag<1>(p, warp, 1, lane);
+    w2[warp][lane] = make_uint4(f0.x, f0.y, f1.x, f1.y);
+  }
+  const uint32_t w10 = b_frag<0>(p, 0, 0, lane).x, w11 = b_frag<0>(p, 0, 1, lane).x;
+  const uint2 w30 = b_frag<2>(p, 0, 0, lane), w31 = b_frag<2>(p, 0, 1, lane);
+  uint2 w4[8];
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int zl = zq * 4 + c, z = z0 + zl;
-      const float v = (x < nx && y < ny && z < nz) ? vol[((long long)y * nx + x) * nz + z] : 0.f;
-      s.raw[zl >> 3][morton8(xi, yj, zl & 7)] = v;
+  for (int k = 0; k < 8; k++) w4[k] = b_frag<3>(p, k, warp, lane);
+  const float4 b1 = b_bias<0>(p, 0, lane), b2 = b_bias<1>(p, 0, lane), b3 = b_bias<2>(p, 0, lane);
+  const float *b4 = p + w_off(3) + kL_K[3] * kL_N[3] + warp * 8 + 2 * t;
+  const float b40 = b4[0], b41 = b4[1];
+  float4 v[2][4];
+  AeCells k0((long long)blockIdx.x * kAeRows + gr, (long long)gridDim.x * kAeRows, nbz, nbx, nby);
+  AeCells k1((long long)blockIdx.x * kAeRows + gr + 8, (long long)gridDim.x * kAeRows, nbz, nbx, nby);
+  auto load = [&]() {  // the cells of k0's and k1's blocks
+    const AeRow r0(k0, nx, nz, warp, t), r1(k1, nx, nz, warp, t);
+#pragma unroll
+    for (int c = 0; c < 4; c++) v[0][c] = ae_load4<VEC>(vol, r0, c, nx, ny, nz);
+#pragma unroll
+    for (int c = 0; c < 4; c++) v[1][c] = ae_load4<VEC>(vol, r1, c, nx, ny, nz);
+    k0.next(), k1.next();
+  };
+  load();
+  for (long long grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
+    float sc[2];
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      float a = 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+        a = fmaxf(fmaxf(fmaxf(a, fabsf(v[r][c].x)), fabsf(v[r][c].y)), fmaxf(fabsf(v[r][c].z), fabsf(v[r][c].w)));
+      a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 1));
+      a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, 2));
+      if (t == 0) red[warp][gr + 8 * r] = a;
     }
-  }
-  __syncthreads();
-  const int bz = (int)(grp % nbzg) * kFusedWarps + warp;
-  if (bz < nbz) {
-    float a = 0.f;
-    for (int i = lane; i < kBlock; i += 32) a = fmaxf(a, fabsf(s.raw[warp][i]));
-    for (int o = 16; o; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
-    const float sc = a;
-    for (int i = lane; i < kBlock; i += 32)
-      s.x[warp][i] = __float2bfloat16_rn(sc > 0.f ? s.raw[warp][i] / sc : 0.f);
-    __syncwarp();
-    const __nv_bfloat16 *w = s.w;
-    const float *b = s.b;
-    __nv_bfloat16 *h1 = s.h1[warp], *h2 = s.h2[warp], *h3 = s.h3[warp];
-    warp_layer<64, 8, 16, 8, true>(s.x[warp], w, b, [&](int m, int n, float v) {
-      h1[(m >> 3) * kLdE2 + (m & 7) * 16 + n] = __float2bfloat16_rn(v);
-    });
-    __syncwarp();
-    w += wt_size<0>(), b += 16;
-    warp_layer<8, 128, 16, kLdE2, true>(h1, w, b, [&](int m, int n, float v) {
-      h2[m * kLdE3 + n] = __float2bfloat16_rn(v);
-    });
-    __syncwarp();
-    w += wt_size<1>(), b += 16;
-    warp_layer<8, 16, 16, kLdE3, true>(h2, w, b, [&](int m, int n, float v) { h3[m * 16 + n] = __float2bfloat16_rn(v); });
-    __syncwarp();
-    w += wt_size<2>(), b += 16;
-    const long long blk = ((long long)by * nbx + bx) * nbz + bz;
-    __nv_bfloat16 *lat = latent + blk * kLatent;
-    warp_layer<1, 128, kLatent, 128, false>(h3, w, b, [&](int, int n, float v) { lat[n] = __float2bfloat16_rn(v); });
-    if (lane == 0) scales[blk] = sc;
-  }
-  __syncthreads();  // the next group overwrites raw
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      sc[r] = red[0][gr + 8 * r];
+#pragma unroll
+      for (int w = 1; w < kAeWarps; w++) sc[r] = fmaxf(sc[r], red[w][gr + 8 * r]);
+    }
+    uint2 x[2][4];  // E1's operands: [row][child pair] of z1 = 0, 1
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const float inv = 1.f / sc[r];
+      const bool far = !(sc[r] > 1e-30f && sc[r] < 1e30f);
+#pragma unroll
+      for (int c = 0; c < 4; c++) x[r][c] = sc[r] > 0.f ? scale4(v[r][c], sc[r], inv, far) : make_uint2(0u, 0u);
+    }
+    float e0[4] = {0.f, 0.f, 0.f, 0.f}, e1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const uint32_t a[4] = {j & 1 ? x[0][j >> 1].y : x[0][j >> 1].x, j & 1 ? x[1][j >> 1].y : x[1][j >> 1].x, 0u, 0u};
+      float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+      mma_bf16(d0, a, w10, 0u);
+      mma_bf16(d1, a, w11, 0u);
+      uint32_t h[4];
+      next_a(h, d0, d1, b1);
+      const uint4 w = w2[j][lane];
+      mma_bf16(e0, h, w.x, w.y);
+      mma_bf16(e1, h, w.z, w.w);
+    }
+    {
+      uint32_t h[4];
+      next_a(h, e0, e1, b2);
+      float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+      mma_bf16(d0, h, w30.x, w30.y);
+      mma_bf16(d1, h, w31.x, w31.y);
+      next_a(h, d0, d1, b3);
+      h3[warp][lane] = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+    if (grp + gridDim.x < ngroups) load();
+    __syncthreads();
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const uint4 h = h3[k][lane];
+      const uint32_t a[4] = {h.x, h.y, h.z, h.w};
+      mma_bf16(d, a, w4[k].x, w4[k].y);
+    }
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const long long blk = grp * kAeRows + gr + 8 * r;
+      if (blk >= nb) continue;
+      __nv_bfloat16 *l = latent + blk * kLatent + warp * 8 + 2 * t;
+      const float l0 = d[2 * r] + b40, l1 = d[2 * r + 1] + b41;
+      if (VEC) {
+        *reinterpret_cast<uint32_t *>(l) = pack_bf16(l0, l1);
+      } else {
+        l[0] = __float2bfloat16_rn(l0), l[1] = __float2bfloat16_rn(l1);
+      }
+      if (warp == 0 && t == 0) scales[blk] = sc[r];
+    }
   }
 }
 
-struct __align__(16) AeDecSmem {
-  __nv_bfloat16 w[half_wt<4>()];
-  float b[half_b(4)];
-  __nv_bfloat16 l[kFusedWarps][kLatent];     // D1 input [1][kLatent]
-  __nv_bfloat16 g1[kFusedWarps][8 * kLdD2];  // D1 output = D2 input [8][16]
-  __nv_bfloat16 g2[kFusedWarps][8 * kLdD3];  // D2 output = D3 input [8][16]
-  __nv_bfloat16 g3[kFusedWarps][64 * kLdD4]; // D3 output = D4 input [64][16]
-  float out[kFusedWarps][kBlock];            // D4 output x scale, Morton order
-};
+constexpr int kLdLat = kLatent + 8;  // row stride of the staged latents: a fragment's loads hit distinct banks
 
-__global__ void __launch_bounds__(32 * kFusedWarps) ae_decode_k(const float *__restrict__ p,
-                                                               const __nv_bfloat16 *__restrict__ latent,
-                                                               const float *__restrict__ scales, int nx, int ny, int nz,
-                                                               float *__restrict__ vol) {
-  extern __shared__ __align__(16) unsigned char smem_ae[];
-  AeDecSmem &s = *reinterpret_cast<AeDecSmem *>(smem_ae);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nbz = (nz + 7) / 8, nbx = (nx + 7) / 8, nby = (ny + 7) / 8, nbzg = (nbz + kFusedWarps - 1) / kFusedWarps;
-  const long long ngroups = (long long)nbzg * nbx * nby;
-  stage_weights<4>(p, s.w, s.b);
-  __syncthreads();
-  for (long long grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
-  const int bx = (int)((grp / nbzg) % nbx), by = (int)(grp / ((long long)nbzg * nbx)), z0 = (int)(grp % nbzg) * 32;
-  const int bz = (int)(grp % nbzg) * kFusedWarps + warp;
-  if (bz < nbz) {
-    const long long blk = ((long long)by * nbx + bx) * nbz + bz;
-    for (int k = lane; k < kLatent; k += 32) s.l[warp][k] = latent[blk * kLatent + k];
-    const float sc = scales[blk];
-    __syncwarp();
-    const __nv_bfloat16 *w = s.w;
-    const float *b = s.b;
-    __nv_bfloat16 *g1 = s.g1[warp], *g2 = s.g2[warp], *g3 = s.g3[warp];
-    float *o = s.out[warp];
-    warp_layer<1, kLatent, 128, kLatent, true>(s.l[warp], w, b, [&](int, int n, float v) {
-      g1[(n >> 4) * kLdD2 + (n & 15)] = __float2bfloat16_rn(v);
-    });
-    __syncwarp();
-    w += wt_size<4>(), b += 128;
-    warp_layer<8, 16, 16, kLdD2, true>(g1, w, b, [&](int m, int n, float v) {
-      g2[m * kLdD3 + n] = __float2bfloat16_rn(v);
-    });
-    __syncwarp();
-    w += wt_size<5>(), b += 16;
-    warp_layer<8, 16, 128, kLdD3, true>(g2, w, b, [&](int m, int n, float v) {
-      g3[(m * 8 + (n >> 4)) * kLdD4 + (n & 15)] = __float2bfloat16_rn(v);
-    });
-    __syncwarp();
-    w += wt_size<6>(), b += 128;
-    warp_layer<64, 16, 8, kLdD4, false>(g3, w, b, [&](int m, int n, float v) { o[m * 8 + n] = sc * v; });
+template <bool VEC>
+__global__ void __launch_bounds__(32 * kAeWarps, 2) ae_decode_k(const float *__restrict__ p,
+                                                                const __nv_bfloat16 *__restrict__ latent,
+                                                                const float *__restrict__ scales, int nx, int ny, int nz,
+                                                                float *__restrict__ vol) {
+  __shared__ uint4 w3[8][32];                                       // D3's fragments of child j, both column tiles
+  __shared__ float4 b3[8][4];                                       // D3's biases of child j by lane & 3
+  __shared__ __align__(16) __nv_bfloat16 lat[2][kAeRows][kLdLat];   // D1's input, by parity of the group
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3;
+  const int nbz = (nz + 7) / 8, nbx = (nx + 7) / 8, nby = (ny + 7) / 8;
+  const long long nb = (long long)nbz * nbx * nby, ngroups = (nb + kAeRows - 1) / kAeRows;
+  {
+    const uint2 f0 = b_frag<6>(p, 0, 2 * warp, lane), f1 = b_frag<6>(p, 0, 2 * warp + 1, lane);
+    w3[warp][lane] = make_uint4(f0.x, f0.y, f1.x, f1.y);
+    if (gr == 0) b3[warp][t] = b_bias<6>(p, 2 * warp, lane);
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 8 * 8 * 8; i += blockDim.x) {
-    const int zq = i & 7, xi = (i >> 3) & 7, yj = i >> 6;
-    const int x = bx * 8 + xi, y = by * 8 + yj;
-    if (x >= nx || y >= ny) continue;
+  uint2 w1[4][2];
+#pragma unroll
+  for (int k = 0; k < 4; k++) w1[k][0] = b_frag<4>(p, k, 2 * warp, lane), w1[k][1] = b_frag<4>(p, k, 2 * warp + 1, lane);
+  const uint2 w20 = b_frag<5>(p, 0, 0, lane), w21 = b_frag<5>(p, 0, 1, lane), w4 = b_frag<7>(p, 0, 0, lane);
+  const float4 b1 = b_bias<4>(p, 2 * warp, lane), b2 = b_bias<5>(p, 0, lane);
+  const float *b4 = p + w_off(7) + kL_K[7] * kL_N[7] + 2 * t;
+  const float b40 = b4[0], b41 = b4[1];
+  // a group's latents: 16 x 128 bytes, 16 to each of the first 128 threads
+  const int lrow = threadIdx.x >> 3, lcol = (threadIdx.x & 7) * 8;
+  uint4 ln = make_uint4(0u, 0u, 0u, 0u);
+  auto fetch = [&](long long grp) {
+    const long long blk = grp * kAeRows + lrow;
+    ln = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x >= 8 * kAeRows || blk >= nb) return;
+    const __nv_bfloat16 *l = latent + blk * kLatent + lcol;
+    if (VEC) {
+      ln = __ldg(reinterpret_cast<const uint4 *>(l));
+    } else {
+      const unsigned short *u = reinterpret_cast<const unsigned short *>(l);
+      ln = make_uint4(u[0] | (unsigned)u[1] << 16, u[2] | (unsigned)u[3] << 16, u[4] | (unsigned)u[5] << 16,
+                      u[6] | (unsigned)u[7] << 16);
+    }
+  };
+  fetch(blockIdx.x);
+  AeCells k0((long long)blockIdx.x * kAeRows + gr, (long long)gridDim.x * kAeRows, nbz, nbx, nby);
+  AeCells k1((long long)blockIdx.x * kAeRows + gr + 8, (long long)gridDim.x * kAeRows, nbz, nbx, nby);
+  int par = 0;
+  for (long long grp = blockIdx.x; grp < ngroups; grp += gridDim.x, par ^= 1) {
+    if (threadIdx.x < 8 * kAeRows) *reinterpret_cast<uint4 *>(&lat[par][lrow][lcol]) = ln;
+    if (grp + gridDim.x < ngroups) fetch(grp + gridDim.x);
+    float sc[2];
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const long long blk = grp * kAeRows + gr + 8 * r;
+      sc[r] = blk < nb ? scales[blk] : 0.f;
+    }
+    __syncthreads();
+    float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const __nv_bfloat16 *l = &lat[par][gr][16 * k + 2 * t];
+      const uint32_t a[4] = {
+          *reinterpret_cast<const uint32_t *>(l), *reinterpret_cast<const uint32_t *>(l + 8 * kLdLat),
+          *reinterpret_cast<const uint32_t *>(l + 8), *reinterpret_cast<const uint32_t *>(l + 8 * kLdLat + 8)};
+      mma_bf16(d0, a, w1[k][0].x, w1[k][0].y);
+      mma_bf16(d1, a, w1[k][1].x, w1[k][1].y);
+    }
+    uint32_t h[4];
+    next_a(h, d0, d1, b1);
+#pragma unroll
+    for (int i = 0; i < 4; i++) d0[i] = d1[i] = 0.f;
+    mma_bf16(d0, h, w20.x, w20.y);
+    mma_bf16(d1, h, w21.x, w21.y);
+    next_a(h, d0, d1, b2);
+    const AeRow r0(k0, nx, nz, warp, t), r1(k1, nx, nz, warp, t);
+    k0.next(), k1.next();
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-      const int zl = zq * 4 + c, z = z0 + zl;
-      if (z < nz) vol[((long long)y * nx + x) * nz + z] = s.out[zl >> 3][morton8(xi, yj, zl & 7)];
+      float o[2][4];  // [row][z]
+#pragma unroll
+      for (int z1 = 0; z1 < 2; z1++) {
+        const int j = 2 * c + z1;
+        const uint4 w = w3[j][lane];
+        float f0[4] = {0.f, 0.f, 0.f, 0.f}, f1[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16(f0, h, w.x, w.y);
+        mma_bf16(f1, h, w.z, w.w);
+        uint32_t a[4];
+        next_a(a, f0, f1, b3[j][t]);
+        mma_bf16(e, a, w4.x, w4.y);
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          o[r][2 * z1] = sc[r] * (e[2 * r] + b40);
+          o[r][2 * z1 + 1] = sc[r] * (e[2 * r + 1] + b41);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const AeRow &k = r ? r1 : r0;
+        if (!k.in(c, nx, ny, nz)) continue;
+        float *q = vol + k.at(c, nx, nz);
+        if (VEC) {
+          *reinterpret_cast<float4 *>(q) = make_float4(o[r][0], o[r][1], o[r][2], o[r][3]);
+        } else {
+#pragma unroll
+          for (int z = 0; z < 4; z++)
+            if (k.z + z < nz) q[z] = o[r][z];
+        }
+      }
     }
-  }
-  __syncthreads();  // the next group overwrites out
   }
 }
 
@@ -519,50 +628,41 @@ long long ae_volume_blocks(int nx, int ny, int nz) {
 
 int ae_prepare(rtm_ae *a) { return ae_reserve(a, kChunkBlocks, false); }
 
-// CTAs of one wave of the persistent codec kernels (set by ae_fused_init)
-static int g_ae_wave = 0;
-
-// shared-memory size of the fused encoder / decoder (beyond the 48 KB default)
-// and the CTAs of one wave; called when a compressor is created (outside any
-// stream capture)
-static bool ae_fused_init() {
-  if (cudaFuncSetAttribute(ae_encode_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AeEncSmem)) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(ae_decode_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AeDecSmem)) !=
-          cudaSuccess)
-    return false;
-  int dev = 0, sms = 0, occ_e = 0, occ_d = 0;
+// CTAs of one wave of a persistent codec kernel on the current device
+template <typename K>
+static int ae_wave(K kernel) {
+  int dev = 0, sms = 0, occ = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_e, ae_encode_k, 32 * kFusedWarps, sizeof(AeEncSmem));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_d, ae_decode_k, 32 * kFusedWarps, sizeof(AeDecSmem));
-  g_ae_wave = std::max(1, sms) * std::max(1, std::min(occ_e, occ_d));
-  return true;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 32 * kAeWarps, 0);
+  return std::max(1, sms) * std::max(1, occ);
+}
+static void ae_waves(rtm_ae *a) {
+  a->wave_enc[0] = ae_wave(ae_encode_k<false>), a->wave_enc[1] = ae_wave(ae_encode_k<true>);
+  a->wave_dec[0] = ae_wave(ae_decode_k<false>), a->wave_dec[1] = ae_wave(ae_decode_k<true>);
+}
+static unsigned ae_grid(int wave, int nx, int ny, int nz) {
+  return (unsigned)std::min<long long>((ae_volume_blocks(nx, ny, nz) + kAeRows - 1) / kAeRows, wave);
+}
+static bool ae_aligned(const void *vol, const void *latent, int nz) {
+  return nz % 4 == 0 && ((reinterpret_cast<uintptr_t>(vol) | reinterpret_cast<uintptr_t>(latent)) & 15) == 0;
 }
 
 // volume -> latents [nb][64] (bfloat16) + scales [nb] (device), on stream st
-// (the fused kernel)
-// CTAs of a persistent codec launch over `groups` work items: one wave
-static unsigned ae_grid(long long groups) {
-  return (unsigned)std::max(1LL, std::min<long long>(groups, std::max(1, g_ae_wave)));
-}
-static long long ae_groups(int nx, int ny, int nz) {
-  return (long long)((((nz + 7) / 8) + kFusedWarps - 1) / kFusedWarps) * ((nx + 7) / 8) * ((ny + 7) / 8);
-}
-
 int ae_compress(rtm_ae *a, const float *w, int nx, int ny, int nz, void *latent, float *scales, cudaStream_t st) {
-  ae_encode_k<<<ae_grid(ae_groups(nx, ny, nz)), 32 * kFusedWarps, sizeof(AeEncSmem), st>>>(
-      a->p, w, nx, ny, nz, static_cast<__nv_bfloat16 *>(latent), scales);
+  const bool vec = ae_aligned(w, latent, nz);
+  auto *k = vec ? ae_encode_k<true> : ae_encode_k<false>;
+  k<<<ae_grid(a->wave_enc[vec], nx, ny, nz), 32 * kAeWarps, 0, st>>>(a->p, w, nx, ny, nz, static_cast<__nv_bfloat16 *>(latent), scales);
   return cudaGetLastError() == cudaSuccess ? RTM_OK : RTM_ERR_CUDA;
 }
-// latents + scales -> volume (device), on stream st (the fused kernel)
+// latents + scales -> volume (device), on stream st
 int ae_decompress(rtm_ae *a, const void *latent, const float *scales, int nx, int ny, int nz, float *w,
                   cudaStream_t st) {
-  ae_decode_k<<<ae_grid(ae_groups(nx, ny, nz)), 32 * kFusedWarps, sizeof(AeDecSmem), st>>>(
-      a->p, static_cast<const __nv_bfloat16 *>(latent), scales, nx, ny, nz, w);
+  const bool vec = ae_aligned(w, latent, nz);
+  auto *k = vec ? ae_decode_k<true> : ae_decode_k<false>;
+  k<<<ae_grid(a->wave_dec[vec], nx, ny, nz), 32 * kAeWarps, 0, st>>>(a->p, static_cast<const __nv_bfloat16 *>(latent), scales, nx, ny, nz, w);
   return cudaGetLastError() == cudaSuccess ? RTM_OK : RTM_ERR_CUDA;
 }
-
 
 // ---- FP16 fallback of the high-energy blocks of a learned snapshot ----------
 // Per slot: a header, the indices of the stored blocks, and each stored block
@@ -745,11 +845,7 @@ int rtm_ae_create(rtm_ae **out) {
     rtm_ae_destroy(a);
     return RTM_ERR_NOMEM;
   }
-  if (!rtm::ae_fused_init()) {
-    cudaGetLastError();
-    rtm_ae_destroy(a);
-    return RTM_ERR_CUDA;
-  }
+  rtm::ae_waves(a);
   *out = a;
   return RTM_OK;
 }
