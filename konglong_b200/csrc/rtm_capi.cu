@@ -313,6 +313,28 @@ static int yseg_v4(Engine *h, int tx, int ctas_per_sm) {
   }
   return best_y;
 }
+// The y segment of the TMA-ring kernels, whose PML and interior tiles run side by
+// side (LaunchPair): places taken as they fall free, so a step lasts for the tiles'
+// work over the places, and half a tile more for the ragged end; a tile's set-up
+// (8 planes of the y queue, the first copies) counts as two planes.  Whole waves of
+// equal tiles, which the one-launch kernels above are modelled by, chose segments
+// of 41, 52 and 134 planes at 330 x 283 x 260, 256^3 TTI and 512 x 400 x 200 VTI: 494,
+// 360 and 961 us a step against 455, 306 and 756 with 12 planes; at 512 x 512 x 400
+// ISO 74 planes take 499 us, 40 take 494 and 12 take 535.
+static int yseg_pair(Engine *h, int tx, int ctas_per_sm) {
+  const int nx = h->d.nx, ny = h->d.ny, nz = h->d.nz;
+  const double bxz = (double)((nz + 31) / 32) * ((nx + tx - 1) / tx);
+  const double res = (double)std::max(1, h->sms) * std::max(1, ctas_per_sm);
+  int best_y = ny;
+  double best = 1e300;
+  for (int nseg = 1; nseg <= std::max(1, ny / 8); nseg++) {
+    const int yseg = (ny + nseg - 1) / nseg;
+    const double cost = (yseg + 2) * (bxz * ((ny + yseg - 1) / yseg) / res + 0.5);
+    if (cost < best) best = cost, best_y = yseg;
+  }
+  return best_y;
+}
+
 // Tile table for tile width tx and y segment yseg: columns touching an x or
 // z PML face are PML tiles over all y; the others are PML tiles over the y
 // faces and interior tiles between.  Built on the host and uploaded (never
@@ -391,11 +413,11 @@ static void launch_pair(Engine *h, const TileSet &t, LaunchPair &edge, LaunchPai
   edge.number = inner.number = h->pair_no;
 }
 
-static int yseg_an4(Engine *h) { return yseg_v4(h, kAniso4TX, aniso4_ctas_per_sm()); }
+static int yseg_an4(Engine *h) { return yseg_pair(h, kAniso4TX, aniso4_ctas_per_sm()); }
 
 static int yseg_iso4(Engine *h) {
   if (h->iso4 == 2)
-    return yseg_v4(h, kIso4TmaShapes[h->v4_shape].tx, iso_tma4_ctas_per_sm(h->v4_shape, h->c.pml3d));
+    return yseg_pair(h, kIso4TmaShapes[h->v4_shape].tx, iso_tma4_ctas_per_sm(h->v4_shape, h->c.pml3d));
   return yseg_v4(h, h->v4_tx, iso_v4_ctas_per_sm(h->v4_tx, h->c.pml3d));
 }
 
