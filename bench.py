@@ -314,7 +314,7 @@ def run_cuda(args, rank, world):
         q.set_extraction(rcv, K)
         q.reset()
         q.set_injection(src, shot.wavelet[None, :K + 1].copy(), s.dt_dxyz)
-        q.modelling(2, -1, 1)  # warm the graph path
+        q.modelling(2, -1, 1)  # warm-up
         q.reset()
         wav = np.ascontiguousarray(shot.wavelet[None, :K + 1])
         R.barrier(ranks)
@@ -537,7 +537,7 @@ def run_rtm_shot(args, ranks):
         p.snapshot_setup(fmt, min(plan["seg_slots"], (Wm + K) // interval + 2))
         p.reset()
         p.set_injection(src, shot.wavelet[None, :], s.dt_dxyz)
-        p.migration(FORWARD, 0, Wm, -1, interval)          # warm-up (graph capture, first launches)
+        p.migration(FORWARD, 0, Wm, -1, interval)          # warm-up (first launches)
         with ClockSampler(ranks.local_rank) as clk:
             p.migration(FORWARD, Wm, Wm + K, -1, interval)
             fwd = p.last_loop_ms

@@ -120,9 +120,8 @@ typedef struct rtm_config {
                          drivers only (the stepwise seam calls return RTM_ERR_UNSUPPORTED) */
   int kernel_variant; /* 0: auto (FD8: 4 z cells per thread with TMA rings when nz % 4 == 0 and,
                          for VTI / TTI, the state is FP32; the autotuner picks among all FD8
-                         kernels; compact FD: line solves and pointwise epilogues with TMA x / y
-                         tiles when nz % 4 == 0, else register-streamed x / y lines; the
-                         autotuner may pick any compact-FD form; FFTWR2R / SINCOS / FFTWR2C /
+                         kernels; compact FD: line solves on shared-memory tiles (x / y by TMA when
+                         nz % 4 == 0) and pointwise epilogues; the autotuner may pick any compact-FD form; FFTWR2R / SINCOS / FFTWR2C /
                          FFTV: line operators on the tensor cores, split TF32, where nz % 4 == 0
                          and lines have at most 512 points), 1: one cell per thread / plain
                          staged tiles (FFTWR2R / SINCOS: FP32 cuBLAS line products; FFTWR2C /
