@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? kEdgeCtas : 0)
 #pragma unroll
   for (int k = 0; k < 2 * R4; k++) {
     const int y = y0 - R4 + k;
-    q[k] = act && y >= 0 && y < ny ? __ldg(w1g + y * nxz4 + col4) : zero4;
+    q[k] = act && y >= 0 && y < ny ? __ldcg(w1g + y * nxz4 + col4) : zero4;
   }
   TilePml<0, TX, EDGE == TILE_PML3> pm;
   if constexpr (EDGE != 0) {
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? kEdgeCtas : 0)
 #pragma unroll
   for (int k = 0; k < 2 * R4; k++) {
     const int y = y0 - R4 + k;
-    q[k] = do_y && act && y >= 0 && y < ny ? __ldg(pyg + y * nxz4 + col4) : zero4;
+    q[k] = do_y && act && y >= 0 && y < ny ? __ldcg(pyg + y * nxz4 + col4) : zero4;
   }
   TilePml<1, TX, EDGE == TILE_PML3> pm;
   if constexpr (EDGE != 0) {

@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
 #pragma unroll
   for (int k = 0; k < 2 * R4; k++) {
     const int y = y0 - R4 + k;
-    q[k] = act && y >= 0 && y < ny ? __ldg(w1g + y * nxz4 + col4) : zero4;
+    q[k] = act && y >= 0 && y < ny ? __ldcg(w1g + y * nxz4 + col4) : zero4;
   }
   // the round-1 memory of a face is one round stride (its component stride) on
   TileFaces<0> pm;

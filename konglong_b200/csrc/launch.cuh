@@ -27,7 +27,9 @@ __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;"
 // each pair), and a second launch that does not find its number waits as usual.  The
 // second launch calls dep_wait() as its last act instead of its first: its end
 // then implies the end of the first, and the kernel after it need wait for
-// nothing more.  No launch waits for one behind it: the second is let in when
+// nothing more.  A second launch reads what the step writes through L2 (TMA, .cg)
+// or by ordinary loads after its acquire, never through the read-only path, which
+// an acquire does not cover.  No launch waits for one behind it: the second is let in when
 // every CTA of the first has its place.
 enum { PAIR_NONE = 0, PAIR_FIRST = 1, PAIR_SECOND = 2 };
 struct LaunchPair {
