@@ -142,13 +142,13 @@ __global__ void __launch_bounds__(8 * TX, EDGE ? kEdgeCtas : 0)
     for (int p = y0; p < min(y0 + R4 + P, y1 + R4); p++) issue_a(p), last_a = p;
     for (int p = y0; p < min(y0 + P, y1); p++) issue_b(p), last_b = p;
   }
-  const float4 *__restrict__ w1g = reinterpret_cast<const float4 *>(a.w1);
+  const float4 *w1g = reinterpret_cast<const float4 *>(a.w1);
   const long long nxz4 = g.nxz / 4, col4 = col / 4;
   float4 q[2 * R4 + 1];
 #pragma unroll
   for (int k = 0; k < 2 * R4; k++) {
     const int y = y0 - R4 + k;
-    q[k] = act && y >= 0 && y < ny ? __ldcg(w1g + y * nxz4 + col4) : zero4;
+    q[k] = act && y >= 0 && y < ny ? ld_l2(w1g + y * nxz4 + col4) : zero4;
   }
   TilePml<0, TX, EDGE == TILE_PML3> pm;
   if constexpr (EDGE != 0) {
@@ -316,13 +316,13 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? kEdgeCtas : 0)
     for (int p = y0 + R4; p < min(y0 + R4 + P, y1 + R4); p++) issue_a(p), last_a = p;
     for (int p = y0; p < min(y0 + P, y1); p++) issue_b(p), last_b = p;
   }
-  const float4 *__restrict__ pyg = reinterpret_cast<const float4 *>(a.py);
+  const float4 *pyg = reinterpret_cast<const float4 *>(a.py);
   const long long nxz4 = g.nxz / 4, col4 = col / 4;
   float4 q[2 * R4 + 1];
 #pragma unroll
   for (int k = 0; k < 2 * R4; k++) {
     const int y = y0 - R4 + k;
-    q[k] = do_y && act && y >= 0 && y < ny ? __ldcg(pyg + y * nxz4 + col4) : zero4;
+    q[k] = do_y && act && y >= 0 && y < ny ? ld_l2(pyg + y * nxz4 + col4) : zero4;
   }
   TilePml<1, TX, EDGE == TILE_PML3> pm;
   if constexpr (EDGE != 0) {

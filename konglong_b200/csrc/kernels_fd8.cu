@@ -29,9 +29,8 @@ namespace {
 constexpr int TZ = 32;
 constexpr int R = 4;  // stencil radius (order 8)
 
-__device__ __forceinline__ float ld_or0(const float *__restrict__ p, long long i, bool ok) {
-  return ok ? __ldg(p + i) : 0.0f;
-}
+// what a step writes is read by ordinary loads (launch.cuh)
+__device__ __forceinline__ float ld_or0(const float *p, long long i, bool ok) { return ok ? p[i] : 0.0f; }
 
 // Halo values a thread stages into the plane tile: two z-halo cells (threads
 // tz < R) and two x-halo cells (threads tx < R).  Fetched two planes ahead so
@@ -41,7 +40,7 @@ struct Halo {
 };
 
 template <int TX>
-__device__ __forceinline__ Halo fetch_halo(const float *__restrict__ f, int iy, int ny, int ix, int iz, int nx, int nz,
+__device__ __forceinline__ Halo fetch_halo(const float *f, int iy, int ny, int ix, int iz, int nx, int nz,
                                            long long nxz, int tx, int tz) {
   Halo h{0.f, 0.f, 0.f, 0.f};
   if (iy < 0 || iy >= ny) return h;
@@ -81,7 +80,7 @@ __device__ __forceinline__ Halo fetch_halo_v(V v, int iy, int ny, int ix, int iz
 
 // FP16 state value: half * per-slab scale
 __device__ __forceinline__ float f16v(const __half *h, const float *s, long long i, int iy) {
-  return __half2float(h[i]) * __ldg(s + iy);
+  return __half2float(h[i]) * s[iy];
 }
 
 template <int TX>
@@ -96,8 +95,8 @@ __device__ __forceinline__ void put_tile(float (*tile)[TZ + 2 * R], const Halo &
 // step.
 // The coefficients and the PML widths are read once into registers.
 template <int TX, int MODE, bool PML3D>
-__device__ __forceinline__ void iso_tile(const IsoArgs &a, const float *__restrict__ w1, float *__restrict__ w0, int bx,
-                                         int by, int bz, float (*tile)[TZ + 2 * R]) {
+__device__ __forceinline__ void iso_tile(const IsoArgs &a, const float *w1, float *w0, int bx, int by,
+                                         int bz, float (*tile)[TZ + 2 * R]) {
   const int nx = a.nx, ny = a.ny, nz = a.nz, yseg = a.yseg;
   const Grid3 g{nx, ny, nz, (long long)nx * nz};
   float c2x[R + 1], c2y[R + 1], c2z[R + 1];
@@ -198,8 +197,8 @@ __global__ void __launch_bounds__(TZ *TX) iso_fd8_step(IsoArgs a) {
 // The gradient pass of one column tile (z tile bz, x tile bx, planes [y0, y1))
 // reading the field w1; every thread of the CTA calls it.
 template <int TX, int MODEL, bool F16, bool EDGE>
-__device__ __forceinline__ void grad_tile(const GradArgs &a, const float *__restrict__ w1, int bz, int bx, int y0,
-                                          int y1, float (&tile)[TX + 2 * R][TZ + 2 * R]) {
+__device__ __forceinline__ void grad_tile(const GradArgs &a, const float *w1, int bz, int bx, int y0, int y1,
+                                          float (&tile)[TX + 2 * R][TZ + 2 * R]) {
   const Grid3 g{a.nx, a.ny, a.nz, (long long)a.nx * a.nz};
   const int tz = threadIdx.x, tx = threadIdx.y;
   const int iz = bz * TZ + tz;
@@ -207,7 +206,7 @@ __device__ __forceinline__ void grad_tile(const GradArgs &a, const float *__rest
   const bool act = iz < a.nz && ix < a.nx;
   const long long col = (long long)ix * a.nz + iz;
   const bool do_y = a.ny > 1;
-  auto v1 = [&](long long i, int iy) -> float { return F16 ? f16v(a.h.w1, a.h.s1, i, iy) : __ldg(w1 + i); };
+  auto v1 = [&](long long i, int iy) -> float { return F16 ? f16v(a.h.w1, a.h.s1, i, iy) : w1[i]; };
 
   float q[2 * R + 1];
 #pragma unroll
@@ -295,8 +294,8 @@ __device__ __forceinline__ DivPlane fetch_div(const DivArgs &a, int iy, int ix, 
 // The divergence pass of one column tile reading w1 and the previous field w0,
 // which it overwrites with the new one; every thread of the CTA calls it.
 template <int TX, int MODE, bool F16, bool EDGE>
-__device__ __forceinline__ void div_tile(const DivArgs &a, const float *__restrict__ w1, float *w0, int bz, int bx,
-                                         int y0, int y1, float (&tpx)[TX + 2 * R][TZ], float (&tpz)[TX][TZ + 2 * R]) {
+__device__ __forceinline__ void div_tile(const DivArgs &a, const float *w1, float *w0, int bz, int bx, int y0, int y1,
+                                         float (&tpx)[TX + 2 * R][TZ], float (&tpz)[TX][TZ + 2 * R]) {
   const Grid3 g{a.nx, a.ny, a.nz, (long long)a.nx * a.nz};
   const int tz = threadIdx.x, tx = threadIdx.y;
   const int iz = bz * TZ + tz;
@@ -314,7 +313,7 @@ __device__ __forceinline__ void div_tile(const DivArgs &a, const float *__restri
   DivPlane d0 = fetch_div<TX>(a, y0, ix, iz, g.nxz, tx, tz, act);
   DivPlane d1 = fetch_div<TX>(a, y0 + 1 < y1 ? y0 + 1 : a.ny, ix, iz, g.nxz, tx, tz, act);
   auto v0 = [&](long long i, int iy) -> float { return F16 ? f16v(a.h.w0, a.h.s0, i, iy) : w0[i]; };
-  auto v1 = [&](long long i, int iy) -> float { return F16 ? f16v(a.h.w1, a.h.s1, i, iy) : __ldg(w1 + i); };
+  auto v1 = [&](long long i, int iy) -> float { return F16 ? f16v(a.h.w1, a.h.s1, i, iy) : w1[i]; };
   float nw0 = act ? v0((long long)y0 * g.nxz + col, y0) : 0.f;
   float nvel = act ? __ldg(a.vel + (long long)y0 * g.nxz + col) : 0.f;
   float nw1 = act && MODE != 0 ? v1((long long)y0 * g.nxz + col, y0) : 0.f;
@@ -351,7 +350,7 @@ __device__ __forceinline__ void div_tile(const DivArgs &a, const float *__restri
       if (MODE == 0) out = t;
       else out = MODE == 1 ? __fsub_rn(__fadd_rn(cw1, cw1), t) : q_update(a.q, i, (long long)a.ny * g.nxz, t, cw1);
       if (F16) {
-        const float sc = __ldg(a.h.sn + iy);
+        const float sc = a.h.sn[iy];
         float hv = out / sc;
         if (fabsf(hv) > 65504.f) hv = copysignf(65504.f, hv);  // saturate; a NaN stays a NaN
         a.h.w0[i] = __float2half_rn(hv);

@@ -28,8 +28,7 @@ __global__ void update2nd_q_k(float *__restrict__ w0, const float *__restrict__ 
 }
 
 // one CTA per (trace, y tap), threads over the x-z taps (z fastest)
-__global__ void inject_scatter_k(TraceDev t, int it, float *__restrict__ w0, const float *__restrict__ vel, int nx,
-                                 int nz) {
+__global__ void inject_scatter_k(TraceDev t, int it, float *w0, const float *__restrict__ vel, int nx, int nz) {
   dep_launch();
   const int r = t.ids ? t.ids[blockIdx.x] : blockIdx.x;
   const int *o = t.off + 3 * r, *l = t.len + 3 * r;
@@ -60,7 +59,7 @@ __global__ void inject_scatter_k(TraceDev t, int it, float *__restrict__ w0, con
 // shared loads, and a tile is split over kInjSplit CTAs to fill the chip.
 // Sums keep the member order.
 constexpr int kInjTile = kGroupTile, kInjChunk = 32, kInjSplit = 4, kInjRows = kInjTile / kInjSplit;
-__global__ void __launch_bounds__(256) inject_group_k(GroupDev g, TraceDev t, int it, float *__restrict__ w0,
+__global__ void __launch_bounds__(256) inject_group_k(GroupDev g, TraceDev t, int it, float *w0,
                                                       const float *__restrict__ vel, int nx, int ny, int nz) {
   constexpr int CELLS = kInjRows * kInjTile;
   dep_launch();
@@ -138,8 +137,7 @@ __global__ void __launch_bounds__(256) inject_group_k(GroupDev g, TraceDev t, in
 // (3072 receivers of 20^3 taps took 112 us), one step at a time waited on memory
 // for each (65 us; now 25).
 constexpr int kBoxZ = 5, kBoxU = 4;
-__device__ __forceinline__ float extract_box(const TraceDev &t, int r, const float *__restrict__ w0, int nx, int nz,
-                                             int lane) {
+__device__ __forceinline__ float extract_box(const TraceDev &t, int r, const float *w0, int nx, int nz, int lane) {
   const int *o = t.off + 3 * r, *l = t.len + 3 * r;
   const int lx = l[0], ly = l[1], lz = l[2];
   const float *kx = t.kx + (long long)r * t.lx, *ky = t.ky + (long long)r * t.ly, *kz = t.kz + (long long)r * t.lz;
@@ -178,8 +176,7 @@ __device__ __forceinline__ float extract_box(const TraceDev &t, int r, const flo
 }
 
 // one warp per receiver over its kernel box
-__global__ void extract_direct_k(TraceDev t, const float *__restrict__ w0, float *__restrict__ out, int jt, int nt_out,
-                                 int nx, int nz) {
+__global__ void extract_direct_k(TraceDev t, const float *w0, float *out, int jt, int nt_out, int nx, int nz) {
   dep_launch();
   dep_wait();
   const int k0 = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
@@ -195,8 +192,8 @@ __global__ void extract_direct_k(TraceDev t, const float *__restrict__ w0, float
 // every load of the tile is in flight at once; with a warp walking 32 columns
 // one after the other, a load and five shuffles each, the pass took 28-30 us
 // on every grid, as long as the stencil of a 128^3 shot.
-__global__ void __launch_bounds__(256) extract_zplane_k(GroupDev g, const float *__restrict__ w0,
-                                                        float *__restrict__ plane, int nx, int ny, int nz) {
+__global__ void __launch_bounds__(256) extract_zplane_k(GroupDev g, const float *w0, float *plane, int nx, int ny,
+                                                        int nz) {
   const int T = g.tile;
   const int tile = blockIdx.x;
   const int c = blockIdx.y * (blockDim.x / 4) + threadIdx.x / 4, zq = threadIdx.x & 3;
@@ -220,8 +217,8 @@ __global__ void __launch_bounds__(256) extract_zplane_k(GroupDev g, const float 
 // indices advanced without divisions.  Bound by the chain record -> taps and
 // plane -> sum, so the member record holds all that the addresses need.
 constexpr int kXyU = 7;
-__global__ void __launch_bounds__(256) extract_xy_k(GroupDev g, TraceDev t, const float *__restrict__ plane,
-                                                    float *__restrict__ out, int jt, int nt_out, int nx) {
+__global__ void __launch_bounds__(256) extract_xy_k(GroupDev g, TraceDev t, const float *plane, float *out, int jt,
+                                                    int nt_out, int nx) {
   const int m = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x & 31;
   dep_launch();
@@ -256,7 +253,7 @@ __global__ void __launch_bounds__(256) extract_xy_k(GroupDev g, TraceDev t, cons
 }
 
 // per-slab max |w| (one CTA per y slab)
-__global__ void slab_max_k(const float *__restrict__ w, float *__restrict__ slab, uint16_t *c16, int fmt, long long nxz) {
+__global__ void slab_max_k(const float *w, float *slab, uint16_t *c16, int fmt, long long nxz) {
   dep_launch();
   dep_wait();
   const int iy = blockIdx.x;

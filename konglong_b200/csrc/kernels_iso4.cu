@@ -389,13 +389,13 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
     for (int p = y0; p < min(y0 + P, y1); p++) issue_b(p), last_b = p;
   }
   // the queue's first 8 planes (y0-4 .. y0+3) of the own column from global memory
-  const float4 *__restrict__ w1g = reinterpret_cast<const float4 *>(a.w1);
+  const float4 *w1g = reinterpret_cast<const float4 *>(a.w1);
   const long long nxz4 = g.nxz / 4, col4 = col / 4;
   float4 q[2 * R4 + 1];
 #pragma unroll
   for (int k = 0; k < 2 * R4; k++) {
     const int y = y0 - R4 + k;
-    q[k] = act && y >= 0 && y < ny ? __ldcg(w1g + y * nxz4 + col4) : zero4;
+    q[k] = act && y >= 0 && y < ny ? ld_l2(w1g + y * nxz4 + col4) : zero4;
   }
   // the round-1 memory of a face is one round stride (its component stride) on
   TileFaces<0> pm;

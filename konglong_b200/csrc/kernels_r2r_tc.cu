@@ -136,7 +136,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // shared memory.  Stage s: raw A | A hi | A lo | B hi | B lo; S stages.
 template <int S>
 __global__ void __launch_bounds__(kTcThreads, 1)
-    r2r_tc_k(const float *__restrict__ in, float *__restrict__ out, const unsigned char *__restrict__ Bg, int n, int npad,
+    r2r_tc_k(const float *in, float *out, const unsigned char *__restrict__ Bg, int n, int npad,
              TcGeom geo, int *err) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   uint64_t *rawf = reinterpret_cast<uint64_t *>(smraw);  // [S] raw A copies and B bytes landed
@@ -341,7 +341,7 @@ struct TtShape {
 
 template <int MODE, int KU>
 __global__ void __launch_bounds__(kTtThreads, 1)
-    r2r_tt_k(const float *__restrict__ in, float *__restrict__ out, const unsigned char *__restrict__ Bg, int n, int npad,
+    r2r_tt_k(const float *in, float *out, const unsigned char *__restrict__ Bg, int n, int npad,
              TtShape sh, TcGeom geo, int *err) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   uint64_t *rawf = reinterpret_cast<uint64_t *>(smraw);  // [S] raw A copies and B bytes landed

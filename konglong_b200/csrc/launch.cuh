@@ -7,7 +7,18 @@
 // and its writes are visible.  What stands before dep_wait() (barriers, tables,
 // trace taps, model constants) runs while the kernel before drains; on a 601 x
 // 300 line shot, whose kernels take 3-8 us, set-up and drain were a third of the
-// step.  Every thread of every such kernel calls dep_wait(), so that one
+// step.
+//
+// Such a kernel is resident while the one before still writes, so what a step
+// writes (wavefields, gradient parts, slab scales, receiver planes, PML and Q
+// memory) is read behind dep_wait() by ordinary loads, ld_l2() or asynchronous
+// copies.  The read-only path (__ldg) asks for data that nobody writes during the
+// kernel's lifetime; a load through a __restrict__ pointer may become one or move
+// above the wait, which such a pointer does not alias; and an intrinsic like
+// __ldcg may move.  __ldg and __restrict__ stay with model volumes and tables.
+// The one-cell FD8 kernels pay nothing for it: see kernels_fd8.cu.
+//
+// Every thread of every such kernel calls dep_wait(), so that one
 // kernel's end implies the end of all before it; a launch without the attribute
 // waits for the whole stream as usual.
 #pragma once
@@ -17,6 +28,15 @@ namespace rtm {
 
 __device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// a coherent load through L2 that stays where it stands, behind the wait
+__device__ __forceinline__ float4 ld_l2(const float4 *p) {
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(__cvta_generic_to_global(p))
+               : "memory");
+  return v;
+}
 
 // Two launches of one pass over disjoint tiles (PML tiles, then interior tiles),
 // the second free to run beside the first: the PML tiles come in one or two
@@ -27,9 +47,7 @@ __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;"
 // each pair), and a second launch that does not find its number waits as usual.  The
 // second launch calls dep_wait() as its last act instead of its first: its end
 // then implies the end of the first, and the kernel after it need wait for
-// nothing more.  A second launch reads what the step writes through L2 (TMA, .cg)
-// or by ordinary loads after its acquire, never through the read-only path, which
-// an acquire does not cover.  No launch waits for one behind it: the second is let in when
+// nothing more.  For its loads the acquire stands in for dep_wait().  No launch waits for one behind it: the second is let in when
 // every CTA of the first has its place.
 enum { PAIR_NONE = 0, PAIR_FIRST = 1, PAIR_SECOND = 2 };
 struct LaunchPair {
