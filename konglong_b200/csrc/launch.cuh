@@ -16,7 +16,6 @@
 // kernel's lifetime; a load through a __restrict__ pointer may become one or move
 // above the wait, which such a pointer does not alias; and an intrinsic like
 // __ldcg may move.  __ldg and __restrict__ stay with model volumes and tables.
-// The one-cell FD8 kernels pay nothing for it: see kernels_fd8.cu.
 //
 // Every thread of every such kernel calls dep_wait(), so that one
 // kernel's end implies the end of all before it; a launch without the attribute
