@@ -479,23 +479,27 @@ int rtm_set_compressor_fallback(rtm_handle *h, float tau, float max_fraction);
 
 /* ---- Batched small shots (many shots side by side on one device) ----
  * A batch steps several FD8 handles (no Q) of different grids and step counts
- * together, all ISO, all VTI or all TTI (no density, FP32 state): each shot's
- * own step, injection and extraction kernels on its own stream, the launches
- * interleaved step by step, so that small grids share the chip.  Each handle must
- * have its model, injection (and, optionally, extraction) set and be reset.
+ * together, all ISO, all VTI or all TTI (no density, FP32 state).  Either each
+ * shot's own step, injection and extraction kernels run on its own stream, the
+ * launches interleaved step by step; or, for shots so small that the host's
+ * launches would bound them, one persistent launch a pass steps all shots' tiles,
+ * one injects and one extracts.  Each handle must have its model, injection (and,
+ * optionally, extraction) set and be reset.
  * No reference counterpart: bgprtm runs one shot per process
  * (bgprtm/Propagator.cpp:1054-1260 per shot). */
 typedef struct rtm_batch rtm_batch;
 int rtm_batch_create(rtm_handle *const *shots, int nshots, rtm_batch **out);
 int rtm_batch_destroy(rtm_batch *b);
 /* rtm_modelling(shots[s], nts[s], it_shift, ntratio) for every shot at once:
- * same wavefields and traces. */
+ * same wavefields and traces (with shared launches receiver sums, and sums of
+ * sources that overlap, may differ in the last bit). */
 int rtm_batch_modelling(rtm_batch *b, const int *nts, int it_shift, int ntratio);
 /* Device time of the last rtm_batch_modelling (ms). */
 int rtm_batch_last_ms(rtm_batch *b, float *ms);
-/* Times `steps` batched steps with the shots' present kernels (0) and with the
- * ones rtm_autotune chooses for each (1), keeps the faster and returns its index;
- * zeroes the shots' wavefields, PML memory and traces (as rtm_reset). */
+/* Times `steps` batched steps with the shots' present kernels (0), with the ones
+ * rtm_autotune chooses for each (1) and with shared ones (2), keeps the fastest and
+ * returns its index; zeroes the shots' wavefields, PML memory and traces (as
+ * rtm_reset). */
 int rtm_batch_autotune(rtm_batch *b, int steps, int *choice);
 
 /* Failure detection.  rtm_check_finite scans field RTM_FIELD_W0 / W1 / IMAGE on

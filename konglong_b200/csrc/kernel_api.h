@@ -28,6 +28,16 @@ struct IsoArgs {
   QDev q;
 };
 
+// one shot of a batched step (device array): its I/O and ISO step arguments, its
+// two wavefield buffers (w1 = wa on even steps) and its tile grid
+struct IsoBatchShot {
+  IsoArgs a;
+  float *wa, *wb;
+  int tiles_z, tiles_x, tiles_y;
+  TraceDev inj, ext;  // source traces (scatter) and receivers (gathered into ext_out)
+  float *ext_out;     // [ext.ntr][ext.nt]
+};
+
 // FP16 wavefield state (per-y-slab scale: value = half * scale[iy])
 struct StateF16 {
   const __half *w1;     // current field, scale s1
@@ -61,6 +71,30 @@ struct DivArgs {
   PmlDev pml;
   QDev q;
 };
+
+// one VTI / TTI shot of a batched two-pass step (device array): its pass
+// arguments, its wavefield buffers and its tile grid
+struct AnisoBatchShot {
+  GradArgs g;
+  DivArgs d;
+  float *wa, *wb;
+  int tiles_z, tiles_x, tiles_y, yseg;
+};
+constexpr int kBatchTX = 8;  // tile width of the batched kernels
+// step `it` of every active shot of a batch (leapfrog): shots[0..nactive) device
+// array, start[] their first tiles (start[nactive] = total), ctas resident CTAs
+void launch_iso_fd8_batch(const IsoBatchShot *shots, const int *start, int nactive, int total, int it, int pml3d,
+                          int ctas, cudaStream_t st);
+void launch_aniso_fd8_batch(const AnisoBatchShot *shots, const int *start, int nactive, int total, int it, int model,
+                            int ctas, cudaStream_t st);
+// the CTAs per SM they keep resident
+int iso_batch_ctas_per_sm(int pml3d);
+int aniso_batch_ctas_per_sm();
+// source injection at trace sample it_src and receiver extraction at sample jt,
+// into the step-`it` output buffers of shots[0..nactive)
+void launch_batch_inject(const IsoBatchShot *shots, int nactive, int max_ntr, int max_ly, int it_src, int it,
+                         cudaStream_t st);
+void launch_batch_extract(const IsoBatchShot *shots, int nactive, int max_ntr, int jt, int it, cudaStream_t st);
 
 // mode: 0 = operator only (w0 -= vel*L), 1 = + leapfrog update, 2 = + Q update
 void launch_iso_fd8(const IsoArgs &a, int mode, int pml3d, int tx, cudaStream_t st);

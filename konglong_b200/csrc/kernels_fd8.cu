@@ -94,7 +94,7 @@ __device__ __forceinline__ void put_tile(float (*tile)[TZ + 2 * R], const Halo &
 
 // One 32 (z) x TX (x) column tile of an ISO step, marching y over segment
 // bz (planes bz*yseg .. ), tile (bx, by); w1 / w0 are the wavefields of this
-// step.
+// step (the batched kernel passes a shot's buffers of the current parity).
 // The coefficients and the PML widths are read once into registers.
 template <int TX, int MODE, bool PML3D>
 __device__ __forceinline__ void iso_tile(const IsoArgs &a, const float *w1, float *w0, int bx, int by,
@@ -191,6 +191,37 @@ __global__ void __launch_bounds__(TZ *TX) iso_fd8_step(IsoArgs a) {
   dep_launch();
   dep_wait();
   iso_tile<TX, MODE, PML3D>(a, a.w1, a.w0, blockIdx.x, blockIdx.y, blockIdx.z, tile);
+}
+
+// The shot of a batch that holds tile w: start[s] = first tile of shot s
+__device__ __forceinline__ int batch_shot(const int *start, int nactive, int w) {
+  int lo = 0, hi = nactive - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (start[mid] <= w) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+// Many shots in one persistent launch, for batches of shots so small that the
+// host's launches of each shot's own kernels bound them (batch_shared in
+// rtm_capi.cu): the work items are the column tiles of the active shots (a prefix
+// of the step-count-sorted batch), laid end to end; each CTA strides over them.
+// Shot s steps its buffers wa / wb in lockstep with the others: at step `it` w1 is
+// wa on even steps and wb on odd ones.  Leapfrog update (MODE 1), no snapshot I/O.
+template <int TX, bool PML3D>
+__global__ void __launch_bounds__(TZ *TX) iso_fd8_batch(const IsoBatchShot *shots, const int *start, int nactive,
+                                                         int total, int it) {
+  __shared__ float tile[TX + 2 * R][TZ + 2 * R];
+  dep_launch();
+  dep_wait();
+  for (int w = blockIdx.x; w < total; w += gridDim.x) {
+    const int s = batch_shot(start, nactive, w), l = w - start[s];
+    const IsoBatchShot &S = shots[s];
+    const int bx = l % S.tiles_z, by = (l / S.tiles_z) % S.tiles_x, bz = l / (S.tiles_z * S.tiles_x);
+    iso_tile<TX, 1, PML3D>(S.a, (it & 1) ? S.wb : S.wa, (it & 1) ? S.wa : S.wb, bx, by, bz, tile);
+  }
 }
 
 // ---- anisotropic two-pass ----------------------------------------------------
@@ -382,6 +413,40 @@ __global__ void __launch_bounds__(TZ *TX) div_fd8(DivArgs a, const Tile4 *__rest
   div_tile<TX, MODE, F16, EDGE>(a, a.w1, a.w0, tl.bz, tl.bx, tl.y0, tl.y1, tpx, tpz);
 }
 
+// Many VTI / TTI shots in two persistent launches per step (gradient pass over
+// every active shot's column tiles, then the divergence pass), the work items laid
+// out as in iso_fd8_batch; every tile takes the PML code path.
+template <int TX, int MODEL>
+__global__ void __launch_bounds__(TZ *TX) grad_fd8_batch(const AnisoBatchShot *shots, const int *start, int nactive,
+                                                          int total, int it) {
+  __shared__ float tile[TX + 2 * R][TZ + 2 * R];
+  dep_launch();
+  dep_wait();
+  for (int w = blockIdx.x; w < total; w += gridDim.x) {
+    const int s = batch_shot(start, nactive, w), l = w - start[s];
+    const AnisoBatchShot &S = shots[s];
+    const int bz = l % S.tiles_z, bx = (l / S.tiles_z) % S.tiles_x, by = l / (S.tiles_z * S.tiles_x);
+    const int y0 = by * S.yseg, y1 = min(S.g.ny, y0 + S.yseg);
+    grad_tile<TX, MODEL, false, true>(S.g, (it & 1) ? S.wb : S.wa, bz, bx, y0, y1, tile);
+  }
+}
+
+template <int TX>
+__global__ void __launch_bounds__(TZ *TX) div_fd8_batch(const AnisoBatchShot *shots, const int *start, int nactive,
+                                                         int total, int it) {
+  __shared__ float tpx[TX + 2 * R][TZ];
+  __shared__ float tpz[TX][TZ + 2 * R];
+  dep_launch();
+  dep_wait();
+  for (int w = blockIdx.x; w < total; w += gridDim.x) {
+    const int s = batch_shot(start, nactive, w), l = w - start[s];
+    const AnisoBatchShot &S = shots[s];
+    const int bz = l % S.tiles_z, bx = (l / S.tiles_z) % S.tiles_x, by = l / (S.tiles_z * S.tiles_x);
+    const int y0 = by * S.yseg, y1 = min(S.d.ny, y0 + S.yseg);
+    div_tile<TX, 1, false, true>(S.d, (it & 1) ? S.wb : S.wa, (it & 1) ? S.wa : S.wb, bz, bx, y0, y1, tpx, tpz);
+  }
+}
+
 }  // namespace
 
 static dim3 fd_grid(int nx, int ny, int nz, int tx, int yseg) {
@@ -408,6 +473,38 @@ void launch_iso_fd8(const IsoArgs &a, int mode, int pml3d, int tx, cudaStream_t 
   if (tx == 4) iso_launch_tx<4>(a, mode, pml3d, st);
   else if (tx == 16) iso_launch_tx<16>(a, mode, pml3d, st);
   else iso_launch_tx<8>(a, mode, pml3d, st);
+}
+
+void launch_iso_fd8_batch(const IsoBatchShot *shots, const int *start, int nactive, int total, int it, int pml3d,
+                          int ctas, cudaStream_t st) {
+  if (total <= 0 || nactive <= 0) return;
+  const unsigned grid = (unsigned)std::max(1, std::min(total, ctas));
+  auto *k = pml3d ? iso_fd8_batch<kBatchTX, true> : iso_fd8_batch<kBatchTX, false>;
+  launch_dep(k, grid, dim3(TZ, kBatchTX), 0, st, shots, start, nactive, total, it);
+}
+
+int iso_batch_ctas_per_sm(int pml3d) {
+  int n = 0;
+  if (pml3d) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, iso_fd8_batch<kBatchTX, true>, TZ * kBatchTX, 0);
+  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, iso_fd8_batch<kBatchTX, false>, TZ * kBatchTX, 0);
+  return std::max(1, n);
+}
+
+void launch_aniso_fd8_batch(const AnisoBatchShot *shots, const int *start, int nactive, int total, int it, int model,
+                            int ctas, cudaStream_t st) {
+  if (total <= 0 || nactive <= 0) return;
+  const unsigned grid = (unsigned)std::max(1, std::min(total, ctas));
+  const dim3 block(TZ, kBatchTX);
+  auto *k = model == 3 ? grad_fd8_batch<kBatchTX, 3> : grad_fd8_batch<kBatchTX, 2>;
+  launch_dep(k, grid, block, 0, st, shots, start, nactive, total, it);
+  launch_dep(div_fd8_batch<kBatchTX>, grid, block, 0, st, shots, start, nactive, total, it);
+}
+
+int aniso_batch_ctas_per_sm() {
+  int a = 0, b = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, grad_fd8_batch<kBatchTX, 3>, TZ * kBatchTX, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, div_fd8_batch<kBatchTX>, TZ * kBatchTX, 0);
+  return std::max(1, std::min(a, b));
 }
 
 template <int TX, bool F16, bool EDGE>

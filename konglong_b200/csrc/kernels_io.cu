@@ -28,15 +28,10 @@ __global__ void update2nd_q_k(float *__restrict__ w0, const float *__restrict__ 
 }
 
 // one CTA per (trace, y tap), threads over the x-z taps (z fastest)
-__global__ void inject_scatter_k(TraceDev t, int it, float *w0, const float *__restrict__ vel, int nx, int nz) {
-  dep_launch();
-  const int r = t.ids ? t.ids[blockIdx.x] : blockIdx.x;
+__device__ __forceinline__ void scatter_taps(const TraceDev &t, int r, int iy, float val, float *w0, const float *vel,
+                                             int nx, int nz) {
   const int *o = t.off + 3 * r, *l = t.len + 3 * r;
-  const int lx = l[0], lz = l[2];
-  const int iy = blockIdx.y;
-  const float val = t.traces[(long long)r * t.nt + it] * t.scaler;
-  const int ntap = lx * lz;
-  dep_wait();
+  const int lx = l[0], lz = l[2], ntap = lx * lz;
   if (iy >= l[1]) return;
   for (int k = threadIdx.x; k < ntap; k += blockDim.x) {
     const int iz = k % lz, ix = k / lz;
@@ -45,6 +40,23 @@ __global__ void inject_scatter_k(TraceDev t, int it, float *w0, const float *__r
     const long long c = ((long long)(iy + o[1]) * nx + ix + o[0]) * nz + o[2] + iz;
     atomicAdd(w0 + c, cx * t.kz[(long long)r * t.lz + iz] * vel[c]);
   }
+}
+__global__ void inject_scatter_k(TraceDev t, int it, float *w0, const float *__restrict__ vel, int nx, int nz) {
+  dep_launch();
+  const int r = t.ids ? t.ids[blockIdx.x] : blockIdx.x;
+  const float val = t.traces[(long long)r * t.nt + it] * t.scaler;
+  dep_wait();
+  scatter_taps(t, r, blockIdx.y, val, w0, vel, nx, nz);
+}
+// the same for every shot of a batch (blockIdx.z = shot), into each shot's step-`it` output
+__global__ void batch_inject_k(const IsoBatchShot *shots, int it_src, int it) {
+  dep_launch();
+  dep_wait();
+  const IsoBatchShot &S = shots[blockIdx.z];
+  const int r = blockIdx.x;
+  if (r >= S.inj.ntr || it_src < 0 || it_src >= S.inj.nt) return;
+  const float val = S.inj.traces[(long long)r * S.inj.nt + it_src] * S.inj.scaler;
+  scatter_taps(S.inj, r, blockIdx.y, val, (it & 1) ? S.wa : S.wb, S.a.vel, S.a.nx, S.a.nz);
 }
 
 // Grouped injection: a CTA of (group tile, quarter of its rows).  Every cell
@@ -185,6 +197,17 @@ __global__ void extract_direct_k(TraceDev t, const float *w0, float *out, int jt
   const int r = t.ids ? t.ids[k0] : k0;
   const float acc = extract_box(t, r, w0, nx, nz, lane);
   if (lane == 0) out[(long long)r * nt_out + jt] = acc;
+}
+
+// the same for every shot of a batch (blockIdx.y = shot)
+__global__ void batch_extract_k(const IsoBatchShot *shots, int jt, int it) {
+  dep_launch();
+  dep_wait();
+  const IsoBatchShot &S = shots[blockIdx.y];
+  const int r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
+  if (r >= S.ext.ntr || jt < 0 || jt >= S.ext.nt) return;
+  const float acc = extract_box(S.ext, r, (it & 1) ? S.wa : S.wb, S.a.nx, S.a.nz, lane);
+  if (lane == 0) S.ext_out[(long long)r * S.ext.nt + jt] = acc;
 }
 
 // z reduction of a group's band on its tiles: plane[iy*nx+ix] = sum kz * w0.
@@ -368,6 +391,17 @@ void launch_inject_scatter(const TraceDev &t, int it, float *w0, const float *ve
   const int cnt = t.ids ? t.nids : t.ntr;
   if (cnt <= 0 || it < 0 || it >= t.nt) return;
   launch_dep(inject_scatter_k, dim3(cnt, t.ly), 256, 0, st, t, it, w0, vel, nx, nz);
+}
+
+void launch_batch_inject(const IsoBatchShot *shots, int nactive, int max_ntr, int max_ly, int it_src, int it,
+                         cudaStream_t st) {
+  if (nactive <= 0 || max_ntr <= 0 || max_ly <= 0) return;
+  launch_dep(batch_inject_k, dim3(max_ntr, max_ly, nactive), 256, 0, st, shots, it_src, it);
+}
+
+void launch_batch_extract(const IsoBatchShot *shots, int nactive, int max_ntr, int jt, int it, cudaStream_t st) {
+  if (nactive <= 0 || max_ntr <= 0) return;
+  launch_dep(batch_extract_k, dim3((max_ntr + 7) / 8, nactive), 256, 0, st, shots, jt, it);
 }
 
 // ---- FP16 wavefield state ----------------------------------------------------

@@ -1353,9 +1353,122 @@ struct rtm_batch {
   cudaStream_t st = nullptr;      // the streams fork from it and join it (timing)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0.f;
+  int form = -1;  // of its steps, if rtm_batch_autotune chose: 0 each shot's own kernels, 1 shared ones
+  // shared steps: device tables of the shots (sorted by step count), room for cap shots
+  rtm::IsoBatchShot *d_shots = nullptr;
+  rtm::AnisoBatchShot *d_ashots = nullptr;  // VTI / TTI
+  int *d_start = nullptr;
+  int cap = 0;
 };
 
 namespace rtm {
+// Whether a batch's steps are launched as shared kernels: one persistent launch a
+// pass over all shots' tiles, one of injection and one of extraction.  They are the
+// one-cell kernels, slower than each shot's own, but a step is 3 or 4 launches for
+// all shots.  A shot's own step costs the host 4 us (VTI / TTI 8) and 2 us for every
+// launch of injection and extraction.  What a shared step takes, fitted to batches
+// of 8 - 128 shots of 28 - 96 cells an axis (us): 30, 1.2 more a shot and 32 a million
+// cells (VTI / TTI 30, 3.2 and 110).  Measured steps, own / shared kernels: 64 ISO
+// shots of 28 - 40 cells 505 / 144 us, of 44 - 64 cells 475 / 315, of 64 - 80 cells
+// 528 / 681; 12 of 64 - 96 cells 121 / 193; 64 VTI shots of 28 - 40 cells 717 / 393,
+// of 36 - 56 cells 676 / 696.
+static bool batch_shared(const rtm_batch *b, const int *nts) {
+  if (b->form >= 0) return b->form == 1;
+  const bool iso = b->shots[0]->lap_iso();
+  double host = 0, cells = 0, steps = 0, most = 0;
+  for (size_t k = 0; k < b->shots.size(); k++) {
+    const Engine *s = b->shots[k];
+    const size_t io = s->inj.groups.size() + 2 * s->ext.groups.size() + (s->inj.n_ungrouped > 0) + (s->ext.n_ungrouped > 0);
+    host += nts[k] * ((iso ? 4.0 : 8.0) + 2.0 * io);
+    cells += 1e-6 * nts[k] * s->n;
+    steps += nts[k];
+    most = std::max(most, (double)nts[k]);
+  }
+  return host > 30 * most + (iso ? 1.2 * steps + 32 * cells : 3.2 * steps + 110 * cells);
+}
+
+constexpr int kBatchYseg = 8;  // y segment of their tiles (16: up to 1.2x slower, whole columns 1.1 - 1.6x)
+// Steps of the shots as shared kernels, the shots sorted by step count: those
+// active at step `it` are the first of the table.
+static int batch_run_shared(rtm_batch *b, const int *nts, int it_shift, int ntratio) {
+  Engine *h = b->shots[0];
+  const int n = (int)b->shots.size();
+  const bool aniso = h->c.model_type != RTM_ISO;
+  std::vector<int> order(n), start(n + 1, 0);
+  for (int k = 0; k < n; k++) order[k] = k;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return nts[x] > nts[y]; });
+  std::vector<IsoBatchShot> hs(n);
+  std::vector<AnisoBatchShot> ha(aniso ? n : 0);
+  int max_inj = 0, max_ly = 0, max_ext = 0;
+  for (int k = 0; k < n; k++) {
+    Engine *s = b->shots[order[k]];
+    const rtm_dims &d = s->d;
+    IsoBatchShot &S = hs[k];
+    S = IsoBatchShot{};
+    IsoArgs &a = S.a;
+    a.nx = d.nx, a.ny = d.ny, a.nz = d.nz, a.yseg = std::min(kBatchYseg, d.ny);
+    a.w1 = s->w1, a.w0 = s->w0, a.vel = s->vel;
+    memcpy(a.c2x, s->c2x, sizeof a.c2x), memcpy(a.c2y, s->c2y, sizeof a.c2y), memcpy(a.c2z, s->c2z, sizeof a.c2z);
+    a.pml = pml_dev(s);
+    S.wa = s->w1, S.wb = s->w0;
+    S.tiles_z = (d.nz + 31) / 32, S.tiles_x = (d.nx + kBatchTX - 1) / kBatchTX, S.tiles_y = (d.ny + a.yseg - 1) / a.yseg;
+    S.inj = s->inj.dev(), S.ext = s->ext.dev(), S.ext_out = s->ext.out;
+    S.inj.ids = nullptr, S.ext.ids = nullptr;
+    if (aniso) {
+      AnisoBatchShot &A = ha[k];
+      A = AnisoBatchShot{};
+      GradArgs &g = A.g;
+      g.nx = d.nx, g.ny = d.ny, g.nz = d.nz, g.yseg = a.yseg, g.pml3d = s->c.pml3d;
+      g.px = s->px, g.py = s->py, g.pz = s->pz;
+      g.eps = s->eps, g.del = s->del, g.pjx = s->pjx, g.pjy = s->pjy;
+      memcpy(g.c1x, s->c1x, sizeof g.c1x), memcpy(g.c1y, s->c1y, sizeof g.c1y), memcpy(g.c1z, s->c1z, sizeof g.c1z);
+      g.pml = a.pml;
+      DivArgs &v = A.d;
+      v.nx = d.nx, v.ny = d.ny, v.nz = d.nz, v.yseg = a.yseg, v.pml3d = s->c.pml3d;
+      v.px = s->px, v.py = s->py, v.pz = s->pz, v.vel = s->vel;
+      memcpy(v.c1x, s->c1x, sizeof v.c1x), memcpy(v.c1y, s->c1y, sizeof v.c1y), memcpy(v.c1z, s->c1z, sizeof v.c1z);
+      v.pml = a.pml;
+      A.wa = S.wa, A.wb = S.wb;
+      A.tiles_z = S.tiles_z, A.tiles_x = S.tiles_x, A.tiles_y = S.tiles_y, A.yseg = a.yseg;
+    }
+    start[k + 1] = start[k] + S.tiles_z * S.tiles_x * S.tiles_y;
+    max_inj = std::max(max_inj, s->inj.ntr), max_ly = std::max(max_ly, s->inj.ly);
+    max_ext = std::max(max_ext, s->ext.ntr);
+  }
+  if (n > b->cap) {
+    cudaFree(b->d_shots), cudaFree(b->d_ashots), cudaFree(b->d_start);
+    b->d_shots = nullptr, b->d_ashots = nullptr, b->d_start = nullptr, b->cap = 0;
+    CK(cudaMalloc(&b->d_shots, n * sizeof(IsoBatchShot)));
+    if (aniso) CK(cudaMalloc(&b->d_ashots, n * sizeof(AnisoBatchShot)));
+    CK(cudaMalloc(&b->d_start, (n + 1) * sizeof(int)));
+    b->cap = n;
+  }
+  CK(cudaMemcpyAsync(b->d_shots, hs.data(), n * sizeof(IsoBatchShot), cudaMemcpyHostToDevice, b->st));
+  if (aniso) CK(cudaMemcpyAsync(b->d_ashots, ha.data(), n * sizeof(AnisoBatchShot), cudaMemcpyHostToDevice, b->st));
+  CK(cudaMemcpyAsync(b->d_start, start.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, b->st));
+  // the shots' streams may still hold work on their buffers
+  for (int k = 0; k < n; k++) {
+    CK(cudaEventRecord(b->done[k], b->shots[k]->st));
+    CK(cudaStreamWaitEvent(b->st, b->done[k], 0));
+  }
+  const int ctas = h->sms * (aniso ? aniso_batch_ctas_per_sm() : iso_batch_ctas_per_sm(h->c.pml3d));
+  CK(cudaEventRecord(b->ev0, b->st));
+  for (int it = 0, na = n; it < nts[order[0]]; it++) {
+    while (nts[order[na - 1]] <= it) na--;
+    if (aniso) launch_aniso_fd8_batch(b->d_ashots, b->d_start, na, start[na], it, h->c.model_type, ctas, b->st);
+    else launch_iso_fd8_batch(b->d_shots, b->d_start, na, start[na], it, h->c.pml3d, ctas, b->st);
+    launch_batch_inject(b->d_shots, na, max_inj, max_ly, it + it_shift, it, b->st);
+    if (ntratio > 0 && it % ntratio == 0) launch_batch_extract(b->d_shots, na, max_ext, it / ntratio, it, b->st);
+    TRY(check_launch(h, "batched step"));
+  }
+  CK(cudaEventRecord(b->ev1, b->st));
+  CK(cudaEventSynchronize(b->ev1));
+  CK(cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1));
+  for (int k = 0; k < n; k++)  // each shot swapped its wavefields once a step
+    if (nts[k] & 1) do_swap(b->shots[k]);
+  return RTM_OK;
+}
+
 // nts[k] steps of every shot, each on its handle's own stream, the launches
 // interleaved step by step.  A small shot leaves most of the chip idle (128^3:
 // 432 PML tiles of a step's 21 us, 88 interior tiles of its 11 us, receiver
@@ -1365,6 +1478,7 @@ namespace rtm {
 // shots of 96 - 160 cells an axis, as long as the shots one after the other.
 // ntratio > 0 records the receivers every ntratio steps.
 static int batch_run(rtm_batch *b, const int *nts, int it_shift, int ntratio) {
+  if (batch_shared(b, nts)) return batch_run_shared(b, nts, it_shift, ntratio);
   const int n = (int)b->shots.size();
   Engine *h = nullptr;  // CK's error text
   CK(cudaEventRecord(b->ev0, b->st));
@@ -2522,6 +2636,7 @@ int rtm_batch_destroy(rtm_batch *b) {
   cudaSetDevice(b->device);
   if (b->st) cudaStreamSynchronize(b->st);
   for (cudaEvent_t e : b->done) cudaEventDestroy(e);
+  cudaFree(b->d_shots), cudaFree(b->d_ashots), cudaFree(b->d_start);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->st) cudaStreamDestroy(b->st);
@@ -2547,21 +2662,23 @@ int rtm_batch_autotune(rtm_batch *b, int steps, int *choice) {
   if (!b || steps < 1) return RTM_ERR_ARG;
   cudaSetDevice(b->device);
   const std::vector<int> nts(b->shots.size(), steps);
-  // candidate 0: the shots' present kernels; 1: each shot's own autotuned ones
-  float ms[2] = {0.f, 0.f};
+  // candidate 0: the shots' present kernels; 1: each shot's own autotuned ones; 2: shared ones
+  float ms[3] = {0.f, 0.f, 0.f};
   std::vector<rtm::LaunchShape> before;
   for (rtm::Engine *h : b->shots) before.push_back(rtm::launch_shape(h));
-  for (int c = 0; c < 2; c++) {
-    if (c)
+  for (int c = 0; c < 3; c++) {
+    if (c == 1)
       for (rtm::Engine *h : b->shots) TRY(rtm_autotune(static_cast<rtm_handle *>(h), steps, nullptr));
+    b->form = c / 2;
     TRY(rtm::batch_run(b, std::vector<int>(nts.size(), 1).data(), 0, 0));  // warm-up
     TRY(rtm::batch_run(b, nts.data(), 0, 0));
     ms[c] = b->last_ms;
   }
-  const int best = ms[1] < ms[0] ? 1 : 0;
+  const int best = (int)(std::min_element(ms, ms + 3) - ms);
+  b->form = best / 2;
   for (size_t k = 0; k < b->shots.size(); k++) {
     rtm::Engine *h = b->shots[k];
-    if (!best) TRY(rtm::set_launch_shape(h, before[k]));
+    if (best != 1) TRY(rtm::set_launch_shape(h, before[k]));
     TRY(rtm::zero_state(h));
     CK(cudaStreamSynchronize(h->st));
   }

@@ -375,10 +375,11 @@ def checkpoint_slots_for_budget(nts_fwd, interval, slot_bytes, ckpt_bytes, budge
 
 
 class Batch:
-    """Several FD8 shots stepped together (rtm_batch_*), each on its own stream,
-    side by side on the device.  The shots keep their own state:
-    after `modelling`, each Propagator holds what its own `modelling` call
-    would have produced."""
+    """Several FD8 shots stepped together (rtm_batch_*): each shot's kernels on its
+    own stream, or, where the shots are so small that launching those would take
+    longer than running them, kernels shared by all shots.  The shots keep their
+    own state: after `modelling`, each Propagator holds what its own `modelling`
+    call would have produced (shared kernels: receiver sums to the last bit)."""
 
     def __init__(self, shots):
         self.L = _lib.lib()
@@ -400,7 +401,7 @@ class Batch:
             pass
 
     def autotune(self, steps=5):
-        """The faster of the shots' present and autotuned kernels (zeroes the shots' state)."""
+        """The fastest of the shots' present, autotuned and shared kernels (zeroes the shots' state)."""
         ch = C.c_int(0)
         _lib.check(self.L.rtm_batch_autotune(self.b, steps, C.byref(ch)), "rtm_batch_autotune")
         return ch.value
