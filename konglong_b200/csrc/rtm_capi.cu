@@ -1153,22 +1153,39 @@ static int stage_join(Engine *h) {
   return RTM_OK;
 }
 
+// f() as well, whatever failed before it: the first error and its text stay
+template <typename F> static int also(Engine *h, int rc, F f) {
+  if (rc == RTM_OK) return f();
+  const std::string first = h->err;
+  f();
+  h->err = first;
+  return rc;
+}
+
+// the end of a loop on stream st: its time, once everything submitted has run
+static int loop_end(Engine *h, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1, float *ms) {
+  CK(cudaEventRecord(ev1, st));
+  CK(cudaEventSynchronize(ev1));
+  CK(cudaEventElapsedTime(ms, ev0, ev1));
+  return RTM_OK;
+}
+
 // Runs fn(step index) for `count` steps, timed with events on the engine's
 // stream.  Plain launches: the host submits a step's 3-12 kernels in less time
 // than the GPU takes for them, and the first starts at once; capturing and
 // instantiating a CUDA graph of a loop that runs once cost 3-4 us per launch
 // before its first kernel could start (601 x 300 line shot of 50 steps: 1.69 ->
-// 1.44 ms, 128^3 shot of 100 steps: 5.2 -> 4.8 ms without it).
+// 1.44 ms, 128^3 shot of 100 steps: 5.2 -> 4.8 ms without it).  After a step that
+// fails, what was submitted before it is waited for all the same.
 template <typename F> static int run_loop(Engine *h, int count, F fn) {
   h->launches = 0;
   CK(cudaEventRecord(h->ev0, h->st));
-  for (int s = 0; s < count; s++) TRY(fn(s));
-  TRY(stage_join(h));
-  CK(cudaEventRecord(h->ev1, h->st));
-  CK(cudaEventSynchronize(h->ev1));
-  CK(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
+  int rc = RTM_OK;
+  for (int s = 0; s < count && rc == RTM_OK; s++) rc = fn(s);
+  rc = also(h, rc, [&] { return stage_join(h); });
+  rc = also(h, rc, [&] { return loop_end(h, h->st, h->ev0, h->ev1, &h->last_ms); });
   if (h->prof_on) prof_collect(h);
-  return check_flag(h);
+  return also(h, rc, [&] { return check_flag(h); });
 }
 
 static int ready(Engine *h) {
@@ -1390,7 +1407,7 @@ static bool batch_shared(const rtm_batch *b, const int *nts) {
 constexpr int kBatchYseg = 8;  // y segment of their tiles (16: up to 1.2x slower, whole columns 1.1 - 1.6x)
 // Steps of the shots as shared kernels, the shots sorted by step count: those
 // active at step `it` are the first of the table.
-static int batch_run_shared(rtm_batch *b, const int *nts, int it_shift, int ntratio) {
+static int batch_submit_shared(rtm_batch *b, const int *nts, int it_shift, int ntratio) {
   Engine *h = b->shots[0];
   const int n = (int)b->shots.size();
   const bool aniso = h->c.model_type != RTM_ISO;
@@ -1461,54 +1478,58 @@ static int batch_run_shared(rtm_batch *b, const int *nts, int it_shift, int ntra
     if (ntratio > 0 && it % ntratio == 0) launch_batch_extract(b->d_shots, na, max_ext, it / ntratio, it, b->st);
     TRY(check_launch(h, "batched step"));
   }
-  CK(cudaEventRecord(b->ev1, b->st));
-  CK(cudaEventSynchronize(b->ev1));
-  CK(cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1));
-  for (int k = 0; k < n; k++)  // each shot swapped its wavefields once a step
+  for (int k = 0; k < n; k++)  // each shot swaps its wavefields once a step
     if (nts[k] & 1) do_swap(b->shots[k]);
   return RTM_OK;
 }
 
-// nts[k] steps of every shot, each on its handle's own stream, the launches
-// interleaved step by step.  A small shot leaves most of the chip idle (128^3:
-// 432 PML tiles of a step's 21 us, 88 interior tiles of its 11 us, receiver
-// kernels of a few us); side by side the shots fill it with the kernels that
-// are fastest for each.  One persistent kernel over all shots' tiles, before,
-// could only be a kernel all shots share, the one-cell one: 0.88 ms a step for 12
-// shots of 96 - 160 cells an axis, as long as the shots one after the other.
-// ntratio > 0 records the receivers every ntratio steps.
-static int batch_run(rtm_batch *b, const int *nts, int it_shift, int ntratio) {
-  if (batch_shared(b, nts)) return batch_run_shared(b, nts, it_shift, ntratio);
+// Steps of every shot by its own kernels, each shot on its handle's own stream, the
+// launches interleaved step by step; the streams fork from the batch's and join it.
+// A small shot leaves much of the chip idle: 12 shots of 96 - 160 cells an axis, 29 -
+// 59 steps, take 19.6 ms side by side and 27.9 ms one after the other (10.1 and 17.8
+// with depths that are multiples of 4).
+static int batch_submit_own(rtm_batch *b, const int *nts, int it_shift, int ntratio) {
+  Engine *h = b->shots[0];
   const int n = (int)b->shots.size();
-  Engine *h = nullptr;  // CK's error text
   CK(cudaEventRecord(b->ev0, b->st));
-  int most = 0;
+  int most = 0, rc = RTM_OK;
   for (int k = 0; k < n; k++) {
     CK(cudaStreamWaitEvent(b->shots[k]->st, b->ev0, 0));
     b->shots[k]->launches = 0;
     most = std::max(most, nts[k]);
   }
-  for (int it = 0; it < most; it++)
-    for (int k = 0; k < n; k++) {
-      if (it >= nts[k]) continue;
-      Engine *s = b->shots[k];
-      TRY(step_kernel(s, 1, io_none()));
-      TRY(do_inject(s, it + it_shift));
-      if (ntratio > 0 && it % ntratio == 0) TRY(do_extract(s, it / ntratio));
-      do_swap(s);
-    }
-  for (int k = 0; k < n; k++) {
-    CK(cudaEventRecord(b->done[k], b->shots[k]->st));
-    CK(cudaStreamWaitEvent(b->st, b->done[k], 0));
-  }
-  CK(cudaEventRecord(b->ev1, b->st));
-  CK(cudaEventSynchronize(b->ev1));
-  CK(cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1));
+  auto step = [&](Engine *s, int it) -> int {
+    TRY(step_kernel(s, 1, io_none()));
+    TRY(do_inject(s, it + it_shift));
+    if (ntratio > 0 && it % ntratio == 0) TRY(do_extract(s, it / ntratio));
+    do_swap(s);
+    return RTM_OK;
+  };
+  for (int it = 0; it < most && rc == RTM_OK; it++)
+    for (int k = 0; k < n && rc == RTM_OK; k++)
+      if (it < nts[k]) rc = step(b->shots[k], it);
+  for (int k = 0; k < n; k++)
+    rc = also(h, rc, [&]() -> int {
+      CK(cudaEventRecord(b->done[k], b->shots[k]->st));
+      CK(cudaStreamWaitEvent(b->st, b->done[k], 0));
+      return RTM_OK;
+    });
+  return rc;
+}
+
+// nts[k] steps of every shot; ntratio > 0 records the receivers every ntratio steps.
+// After a failure every stream is waited for, and every shot's timeout flag taken,
+// all the same; what the batch's own stream fails by is told on the first shot.
+static int batch_run(rtm_batch *b, const int *nts, int it_shift, int ntratio) {
+  Engine *h = b->shots[0];
+  int rc = batch_shared(b, nts) ? batch_submit_shared(b, nts, it_shift, ntratio)
+                                : batch_submit_own(b, nts, it_shift, ntratio);
+  rc = also(h, rc, [&] { return loop_end(h, b->st, b->ev0, b->ev1, &b->last_ms); });
   for (Engine *s : b->shots) {
     if (s->prof_on) prof_collect(s);
-    TRY(check_flag(s));
+    rc = also(s, rc, [&] { return check_flag(s); });
   }
-  return RTM_OK;
+  return rc;
 }
 }  // namespace rtm
 
@@ -2484,12 +2505,15 @@ int rtm_migration(rtm_handle *h, int dir, int it_begin, int it_end, int it_shift
   if (pending.store || pending.ic) {  // the last step's snapshot / image term
     rtm::KScope k(h, RTM_K_IO);
     rtm::launch_fused_io(pending, h->f16 ? rtm::f16_view(h, 1) : h->w1, h->d.nx, h->d.ny, h->d.nz, h->st);
-    TRY(rtm::check_launch(h, "fused_io(last)"));
-    if (off && pending.store) TRY(rtm::offload_d2h(h, pending_slot));
-    TRY(rtm::stage_join(h));
-    CK(cudaStreamSynchronize(h->st));
+    rc = rtm::check_launch(h, "fused_io(last)");
+    if (off && pending.store && rc == RTM_OK) rc = rtm::offload_d2h(h, pending_slot);
+    rc = rtm::also(h, rc, [&] { return rtm::stage_join(h); });
+    rc = rtm::also(h, rc, [&]() -> int {
+      CK(cudaStreamSynchronize(h->st));
+      return RTM_OK;
+    });
   }
-  return RTM_OK;
+  return rc;
 }
 
 int rtm_get(rtm_handle *h, int field, float *dst) {

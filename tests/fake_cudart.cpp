@@ -50,15 +50,18 @@ cudaError_t err(cudaError_t e) {
   if (e != cudaSuccess) S().last = e;
   return e;
 }
-// whether this call of `what` is the one that was asked to fail
-bool fails(const char *what) {
+// whether this call of `what` (a launch: of kernel `name`) is the one that was asked to fail
+bool fails(const std::string &what, const std::string &name = "") {
   State &s = S();
-  return s.fail_after >= 0 && std::string(what).find(s.fail_what) != std::string::npos && s.fail_after-- == 0;
+  const bool is = name.empty() ? s.fail_what == what
+                               : s.fail_what.rfind(what + " ", 0) == 0 &&
+                                     name.find(s.fail_what.substr(what.size() + 1)) != std::string::npos;
+  return s.fail_after >= 0 && is && s.fail_after-- == 0;
 }
 cudaError_t launch(const void *f, cudaStream_t st) {
   State &s = S();
   const std::string &name = s.kernel[f];
-  if (fails(("launch " + name).c_str())) return err(s.fail_code);
+  if (fails("launch", name)) return err(s.fail_code);
   s.count[st]++;
   s.launched.push_back(name);
   return cudaSuccess;
