@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <map>
 #include <string>
 #include <array>
@@ -1225,7 +1226,7 @@ struct TableBlock {
 constexpr size_t kTableIdle = size_t(64) << 20;
 static int upload_traces(Engine *h, TraceSetDev &t, int ntr, int lx, int ly, int lz, const int *off3, const int *len3,
                          const float *kx, const float *ky, const float *kz, const float *traces, int nt, float scaler,
-                         bool extraction) {
+                         bool extraction) try {
   char *mem = t.mem;
   const size_t cap = t.cap;
   t = TraceSetDev{};
@@ -1343,6 +1344,9 @@ static int upload_traces(Engine *h, TraceSetDev &t, int ntr, int lx, int ly, int
   t = std::move(s);
   if (!t.groups.empty() && !h->plane) TRY(h->alloc(h->plane, (size_t)h->d.nx * h->d.ny));
   return RTM_OK;
+} catch (const std::exception &) {  // of the host's containers: the set stays empty
+  h->err = "the trace tables do not fit host memory";
+  return RTM_ERR_NOMEM;
 }
 
 static void edge_taper(int n, int nt, std::vector<float> &w) {
