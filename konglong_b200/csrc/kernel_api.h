@@ -238,12 +238,12 @@ void cfd_tma_box(int n, int *R, int *nb);
 bool cfd_tile_init();
 bool launch_cfd_tile(int axis, const CfdPlanDev &p, const float *in, float *out, int nx, int ny, int nz,
                      const CUtensorMap *tin, const CUtensorMap *tout, int sms, int *err, cudaStream_t st);
-// x / y derivative by the register-streamed kernel (no shared memory)
 // pipelined persistent x / y line solves over TMA tiles (one CTA per SM, a
 // ring of tile buffers, right-hand side fused into the forward pass); false
 // when a ring of three tiles does not fit in shared memory (nothing launched)
 bool launch_cfd_deriv_pipe(int axis, const CfdPlanDev &p, int nx, int ny, int nz, const CUtensorMap *tin,
                            const CUtensorMap *tout, int *err, cudaStream_t st);
+// x / y derivative by the register-streamed kernel (no shared memory)
 void launch_cfd_deriv_stream(int axis, const CfdPlanDev &p, const float *in, float *out, int nx, int ny, int nz,
                              cudaStream_t st);
 
@@ -356,8 +356,7 @@ struct R2rPlans;
 // bounded waits raise
 int r2r_plans_create(R2rPlans **out, int nx, int ny, int nz, float dx, float dy, float dz, cudaStream_t st,
                      bool tensor_cores, int *err);
-// tcgen05 z-line operator (kernels_r2r_tc.cu)
-size_t r2r_tc_smem(int n);
+// tcgen05 line operators (kernels_r2r_tc.cu)
 bool r2r_tc_supported(int axis, int nx, int ny, int nz);
 size_t r2r_tc_bytes(int n);  // the pre-arranged TF32 parts of one n x n line matrix
 int r2r_tc_init();
@@ -372,9 +371,9 @@ void launch_update2nd(float *w0, const float *w1, const QDev *q, long long n, cu
 // atomic scatter of every trace of `t` (Receiver::apply_src)
 void launch_inject_scatter(const TraceDev &t, int it, float *w0, const float *vel, int nx, int ny, int nz,
                            cudaStream_t st);
-// grouped injection: xy plane gather then z expansion
-void launch_inject_group(const GroupDev &gr, const TraceDev &t, int it, float *plane, float *w0, const float *vel,
-                         int nx, int ny, int nz, cudaStream_t st);
+// grouped injection: xy sums of a tile's members, then their z expansion
+void launch_inject_group(const GroupDev &gr, const TraceDev &t, int it, float *w0, const float *vel, int nx, int ny,
+                         int nz, cudaStream_t st);
 void launch_extract_direct(const TraceDev &t, const float *w0, float *out, int jt, int nt_out, int nx, int ny, int nz,
                            cudaStream_t st);
 void launch_extract_group(const GroupDev &gr, const TraceDev &t, const float *w0, float *plane, float *out, int jt,

@@ -688,7 +688,7 @@ __device__ __forceinline__ void div_cell(const CfdDivEpiArgs &a, const Grid3 &g,
 }
 
 // 32 z lines of `in` (line l at l * n) staged through shared memory [l][n + 1]
-// and solved in place (cfd_lines_k's z path); returns the lines in the tile
+// and solved in place; returns the lines in the tile
 __device__ __forceinline__ int zlines_solve(const CfdPlanDev &p, const float *__restrict__ in, float *sm,
                                             long long nlines) {
   const int n = p.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1207,9 +1207,6 @@ __device__ __forceinline__ PmlInterior pml_interior(const PmlDev &P, const Grid3
 }
 // bit d set when coordinate c of dimension d lies in one of its PML layers
 __device__ __forceinline__ int pml_bit(int d, int c, int lo, int hi) { return (c < lo || c >= hi) << d; }
-__device__ __forceinline__ int pml_bits(const PmlInterior &in, int ix, int iy, int iz) {
-  return pml_bit(DX, ix, in.x0, in.x1) | pml_bit(DY, iy, in.y0, in.y1) | pml_bit(DZ, iz, in.z0, in.z1);
-}
 
 // First-derivative PML round `round` on component AXIS of a batch of cells
 // (dm: the layers that hold each cell, 0 = none); skipped when no cell of

@@ -541,9 +541,8 @@ void launch_extract_direct_f16(const TraceDev &t, const __half *h, const float *
   extract_direct_f16_k<<<(t.ntr + 7) / 8, 256, 0, st>>>(t, h, s, out, jt, nt_out, nx, nz);
 }
 
-void launch_inject_group(const GroupDev &gr, const TraceDev &t, int it, float *plane, float *w0, const float *vel,
-                         int nx, int ny, int nz, cudaStream_t st) {
-  (void)plane;
+void launch_inject_group(const GroupDev &gr, const TraceDev &t, int it, float *w0, const float *vel, int nx, int ny,
+                         int nz, cudaStream_t st) {
   if (gr.ntiles <= 0 || it < 0 || it >= t.nt) return;
   launch_dep(inject_group_k, dim3(gr.ntiles, kInjSplit), 256, 0, st, gr, t, it, w0, vel, nx, ny, nz);
 }

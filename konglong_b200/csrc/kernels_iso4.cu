@@ -44,14 +44,6 @@ __device__ __noinline__ float iso4_pml_cell(const PmlDev &P, Grid3 g, float lz, 
   return lz + lx + ly;
 }
 
-__device__ __forceinline__ float comp(const float4 &v, int c) { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
-__device__ __forceinline__ void setc(float4 &v, int c, float x) {
-  if (c == 0) v.x = x;
-  else if (c == 1) v.y = x;
-  else if (c == 2) v.z = x;
-  else v.w = x;
-}
-
 // The split-field PML memory of the face of dimension d that covers the
 // thread's 4 z cells (null when none does) and the layer of its first cell;
 // every face array keeps z fastest, so the 4 cells are one aligned float4.
@@ -220,12 +212,12 @@ __global__ void __launch_bounds__(8 * TX) iso_fd8_v4(const __grid_constant__ Iso
 #pragma unroll
         for (int m = 1; m <= R4; m++) {
           lz += c2z[m] * (zw[4 + c - m] + zw[4 + c + m]);
-          lx += c2x[m] * (comp(xm[m - 1], c) + comp(xp[m - 1], c));
+          lx += c2x[m] * (cmp4(xm[m - 1], c) + cmp4(xp[m - 1], c));
         }
         if (do_y) {
           ly = c2y[0] * u;
 #pragma unroll
-          for (int m = 1; m <= R4; m++) ly += c2y[m] * (comp(q[slot(-m)], c) + comp(q[slot(m)], c));
+          for (int m = 1; m <= R4; m++) ly += c2y[m] * (cmp4(q[slot(-m)], c) + cmp4(q[slot(m)], c));
         }
         lzv[c] = lz, lxv[c] = lx, lyv[c] = ly;
       }
@@ -253,7 +245,7 @@ __global__ void __launch_bounds__(8 * TX) iso_fd8_v4(const __grid_constant__ Iso
       if (a.io.store | a.io.ic) fused_io4(a.io, g, i0, ix, iy, iz4, col, u4);
       float4 t4, out4;
 #pragma unroll
-      for (int c = 0; c < 4; c++) setc(t4, c, comp(cw0, c) - v[c] * comp(cvel, c));
+      for (int c = 0; c < 4; c++) set4(t4, c, cmp4(cw0, c) - v[c] * cmp4(cvel, c));
       if (MODE == 0) out4 = t4;  // KernelCPU seam: w0 -= vel * L[w1]
       else if (MODE == 1)        // + update2nd (leapfrog)
         out4 = make_float4((u4.x + u4.x) - t4.x, (u4.y + u4.y) - t4.y, (u4.z + u4.z) - t4.z, (u4.w + u4.w) - t4.w);
@@ -435,7 +427,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
 #pragma unroll
         for (int c = 0; c < 4; c++) {
           lzv[c] += a.c2z[m] * (zw[4 + c - m] + zw[4 + c + m]);
-          lxv[c] += a.c2x[m] * (comp(xm, c) + comp(xp, c));
+          lxv[c] += a.c2x[m] * (cmp4(xm, c) + cmp4(xp, c));
         }
       }
 #pragma unroll
@@ -444,7 +436,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
         if (do_y) {
           ly = a.c2y[0] * zw[4 + c];
 #pragma unroll
-          for (int m = 1; m <= R4; m++) ly += a.c2y[m] * (comp(q[R4 - m], c) + comp(q[R4 + m], c));
+          for (int m = 1; m <= R4; m++) ly += a.c2y[m] * (cmp4(q[R4 - m], c) + cmp4(q[R4 + m], c));
         }
         lyv[c] = ly;
       }
@@ -484,7 +476,7 @@ __global__ void __launch_bounds__(8 * TX, EDGE && MODE != 2 ? 512 / (8 * TX) : 0
       const float4 cw0 = s.w0[sb][tx][tzq], cvel = s.vel[sb][tx][tzq];
       float4 t4, out4;
 #pragma unroll
-      for (int c = 0; c < 4; c++) setc(t4, c, comp(cw0, c) - v[c] * comp(cvel, c));
+      for (int c = 0; c < 4; c++) set4(t4, c, cmp4(cw0, c) - v[c] * cmp4(cvel, c));
       if (MODE == 0) out4 = t4;
       else if (MODE == 1)
         out4 = make_float4((u4.x + u4.x) - t4.x, (u4.y + u4.y) - t4.y, (u4.z + u4.z) - t4.z, (u4.w + u4.w) - t4.w);

@@ -145,8 +145,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   uint64_t *accf = rawf + 24;                             // every MMA finished
   uint32_t *tslot = reinterpret_cast<uint32_t *>(smraw + 256);
   unsigned char *ops = smraw + 1024;
-  // this CTA's output columns [c_lo, c_lo + nw) (all npad of them: one column block per line tile)
-  const int c_lo = 0, nw = npad;
+  const int nw = npad;  // output columns
   const uint32_t a_bytes = kTcM * kTcBK * 4, b_bytes = (uint32_t)nw * kTcBK * 4;
   const size_t bfull = (size_t)npad * kTcBK * 4;  // one part of a K block of Bg
   const uint32_t stage_bytes = 3 * a_bytes + 2 * b_bytes;
@@ -154,7 +153,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   // lines m0 .. m0 + 127 of length n, element (m, k) at in[m n + k]
   const long long m0 = (long long)blockIdx.x * kTcM;
   const long long M = geo.lines;
-  const uint32_t ncols = nw <= 32 ? 32 : nw <= 64 ? 64 : nw <= 128 ? 128 : nw <= 256 ? 256 : 512;
+  const uint32_t ncols = nw <= 256 ? 256 : 512;
   const int nkb = (n + kTcBK - 1) / kTcBK;
 
   dep_launch();
@@ -199,8 +198,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         cp_async16(raw + kblock_off(r, q, kTcM), v ? in + (m0 + r) * n + k : in, v ? 16u : 0u);
       }
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(rawf + s)) : "memory");
-      if (lane == 0) {  // rows [c_lo, c_lo + nw) of the block's hi and lo parts (8-row groups of 256 B)
-        const unsigned char *blk = Bg + (size_t)kb * 2 * bfull + (size_t)c_lo * 32;
+      if (lane == 0) {  // the block's hi and lo parts (8-row groups of 256 B)
+        const unsigned char *blk = Bg + (size_t)kb * 2 * bfull;
         mbar_expect_tx(rawf + s, 2 * b_bytes);
         bulk_load(raw + 3 * a_bytes, blk, b_bytes, rawf + s);
         bulk_load(raw + 3 * a_bytes + b_bytes, blk + bfull, b_bytes, rawf + s);
@@ -230,7 +229,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       mbar_arrive(conv + s);
     }
   } else if (lane == 0) {
-    int issued = 0;
     for (int kb = 0; kb < nkb; kb++) {
       const int s = kb % S;
       if (!mbar_wait(conv + s, (uint32_t)(kb / S) & 1u, err)) {
@@ -250,9 +248,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         mma_tf32(d, dal, kmajor_desc(bh, 128, 256), idesc, 1u);
       }
       mma_commit(empty + s);
-      issued = kb + 1;
     }
-    (void)issued;
     mma_commit(accf);  // completes once every MMA issued above has finished
   }
   ok = __syncthreads_and(ok);
@@ -280,10 +276,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       tmem_ld32(taddr + (uint32_t)c0, v);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (row < M) {
-        float *o = out + row * n + c_lo + c0;
+        float *o = out + row * n + c0;
 #pragma unroll
         for (int j = 0; j < 32; j += 4)
-          if (c_lo + c0 + j + 4 <= n)
+          if (c0 + j + 4 <= n)
             __stcs(reinterpret_cast<float4 *>(o + j), make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
                                                                   __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])));
       }
@@ -557,9 +553,9 @@ __global__ void tf32_arrange_k(const float *__restrict__ D, unsigned char *Bg, i
 }
 }  // namespace
 
-// stages: lines of up to 256 points keep a CTA within half the shared memory
-// (two CTAs of at most 256 accumulator columns share an SM; 2-4 stages);
-// longer lines take one CTA per SM with a 512-column accumulator (up to 6)
+// stages of r2r_tc_k: lines of 129 to 256 points keep a CTA within half the shared
+// memory (two CTAs of 256 accumulator columns share an SM; 3 or 4 stages); longer
+// lines take one CTA per SM with a 512-column accumulator (5 or 6)
 static int tc_stages(int npad) {
   const size_t stage = 3 * (size_t)kTcM * kTcBK * 4 + 2 * (size_t)npad * kTcBK * 4;
   if (npad <= 256) return (int)std::min<size_t>(4, (113 * 1024 - 2048) / stage);  // two CTAs (1 KB reserved each)
@@ -581,8 +577,7 @@ static TtShape tt_shape(int npad) {
   return s;
 }
 
-size_t r2r_tc_smem(int n) {
-  const int npad = (n + 15) / 16 * 16;
+static size_t tc_smem(int npad) {
   return 1024 + (size_t)tc_stages(npad) * (3 * (size_t)kTcM * kTcBK * 4 + 2 * (size_t)npad * kTcBK * 4);
 }
 
@@ -590,7 +585,7 @@ size_t r2r_tc_smem(int n) {
 // (16-byte copies along z) and a line matrix of at most 512 rows
 bool r2r_tc_supported(int axis, int nx, int ny, int nz) {
   const int n = axis == 0 ? nx : axis == 1 ? ny : nz;
-  return nz % 4 == 0 && n >= 2 && n <= 512 && tc_stages((n + 15) / 16 * 16) >= 2 && r2r_tc_smem(n) <= 227 * 1024;
+  return nz % 4 == 0 && n >= 2 && n <= 512;
 }
 
 size_t r2r_tc_bytes(int n) {
@@ -598,7 +593,7 @@ size_t r2r_tc_bytes(int n) {
   return (size_t)((n + kTcBK - 1) / kTcBK) * 2 * npad * kTcBK * 4;
 }
 
-#define RTM_TC_ALL(X) X(2) X(3) X(4) X(5) X(6)
+#define RTM_TC_ALL(X) X(3) X(4) X(5) X(6)
 
 int r2r_tc_init() {
   const int mx = 227 * 1024;
@@ -641,7 +636,7 @@ void launch_r2r_tc(int axis, const float *in, float *out, const unsigned char *B
   // second column block reads and splits the strided lines again (200 points, 13.1 M
   // cells: 51 us, 60 as two blocks; 100 points, 10.2 M cells: 40, 33 as one block)
   if (axis == 2 && npad > 128) {
-    const size_t sm = r2r_tc_smem(n);
+    const size_t sm = tc_smem(npad);
     const int S = tc_stages(npad);
 #define RTM_TC_LAUNCH(SS) \
   if (S == SS) launch_dep(r2r_tc_k<SS>, (unsigned)tiles, kTcThreads, sm, st, in, out, Bg, n, npad, geo, err);

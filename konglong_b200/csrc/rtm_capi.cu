@@ -338,8 +338,7 @@ static int yseg_pair(Engine *h, int tx, int ctas_per_sm) {
 
 // Tile table for tile width tx and y segment yseg: columns touching an x or
 // z PML face are PML tiles over all y; the others are PML tiles over the y
-// faces and interior tiles between.  Built on the host and uploaded (never
-// inside a stream capture).
+// faces and interior tiles between.  Built on the host and uploaded.
 static int build_tiles(Engine *h, TileSet &t, int tx, int yseg) {
   yseg = std::max(1, yseg);
   if (t.current(tx, yseg)) return RTM_OK;
@@ -956,7 +955,7 @@ static int do_inject(Engine *h, int it) {
   }
   KScope k(h, RTM_K_INJECT, (int)t.groups.size() + (t.n_ungrouped ? 1 : 0));
   for (const GroupDev &g : t.groups)
-    launch_inject_group(g, td, it, h->plane, h->w0, h->vel, h->d.nx, h->d.ny, h->d.nz, h->st);
+    launch_inject_group(g, td, it, h->w0, h->vel, h->d.nx, h->d.ny, h->d.nz, h->st);
   if (t.n_ungrouped) {
     td.ids = t.ungrouped, td.nids = t.n_ungrouped;
     launch_inject_scatter(td, it, h->w0, h->vel, h->d.nx, h->d.ny, h->d.nz, h->st);
