@@ -3,7 +3,7 @@
 // every grid line (FdEngine_cfd::banmul_* / banbks_*,
 // bgprtm/FdEngine_cfd.cpp:164-356).  A CTA holds 32 lines (lane = line), one HBM
 // read and one write per cell:
-//   1  four warps form the 11-point right-hand sides, a run of rows each;
+//   1  its warps form the 11-point right-hand sides, a run of rows each;
 //   2  one warp runs the two recurrences of the band LU.
 //
 // What bounds it: shared memory caps the lines in flight (three 512-point tiles
@@ -32,8 +32,8 @@
 //     table rows one quad ahead was slower (z lines 232 us): the copies cost
 //     more than the wait;
 //   - resident CTAs solve on different schedulers (285 -> 259 us);
-//   - eight warps form the right-hand sides of long lines, four of short ones,
-//     whose CTAs fill the SM (the line at kLongLine points);
+//   - four warps where four or more tiles fit an SM, eight where fewer do
+//     (tile_threads);
 //   - the tile that a resident CTA's successor will load is prefetched into L2
 //     (250 -> 240 us).
 #include <algorithm>
@@ -355,14 +355,27 @@ __global__ void __launch_bounds__(256, 3) cfd_tile_k(const __grid_constant__ Cfd
 }
 
 constexpr size_t kTileSmem = 227 * 1024;
-constexpr int kLongLine = 250;
+
+// Tiles whose shared memory fits an SM together
+int tiles_fit(size_t smem) { return (int)((228 * 1024) / (smem + 1024)); }
+
+// Threads of a tile of `smem` bytes.  The registers let six CTAs of 128 threads or
+// three of 256 onto an SM.  While four or more tiles fit, their number hides more
+// than their warps: lines of 256 points, 512 x 400 of them, take 105 us (x) and 106
+// us (z) with 128 threads, 144 and 127 with 256; of 400 points, 400 x 400, 142 and
+// 136 against 158 and 136.  Where three fit, either way (512 points: 236 and 221
+// against 236 and 223), eight warps copy faster if the copies are not asynchronous
+// (512 points, depth 151: 95 and 63 against 79 and 61 us).  Plain copies already
+// want them where four tiles fit: 320 points, five tiles, 150 us against 156, 330
+// points, four tiles, 67 against 59.
+int tile_threads(size_t smem, bool async) { return tiles_fit(smem) >= (async ? 4 : 5) ? 128 : 256; }
 
 // byte offset of the tile after the barrier and the factor table of `tab` rows
 int tile_off(int tab) { return (128 + tab * 36 + 127) / 128 * 128; }
 
 // CTAs of `threads` threads and `smem` bytes resident on the device at once
 int tiles_ahead(int sms, int threads, size_t smem) {
-  return sms * (int)std::max<size_t>(1, std::min<size_t>(768 / threads, (228 * 1024) / (smem + 1024)));
+  return sms * std::max(1, std::min(768 / threads, tiles_fit(smem)));
 }
 
 template <int IO>
@@ -385,7 +398,6 @@ bool launch_cfd_tile(int axis, const CfdPlanDev &p, const float *in, float *out,
   a.tab = p.k0 + n4 - p.k1;
   a.off = tile_off(a.tab);
   const CUtensorMap none{};
-  const int threads = p.n > kLongLine ? 256 : 128;
   if (axis == DZ) {
     a.nlines = (long long)nx * ny;
     // lines 4 floats (mod 32) apart: a quad load of eight lanes meets every bank once
@@ -396,6 +408,7 @@ bool launch_cfd_tile(int axis, const CfdPlanDev &p, const float *in, float *out,
     const size_t smem = bytes(a.lines);
     if (smem > kTileSmem) return false;
     const unsigned grid = (unsigned)((a.nlines + a.lines - 1) / a.lines);
+    const int threads = tile_threads(smem, nz % 4 == 0);
     a.ahead = tiles_ahead(sms, threads, smem);
     if (nz % 4 == 0) launch_dep(cfd_tile_k<IO_LINES_BULK>, grid, threads, smem, st, p, none, none, a, err);
     else launch_dep(cfd_tile_k<IO_LINES>, grid, threads, smem, st, p, none, none, a, err);
@@ -409,6 +422,7 @@ bool launch_cfd_tile(int axis, const CfdPlanDev &p, const float *in, float *out,
   const size_t smem = a.off + (size_t)rows * 128;
   if (smem > kTileSmem) return false;
   const dim3 grid((nz + 31) / 32, axis == DX ? ny : nx);
+  const int threads = tile_threads(smem, tin && tout);
   a.ahead = tiles_ahead(sms, threads, smem);
   if (tin && tout) launch_dep(cfd_tile_k<IO_ROWS_TMA>, grid, threads, smem, st, p, *tin, *tout, a, err);
   else launch_dep(cfd_tile_k<IO_ROWS>, grid, threads, smem, st, p, none, none, a, err);

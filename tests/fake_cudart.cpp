@@ -58,12 +58,12 @@ bool fails(const std::string &what, const std::string &name = "") {
                                      name.find(s.fail_what.substr(what.size() + 1)) != std::string::npos;
   return s.fail_after >= 0 && is && s.fail_after-- == 0;
 }
-cudaError_t launch(const void *f, cudaStream_t st) {
+cudaError_t launch(const void *f, dim3 b, cudaStream_t st) {
   State &s = S();
   const std::string &name = s.kernel[f];
   if (fails("launch", name)) return err(s.fail_code);
   s.count[st]++;
-  s.launched.push_back(name);
+  s.launched.push_back(name + " [" + std::to_string(b.x * b.y * b.z) + "]");
   return cudaSuccess;
 }
 int encode_ok(...) { return 0; }
@@ -72,6 +72,7 @@ int encode_ok(...) { return 0; }
 extern "C" {
 // ---- what tests call ----
 void fake_clear() { S().launched.clear(); }
+// launches whose "name [threads]" holds `part`
 long fake_launched(const char *part) {
   long n = 0;
   for (auto &l : S().launched) n += l.find(part) != std::string::npos;
@@ -117,8 +118,10 @@ cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *s, void *st) {
   *g = call.g, *b = call.b, *s = call.s, *(cudaStream_t *)st = call.st;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **, size_t, cudaStream_t st) { return launch(f, st); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) { return launch(f, c->stream); }
+cudaError_t cudaLaunchKernel(const void *f, dim3, dim3 b, void **, size_t, cudaStream_t st) { return launch(f, b, st); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) {
+  return launch(f, c->blockDim, c->stream);
+}
 cudaError_t cudaGetLastError() {
   cudaError_t e = S().last;
   S().last = cudaSuccess;

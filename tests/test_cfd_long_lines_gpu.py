@@ -1,7 +1,8 @@
 """Compact-FD lines longer than a shared-memory tile of 32 lines: z tiles of 16 and 8
 lines (the last one ragged, nz that allows bulk copies and not), the longest that
 take 32, and x / y lines around the length at which the streamed kernel takes over.
-Up to 1815 points the z solve that carries the epilogue (kernel_variant 9) fits and
+Likewise the lines at which a tile goes from four warps to eight: 316 and 336 points
+with plain copies, 416 and 448 with asynchronous ones.  Up to 1815 points the z solve that carries the epilogue (kernel_variant 9) fits and
 gives the same bits, as does the streamed kernel (5) for x / y lines; longer z lines
 are within twice the FP32 oracle's distance from the FP64 one (rounding grows some
 hundred times in the band solves, whose symbol falls to 3e-5 at the Nyquist
@@ -38,6 +39,8 @@ def _variant(spec, model, w0, w1, variant):
 
 
 @pytest.mark.parametrize("shape, other", [
+    ((316, 17, 33), 5), ((336, 16, 33), 5), ((17, 331, 37), 5), ((17, 16, 315), 9), ((17, 16, 333), 9),
+    ((416, 16, 36), 5), ((448, 17, 36), 5), ((16, 444, 40), 5), ((17, 17, 416), 9), ((17, 17, 448), 9),
     ((17, 17, 1764), 9), ((17, 17, 1784), 9), ((17, 17, 1792), 9), ((19, 17, 1813), 9),
     ((1780, 16, 36), 5), ((1781, 16, 33), 5), ((1796, 16, 36), 5), ((1900, 16, 33), 5), ((16, 1780, 36), 5), ((16, 1900, 36), 5)])
 def test_long_lines_equal_other_forms(shape, other):
