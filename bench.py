@@ -86,24 +86,29 @@ def kernel_alg_bytes(spec, m):
 # launch, from ncu captures of the same kernels on the 0.75-scale grid of the
 # vti_cfd workload.  The PML slabs scale with the grid, so bytes per cell carry
 # over to the full grid.  Each entry records the SHA-256 prefix of the kernel
-# source it was captured on; when the source has changed since, the figure no
+# sources it was captured on; when a source has changed since, the figure no
 # longer describes the kernel that runs and the bench reports traffic as null.
-MEASURED_DRAM_B_PER_CELL = {"vti_cfd": {"cfd_div_epilogue": 37.9, "cfd_grad_epilogue": 38.7,
-                                        "cfd_x": 6.75, "cfd_y": 6.83, "cfd_z": 6.83}}
-MEASURED_DRAM_SOURCE = {"vti_cfd": ("konglong_b200/csrc/kernels_cfd.cu", "f002906f4d2b116c")}
+MEASURED_DRAM_B_PER_CELL = {"vti_cfd": {"cfd_div_epilogue": 36.9, "cfd_grad_epilogue": 38.0,
+                                        "cfd_x": 6.85, "cfd_y": 7.47, "cfd_z": 6.90}}
+MEASURED_DRAM_SOURCE = {"vti_cfd": (tuple("konglong_b200/csrc/" + f for f in
+                                          ("kernels_cfd_tile.cu", "kernels_cfd_epi.cu", "cfd_rows.cuh", "cfd_epi.cuh")),
+                                    "c1912721f63c7b8e")}
 
 
 def measured_traffic_current(workload):
-    """True when the kernel source behind MEASURED_DRAM_B_PER_CELL[workload] is unchanged."""
+    """True when the kernel sources behind MEASURED_DRAM_B_PER_CELL[workload] are unchanged."""
     import hashlib
     src = MEASURED_DRAM_SOURCE.get(workload)
     if not src:
         return False
+    sha = hashlib.sha256()
     try:
-        with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), src[0]), "rb") as f:
-            return hashlib.sha256(f.read()).hexdigest()[:16] == src[1]
+        for name in src[0]:
+            with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), name), "rb") as f:
+                sha.update(f.read())
     except OSError:
         return False
+    return sha.hexdigest()[:16] == src[1]
 
 
 class ClockSampler:
@@ -346,8 +351,8 @@ def run_small_shots(args, ranks):
     """Batched small-shot workload (64 seeded shots, grids 96-256 per axis,
     500-2000 steps, receivers every step; ISO, or VTI with per-layer Thomsen
     parameters for small_shots_vti): every shot's full modelling run, once per
-    shot by itself and once for all shots together (each on its own stream,
-    side by side on the device).  Metric: shots per second of the batched run."""
+    shot by itself and once for all shots together (shots of these sizes each on
+    its own stream, side by side on the device).  Metric: shots per second of the batched run."""
     from konglong_b200 import workloads as W
     from konglong_b200.propagator import Batch, Propagator, spread_coeffs
     from konglong_b200.spec import ISO, VTI

@@ -391,7 +391,9 @@ int rtm_illum_compensate(rtm_handle *h, int smooth_xy, int smooth_z, float amp_d
 
 /* Propagator::modelling loop (bgprtm/Propagator.cpp:1099-1153): for it in
  * [0, nts): kernel, update2nd, inject(it + it_shift), extract(it / ntratio)
- * when it % ntratio == 0, swap.  Fused kernels, launched step by step. */
+ * when it % ntratio == 0, swap.  Fused kernels, launched step by step.  Returns when
+ * all of them have run, after an error too: the state is then that of some step of
+ * the loop, until rtm_reset or rtm_put. */
 int rtm_modelling(rtm_handle *h, int nts, int it_shift, int ntratio);
 
 /* Propagator::migration loop (bgprtm/Propagator.cpp:1210-1255).

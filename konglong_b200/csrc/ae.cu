@@ -289,10 +289,10 @@ constexpr int kChunkBlocks = 8192;  // blocks per encode / decode pass over a vo
 // largest |value|, E3's tiles and D1's latents pass through shared memory.
 // One warp per block with the layer outputs in shared memory, before, used 8 or
 // 1 of the 16 rows in five layers of eight and moved every value through shared
-// memory: encode + decode of 400 x 400 x 320 took 904 us, now 91 + 68 us.  The
-// MMAs with full rows take 27 us of tensor time and the volumes 67 us of memory
-// time; what bounds the kernels is issue slots at 16 warps an SM (half of them
-// used) and, decoding, the half-sector stores.
+// memory: encode + decode of 400 x 400 x 320 took 907 us, now 151 (84 + 65 us by
+// events over repeated calls).  The MMAs with full rows take 27 us of tensor time and
+// the volumes 67 us of memory time; what bounds the kernels is issue slots at 16
+// warps an SM (half of them used) and, decoding, the half-sector stores.
 // Each output element is the same mma.sync chain over k in steps of 16 as in
 // gemm_bf16_k, with the same operand roundings, bias and activation, so the
 // results equal the layer-by-layer path bit for bit.

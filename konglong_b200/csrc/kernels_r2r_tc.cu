@@ -633,8 +633,9 @@ void launch_r2r_tc(int axis, const float *in, float *out, const unsigned char *B
     tiles = (geo.total_m + kTcM - 1) / kTcM;
   }
   // z lines of more than 128 points: the whole line's columns in one CTA, since a
-  // second column block reads and splits the strided lines again (200 points, 13.1 M
-  // cells: 51 us, 60 as two blocks; 100 points, 10.2 M cells: 40, 33 as one block)
+  // second column block reads and splits the strided lines again (65536 lines of 132
+  // points: 41 us, 47 by r2r_tt_k; 256: 74, 82; 512: 179, 221; shorter lines are one
+  // block there, 128: 39, 33; 64: 24, 21)
   if (axis == 2 && npad > 128) {
     const size_t sm = tc_smem(npad);
     const int S = tc_stages(npad);
